@@ -359,6 +359,27 @@ cr_status ensure_queues(cr_context* ctx, uint64_t ntWant, uint64_t hugeWant) {
     return CR_OK;
 }
 
+// The chain heads of the binned stage 3 for a frame of `tiles` screen tiles;
+// without memory for them the frame takes the unbinned stage 3.
+void ensure_bins(cr_context* ctx, uint64_t tiles) {
+    if (tiles <= ctx->binTiles) return;
+    if (cudaDeviceSynchronize() != cudaSuccess) return;
+    const size_t bytes = tiles * CR_BIN_CHAINS * 8;
+    ctx->dev_free(ctx->binHeads, ctx->binTiles * CR_BIN_CHAINS * 8);
+    ctx->binHeads = nullptr;
+    ctx->binTiles = 0;
+    void* heads = nullptr;
+    if (ctx->dev_alloc(&heads, bytes, "stage-3 bins") != CR_OK) return;
+    if (cudaMemset(heads, 0, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->dev_free(heads, bytes);
+        return;
+    }
+    ctx->binHeads = (unsigned long long*)heads;
+    ctx->binTiles = tiles;
+    ctx->binStamp = 0;
+}
+
 // Allocates (once) and launches the mesh's box pass on the legacy stream.
 cr_status launch_mesh_boxes(cr_context* ctx, MeshRec& m) {
     const size_t ib = align_up((size_t)((m.numTriangles + CR_BATCH - 1) / CR_BATCH) * 24, 256);
@@ -720,6 +741,7 @@ cr_status cr_destroy(cr_context* ctx) {
     if (ctx->ntList) cudaFree(ctx->ntList);
     if (ctx->s1List) cudaFree(ctx->s1List);
     if (ctx->hugeList) cudaFree(ctx->hugeList);
+    if (ctx->binHeads) cudaFree(ctx->binHeads);
     if (ctx->counters) cudaFree(ctx->counters);
     if (ctx->dFrame) cudaFree(ctx->dFrame);
     if (ctx->hFrame) cudaFreeHost(ctx->hFrame);
@@ -1307,7 +1329,27 @@ cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_
     rp.counters = ctx->counters;
     rp.hostCounters = ctx->hCounters;
 
+    // Stage 3 binned by screen tile.  Not for the reference build's
+    // arithmetic (its rounding follows the compiled expressions), nor where
+    // the heads would be large (1 KB per tile: 16 MB at 8192 x 8192) or a memory
+    // budget is kept for the scene and the queues.
+    const uint64_t binTiles = (uint64_t)((cam->width + CR_TILE_SIZE - 1) / CR_TILE_SIZE) *
+                              (uint64_t)((cam->height + CR_TILE_SIZE - 1) / CR_TILE_SIZE);
+    const bool bins = !refMath && count > 0 && !(flags & kRenderResolveOnly) && ctx->cfg.memory_budget == 0 &&
+                      cam->width <= 8192 && cam->height <= 8192;
+    if (bins) ensure_bins(ctx, binTiles);
+    fp.binTilesX = (uint32_t)((cam->width + CR_TILE_SIZE - 1) / CR_TILE_SIZE);
+    fp.binTilesY = (uint32_t)((cam->height + CR_TILE_SIZE - 1) / CR_TILE_SIZE);
+
     auto issue = [&](cudaEvent_t* tev, cudaEvent_t rasterEnd) -> cr_status {
+        if (bins && ctx->binHeads && ctx->hugeCap < 0xffffffffull) {
+            if (++ctx->binStamp == 0) {  // the stamps wrapped: empty every chain
+                CR_CUDA(cudaMemsetAsync(ctx->binHeads, 0, ctx->binTiles * CR_BIN_CHAINS * 8, stream), "stage-3 bins");
+                ctx->binStamp = 1;
+            }
+            fp.binHeads = ctx->binHeads;
+            fp.binStamp = ctx->binStamp;
+        }
         fp.ntList = ctx->ntList;
         fp.ntCap = ctx->ntCap;
         fp.hugeList = ctx->hugeList;

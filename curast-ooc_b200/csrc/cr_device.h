@@ -42,6 +42,7 @@
 #define CR_CTR_UNITS 7          // item groups the group cull leaves for the item cull
 #define CR_CTR_CGROUPS 8        // chunk groups the group cull leaves for the chunk cull
 #define CR_CTR_VSLICES 9        // slices the vertex pass evaluated (frames with slice stamps)
+#define CR_CTR_S3UNIT 10        // quadrants of screen tiles taken by k_stage3_bins
 #define CR_CTR_COUNT 16
 
 // Compressed geometry (the reference's IX_PU16 meshes, CMesh fields
@@ -152,9 +153,11 @@ static_assert(sizeof(CrSegment) == 144, "CrSegment layout");
 struct alignas(16) CrTile {     // HugeTriangle, HostDeviceInterface.h:254-259
     int32_t instance;           // instance | view << 26 (view 0 in single-view frames)
     int32_t triangle;
-    int32_t tile_x;
-    int32_t tile_y;
+    int32_t tile_x;             // binned frames (CrFrameParams::binHeads): the next entry
+    int32_t tile_y;             // of its chain (0xffffffff: none); tile_y unused
 };
+// Binned stage 3: chains per 64x64 screen tile, each a list of queue entries.
+#define CR_BIN_CHAINS 128
 
 // Stage-2 queue entry: (view << 58) | (instance << 32) | triangle; single-view
 // frames use view 0, i.e. the reference's packing (tv.cu:192-197).
@@ -280,6 +283,16 @@ struct CrFrameParams {
     // 1: stage 2 runs as k_stage2_dense (the host's estimate from the
     // context's last measured frame: many queued triangles)
     uint32_t dense2;
+    // > 0: stage 1 takes every triangle of the frame (this many, CrInstance::cum
+    // their prefix sum) straight through the per-triangle path: no frame cull,
+    // no vertex pass, no records
+    uint64_t direct;
+    // binned stage 3 (k_stage3_bins; nullptr: k_stage3): per screen tile
+    // CR_BIN_CHAINS chain heads, (stamp << 32) | first queue entry; a head of
+    // another stamp is an empty chain, so no frame clears them
+    unsigned long long* binHeads;
+    uint32_t binStamp;
+    uint32_t binTilesX, binTilesY;
 };
 #define CR_CHUNK_EVAL 0xffu
 
@@ -350,6 +363,7 @@ struct CrLaunchShape {
     int s1RasterBlocks;         // k_s1raster, warp-wide tiny rasters
     int stage2DenseBlocks;      // k_stage2_dense
     int s1RasterOwnBlocks;      // k_s1raster, each lane its own tiny raster
+    int stage3BinBlocks;        // k_stage3_bins
 };
 
 int cr_query_launch_shape(int device, CrLaunchShape* out);

@@ -33,6 +33,7 @@
 #include <cstdint>
 
 #include "raster_core.cuh"
+#include "stage3_bins.cuh"
 
 namespace {
 
@@ -1045,6 +1046,9 @@ int cr_query_launch_shape(int device, CrLaunchShape* out) {
         return -1;
     out->s1RasterOwnBlocks = sms * (bo > 0 ? bo : 1);
     out->stage3Blocks = sms * (b3 > 0 ? b3 : 1);
+    int bb = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bb, k_stage3_bins, B3_THREADS, 0) != cudaSuccess) return -1;
+    out->stage3BinBlocks = sms * (bb > 0 ? bb : 1);
     return 0;
 }
 
@@ -1124,5 +1128,10 @@ int cr_launch_stage2(const CrFrameParams& p, const CrLaunchShape& s, void* strea
 }
 
 int cr_launch_stage3(const CrFrameParams& p, const CrLaunchShape& s, void* stream) {
+    if (p.binHeads) {
+        const uint64_t units = 4ull * p.binTilesX * p.binTilesY;
+        return launch_pdl(k_stage3_bins, (unsigned)std::min<uint64_t>(units, (uint64_t)s.stage3BinBlocks), B3_THREADS,
+                          stream, p);
+    }
     return launch_pdl(k_stage3<S3_WARPS, false>, (unsigned)s.stage3Blocks, S3_WARPS * 32, stream, p);
 }

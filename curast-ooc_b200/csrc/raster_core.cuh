@@ -1283,6 +1283,17 @@ __device__ __forceinline__ void stage2_run(const CrFrameParams& p) {
                         t.triangle = (int32_t)(pk & 0xffffffffu);
                         t.tile_x = tx + (int)(i % (uint32_t)tsx);
                         t.tile_y = ty + (int)(i / (uint32_t)tsx);
+                        if (!MULTI && !REF_MATH && p.binHeads) {  // linked into its screen tile's chain
+                            const bool in = (uint32_t)t.tile_x < p.binTilesX && (uint32_t)t.tile_y < p.binTilesY;
+                            const uint64_t tile = (uint64_t)t.tile_y * p.binTilesX + (uint32_t)t.tile_x;
+                            t.tile_x = -1;
+                            if (in) {  // always: a triangle's box is clamped to the screen
+                                const unsigned long long prev = atomicExch(
+                                    &p.binHeads[tile * CR_BIN_CHAINS + (slot & (CR_BIN_CHAINS - 1))],
+                                    ((unsigned long long)p.binStamp << 32) | slot);
+                                if ((uint32_t)(prev >> 32) == p.binStamp) t.tile_x = (int32_t)(uint32_t)prev;
+                            }
+                        }
                         p.hugeList[slot] = t;
                     } else {
                         atomicOr(&p.counters[CR_CTR_OVERFLOW], 2ull);

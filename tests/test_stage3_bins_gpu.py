@@ -1,0 +1,55 @@
+"""The binned stage 3 (k_stage3_bins): screen-filling, near-plane and sliver
+triangles at the edges of its tiles, regions and rounds, against the CPU oracle
+and against the unbinned kernel, which a context with a memory budget takes."""
+import numpy as np
+import pytest
+
+import oracle_lib as ol
+import pycurast as pc
+import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def triangles(n, seed):
+    """Triangles of every size stage 3 sees, some with hostile coordinates."""
+    rng = np.random.default_rng(seed)
+    z = -rng.uniform(0.3, 6.0, n)
+    z[: n // 10] = rng.uniform(-0.2, 0.15, n // 10)  # across the camera plane
+    centre = np.stack([rng.uniform(-2, 2, n), rng.uniform(-1.2, 1.2, n), z], -1)
+    tri = centre[:, None, :] + rng.normal(size=(n, 3, 3)) * np.exp(rng.normal(0.0, 1.0, n))[:, None, None]
+    thin = slice(n // 3, n // 2)  # slivers: the third corner close to the first edge
+    t = rng.uniform(0, 1, n)[thin, None]
+    tri[thin, 2] = tri[thin, 0] * (1 - t) + tri[thin, 1] * t + rng.normal(size=tri[thin, 2].shape) * 1e-3
+    tri[5, 1] = tri[5, 0]                            # no area
+    tri[6, 0, 0], tri[7, 1, 2], tri[8, 2, 1] = np.nan, np.inf, 1e30
+    tri[9] *= 1e-12
+    pos = tri.reshape(-1, 3).astype(np.float32)
+    return pos, np.arange(3 * n, dtype=np.uint32).reshape(n, 3), rng.integers(0, 2**32, 3 * n, np.uint64).astype(np.uint32)
+
+
+# one tile and one past it, columns past the right edge that wrap into the next
+# row, many rounds of one tile (1500 triangles over 6 tiles), a wide window
+@pytest.mark.parametrize("n,W,H", [(60, 64, 64), (60, 65, 129), (1500, 130, 70), (300, 333, 197), (200, 1917, 300)])
+def test_bins_match_the_oracle_and_the_unbinned_kernel(gpu, n, W, H):
+    import torch
+
+    mesh = triangles(n, 100 + n + W)
+    view, proj = scenes.identity(), scenes.perspective(60.0, W / H, 0.01, 100.0)
+    got = []
+    for budget in (0, 8 << 30):
+        with pc.Context(memory_budget=budget) as ctx:
+            inst = [(ctx.mesh_from_host(*mesh), scenes.identity())]
+            vis = torch.empty(W * H, dtype=torch.int64, device="cuda")
+            rgba = torch.empty(W * H, dtype=torch.int32, device="cuda")
+            cam = pc.make_camera(view, proj, W, H)
+            for _ in range(2):  # the second frame's chains lie over the first's
+                ctx.render(inst, cam, vis.data_ptr(), rgba.data_ptr())
+            torch.cuda.synchronize()
+            st, stats = ctx.stats()
+            assert st == pc.CR_OK and stats.huge_tiles > 0
+            got.append((vis.cpu().numpy().view(np.uint64), int(stats.huge_tiles)))
+    assert got[0][1] == got[1][1]
+    assert np.array_equal(got[0][0], got[1][0])
+    fb, _ = ol.raster(ol.Frame([(*mesh, scenes.identity())], view), W, H, proj[5])
+    assert np.array_equal(got[0][0], fb)
