@@ -1099,6 +1099,9 @@ struct S2Span {
 __device__ __forceinline__ S2Span s2_span_setup(float start_x, float start_y, int size_x, int size_y, float asx,
                                                 float asy, float abx, float aby, float acx, float acy, float inv_det) {
     const double u = 5.9604644775390625e-08;
+    // the fast-math build contracts products (fewer roundings, so the same
+    // bound holds) and flushes denormal products and differences to zero
+    const double FZ = REF_MATH ? 1e-36 : 0.0;
     S2Span P;
     P.size_x = size_x;
     P.px0 = (double)start_x;
@@ -1118,8 +1121,8 @@ __device__ __forceinline__ S2Span s2_span_setup(float start_x, float start_y, in
     };
     const double Smax = absmax(aS, cS0, cS1), Tmax = absmax(aT, cT0, cT1);
     const double adi = fabs(di);
-    const double Es = 16.0 * u * adi * (fabs((double)acy) * AX + fabs((double)acx) * AY) + 4.0 * u * Smax + 1e-37;
-    const double Et = 16.0 * u * adi * (fabs((double)abx) * AY + fabs((double)aby) * AX) + 4.0 * u * Tmax + 1e-37;
+    const double Es = 16.0 * u * adi * (fabs((double)acy) * AX + fabs((double)acx) * AY) + 4.0 * u * Smax + 1e-37 + FZ * adi;
+    const double Et = 16.0 * u * adi * (fabs((double)abx) * AY + fabs((double)aby) * AX) + 4.0 * u * Tmax + 1e-37 + FZ * adi;
     const double Ev = 2.0 * (Es + Et) + 4.0 * u * (Smax + Tmax + 1.0) + 1e-37;
     const double A[3] = {aS, aT, -(aS + aT)};
     const double B0[3] = {cS0, cT0, 1.0 - cS0 - cT0};
@@ -1313,13 +1316,8 @@ __device__ __forceinline__ void stage2_run(const CrFrameParams& p) {
             o.start_y = floorf(su.min_y);
             o.size_x = su.size_x;
             o.size_y = su.numFragments / su.size_x;
-            if constexpr (REF_MATH) {  // every fragment of the box is tested
-                o.sp.whole = true;
-                o.sp.size_x = o.size_x;
-            } else {
-                o.sp = s2_span_setup(o.start_x, o.start_y, o.size_x, o.size_y, su.asx, su.asy, su.abx, su.aby,
-                                     su.acx, su.acy, su.inv_det);
-            }
+            o.sp = s2_span_setup(o.start_x, o.start_y, o.size_x, o.size_y, su.asx, su.asy, su.abx, su.aby,
+                                 su.acx, su.acy, su.inv_det);
             o.fb = MULTI ? tg.fb : p.fb;
             o.asx = su.asx;
             o.asy = su.asy;
@@ -1449,6 +1447,12 @@ __device__ __forceinline__ float intersect_mt(V3 dir, V3 v0, V3 e1, V3 e2) {
 // margins below over-cover all of them by 2x, in double precision, so a
 // column outside the span cannot pass the float test.  A triangle whose T is
 // within its error bound of 0, or with non-finite values, is not pruned.
+//
+// The fast-math build (REF_MATH) divides and takes square roots within 2 ulp
+// instead of half of one, which no term above exceeds by more than 3x, and
+// flushes denormals: its margins are 4x with an absolute floor.
+constexpr double S3_SLACK = REF_MATH ? 4.0 : 1.0;
+constexpr double S3_FLOOR = REF_MATH ? 1e-35 : 0.0;
 struct S3Prune {
     bool on;
     int s;
@@ -1475,14 +1479,16 @@ __device__ __forceinline__ S3Prune s3_prune_setup(V3 av, V3 e1f, V3 e2f, float f
     const double T = e2[0] * P.q[0] + e2[1] * P.q[1] + e2[2] * P.q[2];
     auto n1s = [](const double* v) { return fabs(v[0]) + fabs(v[1]) + fabs(v[2]); };
     const double St = n1s(t), S1 = n1s(e1), S2 = n1s(e2);
-    const double eD = 8.0 * u * 1.001 * S1 * S2, eU = 8.0 * u * 1.001 * St * S2, eV = 8.0 * u * 1.001 * St * S1;
-    const double eT = 8.0 * u * S2 * St * S1;
+    const double L = S3_SLACK, Z = S3_FLOOR;
+    const double eD = L * 8.0 * u * 1.001 * S1 * S2 + Z, eU = L * 8.0 * u * 1.001 * St * S2 + Z;
+    const double eV = L * 8.0 * u * 1.001 * St * S1 + Z;
+    const double eT = L * 8.0 * u * S2 * St * S1 + Z;
     P.mD = eD;
     P.mU = eU;
     P.mV = eV;
-    P.mK = 6.0 * u * 1.001 * n1s(P.n1) + 1.01 * eD + eU + eV;
-    P.ex = 8.0 * u * (1.0 / (double)fa);
-    P.ey = 8.0 * u * (1.0 / (double)f);
+    P.mK = L * 6.0 * u * 1.001 * n1s(P.n1) + 1.01 * eD + eU + eV;
+    P.ex = L * 8.0 * u * (1.0 / (double)fa);
+    P.ey = L * 8.0 * u * (1.0 / (double)f);
     P.on = isfinite(T) && isfinite(eT) && fabs(T) > 2.0 * eT && isfinite(P.mK);
     P.s = T > 0.0 ? 1 : -1;
     return P;
@@ -1503,13 +1509,13 @@ __device__ __forceinline__ void s3_row_span(const S3Prune& P, float fx0, float p
     const double ry = ib * (2.0 * ((double)py + 0.5) / (double)Hf - 1.0);
     const double dxm = fmax(fabs(B), fabs(A * 63.0 + B)) + P.ex, dym = fabs(ry) + P.ey;
     const double dn = sqrt(dxm * dxm + dym * dym + 1.0) * (1.0 + 16.0 * u);
-    const double ex = P.ex + 2.0 * u * dxm, ey = P.ey + 2.0 * u * dym;
+    const double ex = P.ex + S3_SLACK * 2.0 * u * dxm, ey = P.ey + S3_SLACK * 2.0 * u * dym;
     double lo = 0.0, hi = 63.0;
     bool empty = false;
     // keep columns with sg * (N . d) >= -margin, d = (A c + B, ry, -1)
     auto keep = [&](const double* N, double sg, double eps) {
         const double m = 2.0 * (eps * dn + fabs(N[0]) * ex + fabs(N[1]) * ey +
-                                8.0 * u * (fabs(N[0]) * dxm + fabs(N[1]) * dym + fabs(N[2])));
+                                S3_SLACK * 8.0 * u * (fabs(N[0]) * dxm + fabs(N[1]) * dym + fabs(N[2])));
         const double a = sg * N[0] * A;
         const double b = sg * (N[0] * B + N[1] * ry - N[2]);
         if (a > 0.0) lo = fmax(lo, (-m - b) / a);
@@ -1587,14 +1593,12 @@ __global__ void __launch_bounds__(WARPS * 32, 3) k_stage3(const CrFrameParams p)
 #pragma unroll
         for (int g = 0; g < 2; ++g)
             if (g < groups && 32 * g + lane < rpb) spanLen[g] = CR_TILE_SIZE;
-        if constexpr (!REF_MATH) {  // the fast-math build traces every pixel of the tile
-            const S3Prune P = s3_prune_setup(av, e1, e2, fa, f);
+        const S3Prune P = s3_prune_setup(av, e1, e2, fa, f);
 #pragma unroll
-            for (int g = 0; g < 2; ++g)
-                if (spanLen[g])
-                    s3_row_span(P, fx0, (float)(int)(fy0 + (float)(row0 + 32 * g + lane)), Wf, Hf, fa, f,
-                                spanLo[g], spanLen[g]);
-        }
+        for (int g = 0; g < 2; ++g)
+            if (spanLen[g])
+                s3_row_span(P, fx0, (float)(int)(fy0 + (float)(row0 + 32 * g + lane)), Wf, Hf, fa, f, spanLo[g],
+                            spanLen[g]);
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
             if (g >= groups) break;
