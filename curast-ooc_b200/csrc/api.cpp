@@ -550,6 +550,10 @@ void read_counters(cr_context* ctx) {
     ctx->last.vertex_slices_evaluated =
         !ctx->last.vertex_chunks ? 0 : ctx->lastStamps ? c[CR_CTR_VSLICES] : c[CR_CTR_CHUNKS] * (CR_VCHUNK / CR_VSLICE);
     ctx->last.stage1_survivors = c[CR_CTR_SURVIVORS];
+    if (ctx->lastDirect) {  // nothing culled ahead of the per-triangle path
+        ctx->last.work_items_drawn = ctx->last.work_items;
+        ctx->last.stage1_survivors = ctx->lastDirect;
+    }
 }
 
 cr_status run_frame(cr_context* ctx, uint32_t flags, cudaStream_t stream, uint64_t instances, uint64_t triangles,
@@ -1154,6 +1158,17 @@ cr_status cr_render(cr_context* ctx, const cr_instance* instances, uint32_t coun
 
 }  // extern "C"
 
+// Frames of at most this many triangles take every triangle straight through
+// the per-triangle path (CrFrameParams::direct).
+#ifndef CR_DIRECT_RECORDS
+#define CR_DIRECT_RECORDS (1ull << 17)
+#endif
+#ifndef CR_DIRECT_BOXES
+#define CR_DIRECT_BOXES (4ull << 20)
+#endif
+static constexpr uint64_t kDirectRecords = CR_DIRECT_RECORDS;
+static constexpr uint64_t kDirectBoxes = CR_DIRECT_BOXES;
+
 cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_t count, const uint64_t* firstIds,
                           const cr_camera* cam, uint64_t d_visbuffer, uint64_t d_rgba, uint64_t d_colorbuffer,
                           int32_t display, uint32_t flags, void* stream_, uint64_t resolveIdLo,
@@ -1190,8 +1205,17 @@ cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_
         cellMode = CR_REC_OUTCODES;  // cells hold 16-bit coordinates
     else if (cellMode == CR_REC_CELLS && cam->width <= 4096 && cam->height <= 4096)
         cellMode = CR_REC_CELLS32;  // 12-bit coordinates fit: half the record bytes
-    const bool direct = cellMode == CR_REC_BOXES;
-    if (direct && !refMath && !(flags & kRenderResolveOnly))
+    const bool boxes = cellMode == CR_REC_BOXES;
+    uint64_t triangles = 0;
+    for (uint32_t i = 0; i < count; i++)
+        if (instances[i].mesh < ctx->meshes.size()) triangles += ctx->meshes[instances[i].mesh].numTriangles;
+    const uint64_t directLimit = boxes ? kDirectBoxes : kDirectRecords;
+    // explicit ids may have gaps, a forced record mode is kept, and the
+    // failure-detection hook drops a copy that the direct path does not make
+    const bool mayDirect = rec == CR_CULL_AUTO && !refMath && !firstIds && count > 0 && triangles > 0 &&
+                           !(flags & kRenderResolveOnly) && ctx->cfg.debug_flags == 0;
+    bool direct = mayDirect && triangles <= directLimit;
+    if (boxes && !direct && !refMath && !(flags & kRenderResolveOnly))
         for (uint32_t i = 0; i < count; i++) {
             const uint32_t m = instances[i].mesh;
             if (m < ctx->meshes.size() && ctx->meshes[m].live) ensure_local_lists(ctx, ctx->meshes[m]);
@@ -1205,20 +1229,23 @@ cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_
         const float f = cam->proj[5];
         const float fa = f / ((float)cam->width / (float)cam->height);
         double area = 0.0, tris = 0.0;
+        bool inside = true;
         for (uint32_t r = 0; r < count; r++) {
             const MeshRec& m = ctx->meshes[instances[A.order[r]].mesh];
             A.inst[r].meshClass = classify_mesh_box(&A.worldView[16ull * r], fa, f, m.box);
             area += screen_box_area(&A.worldView[16ull * r], fa, f, cam->width, cam->height, m.box);
             tris += (double)m.numTriangles;
+            inside = inside && (A.inst[r].meshClass & CR_MESH_INSIDE);
         }
         if (tris > 0.0) pxPerTriangle = (float)(area / tris);
+        if (mayDirect && !boxes && inside && pxPerTriangle >= 0.5f) direct = true;
     }
     // frame tables, queues and counters are shared by consecutive frames,
     // which may be issued on different streams
     CR_CUDA(cudaStreamWaitEvent(stream, ctx->frameDone, 0), "stream wait");
     const uint64_t numPixels = (uint64_t)cam->width * (uint64_t)cam->height;
 
-    s = ensure_records(ctx, direct ? 0 : A.outBytes * (cellMode == CR_REC_CELLS ? 8 : cellMode == CR_REC_CELLS32 ? 4 : 1));
+    s = ensure_records(ctx, boxes || direct ? 0 : A.outBytes * (cellMode == CR_REC_CELLS ? 8 : cellMode == CR_REC_CELLS32 ? 4 : 1));
     if (s) return s;
     if (A.numItems > ctx->itemCap || A.numVChunks > ctx->chunkCap || A.numUnits > ctx->unitCap ||
         A.numChunkGroups > ctx->cgroupCap) {
@@ -1276,7 +1303,7 @@ cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_
     fp.cgroupList = ctx->cgroupList;
     // the vertex pass evaluates only the slices that hold a vertex of a drawn
     // item, when every mesh of the frame has its items' slices
-    bool stamps = !direct && !refMath && count > 0 && ctx->sliceNeed != nullptr;
+    bool stamps = !boxes && !direct && !refMath && count > 0 && ctx->sliceNeed != nullptr;
     for (const CrSegment& sg : A.seg) stamps = stamps && sg.itemSlices != nullptr;
     if (stamps) {
         if (++ctx->needStamp == 0) {  // the stamps wrapped: clear them
@@ -1288,7 +1315,9 @@ cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_
         fp.needStamp = ctx->needStamp;
     }
     ctx->lastStamps = stamps;
-    if (direct) {  // no vertex pass: no chunks to classify or evaluate
+    fp.direct = direct ? A.totalTriangles : 0;
+    ctx->lastDirect = fp.direct;
+    if (boxes || direct) {  // no vertex pass: no chunks to classify or evaluate
         fp.chunkList = nullptr;
         fp.chunkClass = nullptr;
         fp.numVChunks = 0;
@@ -1388,7 +1417,7 @@ cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_
             CR_CUDA(mark(6), "event");
             return CR_OK;
         }
-        if (raster && count && (cr_launch_cull(fp, ctx->shape, stream) || cr_launch_vertex(fp, ctx->shape, stream)))
+        if (raster && count && !fp.direct && (cr_launch_cull(fp, ctx->shape, stream) || cr_launch_vertex(fp, ctx->shape, stream)))
             return fail(CR_ERR_CUDA, "vertex-pass launch: %s", cudaGetErrorString(cudaGetLastError()));
         CR_CUDA(mark(2), "event");
         if (raster && count && cr_launch_stage1(fp, ctx->shape, stream))

@@ -362,6 +362,7 @@ cr_status render_batch(cr_context* ctx, const cr_instance* instances, uint32_t c
         fp.hugeCap = ctx->hugeCap;
         return issue_batch(fp, rp, B, sh, count, flags, stream, tev, rasterEnd);
     };
+    ctx->lastDirect = 0;
     return run_frame(ctx, flags, stream, count, A.totalTriangles * nv, issue, A.numItems, A.numVChunks);
 }
 

@@ -150,6 +150,7 @@ struct cr_context {
     uint32_t* sliceNeed = nullptr;  // per slice of chunkCap chunks: the stamp of the last
                                     // frame a drawn item used one of its vertices
     uint32_t needStamp = 0;         // the last frame's stamp (0 is never issued)
+    uint64_t lastDirect = 0;        // triangles of the last frame if it took the direct path, else 0
     bool lastStamps = false;        // the last frame's vertex pass evaluated stamped slices only
     uint64_t lastNontrivial = 0;    // stage-2 queue entries of the last frame whose counters were read
     bool countersPublished = false; // the frame being issued has its resolve copy the counters

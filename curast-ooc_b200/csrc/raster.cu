@@ -709,14 +709,15 @@ __global__ void __launch_bounds__(WARPS * 32, S1C_MIN_BLOCKS) k_s1cull(const CrF
 // (stage1_triangle: transform, culls, the tiny raster or the stage-2 queue).
 // Survivors of one item are consecutive in the list, so a warp's gathers stay
 // within a few items.  COOP: frames of pixel-sized triangles spread the
-// lanes' tiny rasters over the warp.
-template <int WARPS, bool PACKED, bool COOP>
+// lanes' tiny rasters over the warp.  DIRECT: there is no list, every triangle
+// of every instance is taken (CrFrameParams::direct).
+template <int WARPS, bool PACKED, bool COOP, bool DIRECT = false>
 __global__ void __launch_bounds__(WARPS * 32) k_s1raster(const CrFrameParams p) {
     pdl_enter();
     const int lane = threadIdx.x & 31;
     const uint64_t gw = (uint64_t)blockIdx.x * WARPS + (threadIdx.x >> 5);
     const uint64_t nw = (uint64_t)gridDim.x * WARPS;
-    const uint64_t n = min((uint64_t)p.counters[CR_CTR_SURVIVORS], p.s1Cap);
+    const uint64_t n = DIRECT ? p.direct : min((uint64_t)p.counters[CR_CTR_SURVIVORS], p.s1Cap);
     const Target tg = target_of(p);
     const float fa = tg.fa;
     for (uint64_t base = gw * 32; base < n; base += nw * 32) {
@@ -726,9 +727,19 @@ __global__ void __launch_bounds__(WARPS * 32) k_s1raster(const CrFrameParams p) 
         S1Raster ras;
         uint64_t rid = 0;
         if (j < n) {
-            const uint64_t e = __ldg(p.s1List + j);
-            inst = (uint32_t)(e >> 32);
-            tri = (uint32_t)e;
+            if constexpr (DIRECT) {  // triangle j of the frame's prefix sum over its instances
+                uint32_t hi = p.numInstances - 1;
+                while (inst < hi) {
+                    const uint32_t mid = (inst + hi + 1) >> 1;
+                    if (__ldg(&p.instances[mid].cum) <= j) inst = mid;
+                    else hi = mid - 1;
+                }
+                tri = (uint32_t)(j - __ldg(&p.instances[inst].cum));
+            } else {
+                const uint64_t e = __ldg(p.s1List + j);
+                inst = (uint32_t)(e >> 32);
+                tri = (uint32_t)e;
+            }
             const CrInstance* I = p.instances + inst;
             const GeomRef g = geom_of_t<PACKED>(I);
             const uint32_t i0 = geom_index(g, 3ull * tri + 0);
@@ -1102,6 +1113,16 @@ int cr_launch_cull(const CrFrameParams& p, const CrLaunchShape& s, void* stream)
 // survivor list) then k_s1raster (survivors -> visbuffer / stage-2 queue).
 int cr_launch_stage1(const CrFrameParams& p, const CrLaunchShape& s, void* stream) {
     if (p.numItems == 0) return 0;
+    if (p.direct) {
+        const uint64_t want = (p.direct + S1_WARPS * 32 - 1) / (S1_WARPS * 32);
+        const unsigned b = (unsigned)std::min<uint64_t>(want, (uint64_t)s.s1RasterBlocks);
+        const unsigned T = S1_WARPS * 32;
+        if (p.coopRaster)
+            return p.anyPacked ? launch_pdl(k_s1raster<S1_WARPS, true, true, true>, b, T, stream, p)
+                               : launch_pdl(k_s1raster<S1_WARPS, false, true, true>, b, T, stream, p);
+        return p.anyPacked ? launch_pdl(k_s1raster<S1_WARPS, true, false, true>, b, T, stream, p)
+                           : launch_pdl(k_s1raster<S1_WARPS, false, false, true>, b, T, stream, p);
+    }
     const uint64_t itemBlocks = (p.numItems + S1_WARPS - 1) / S1_WARPS;
     const unsigned T = S1_WARPS * 32;
     if (p.cellMode == CR_REC_BOXES) {
