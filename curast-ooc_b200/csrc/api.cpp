@@ -63,13 +63,13 @@ float det3_glm(const float* m) {
     return (x * c2[0] + y * c2[1]) + z * c2[2];
 }
 
-// The back-face proof's data of one instance (CR_BACK_DOUBLES) from its float
-// world-view matrix (column-major): R its 3x3 part, t its translation, all
-// exact in double.  e = -R^-1 t by cofactors; |det R| only when it exceeds
+// The item proofs' data of one instance (CR_PROOF_F4) from its float world-view
+// matrix (column-major) and its mesh's box: R its 3x3 part, t its translation,
+// all exact in double.  e = -R^-1 t by cofactors; |det R| only when it exceeds
 // 1e-4 of the product of the columns' 1-norms, which bounds the float
 // det3_glm's error far below it, so the mirror flag the kernels use has the
-// exact sign (else 0: no proof for this instance).
-void back_face_data(const float* wv, double* o) {
+// exact sign (else 0: no back-face proof for this instance).
+void proof_data(const float* wv, const float* box, float* o) {
     double R[3][3];
     for (int i = 0; i < 3; i++)
         for (int j = 0; j < 3; j++) R[i][j] = wv[j * 4 + i];
@@ -82,21 +82,33 @@ void back_face_data(const float* wv, double* o) {
     const double det = R[0][0] * a00 + R[0][1] * a10 + R[0][2] * a20;
     double had = 1.0, frob = 0.0, rowAbs = 0.0, tAbs = 0.0;
     for (int j = 0; j < 3; j++) had *= fabs(R[0][j]) + fabs(R[1][j]) + fabs(R[2][j]);
+    double S[3];
     for (int i = 0; i < 3; i++) {
         rowAbs = std::max(rowAbs, fabs(R[i][0]) + fabs(R[i][1]) + fabs(R[i][2]));
         tAbs = std::max(tAbs, fabs(t[i]));
-        for (int j = 0; j < 3; j++) frob += R[i][j] * R[i][j];
+        S[i] = fabs(t[i]);
+        for (int j = 0; j < 3; j++) {
+            frob += R[i][j] * R[i][j];
+            S[i] += fabs(R[i][j]) * std::max(fabs((double)box[j]), fabs((double)box[3 + j]));
+        }
     }
-    o[0] = -(a00 * t[0] + a01 * t[1] + a02 * t[2]) / det;
-    o[1] = -(a10 * t[0] + a11 * t[1] + a12 * t[2]) / det;
-    o[2] = -(a20 * t[0] + a21 * t[1] + a22 * t[2]) / det;
-    const bool ok = std::isfinite(det) && fabs(det) > 1e-4 * had && std::isfinite(o[0]) && std::isfinite(o[1]) &&
-                    std::isfinite(o[2]) && std::isfinite(tAbs) && std::isfinite(frob);
-    o[3] = ok ? fabs(det) : 0.0;
-    o[4] = sqrt(frob);
-    o[5] = rowAbs;
-    o[6] = tAbs;
-    o[7] = sqrt(o[0] * o[0] + o[1] * o[1] + o[2] * o[2]);
+    double e[3] = {-(a00 * t[0] + a01 * t[1] + a02 * t[2]) / det, -(a10 * t[0] + a11 * t[1] + a12 * t[2]) / det,
+                   -(a20 * t[0] + a21 * t[1] + a22 * t[2]) / det};
+    const bool ok = std::isfinite(det) && fabs(det) > 1e-4 * had && std::isfinite(e[0]) && std::isfinite(e[1]) &&
+                    std::isfinite(e[2]) && std::isfinite(tAbs) && std::isfinite(frob);
+    const double up = 1.0 + 1e-6, dn = 1.0 - 1e-6;  // above the rounding to float
+    for (int j = 0; j < 3; j++) o[j] = ok ? (float)e[j] : 0.0f;
+    o[3] = (float)(sqrt(e[0] * e[0] + e[1] * e[1] + e[2] * e[2]) * up);
+    o[4] = ok ? (float)(fabs(det) * dn) : 0.0f;
+    o[5] = (float)(sqrt(frob) * up);
+    o[6] = (float)(rowAbs * up);
+    o[7] = (float)(tAbs * up);
+    for (int i = 0; i < 3; i++) {
+        bool fin = std::isfinite(S[i]);
+        for (int j = 0; j < 6; j++) fin = fin && std::isfinite(box[j]);
+        o[8 + i] = fin ? (float)(S[i] * up) : INFINITY;
+    }
+    o[11] = 0.0f;
 }
 
 // glm::inverse for mat4 (libs/glm/glm/detail/func_matrix.inl:296-360)
@@ -255,7 +267,7 @@ cr_status assemble(cr_context* ctx, const cr_instance* instances, uint32_t count
         count, firstIds ? (flags | CR_RENDER_KEEP_ORDER) : flags, [&](uint32_t i) { return instances[i].mesh; },
         [&](uint32_t i) { return ctx->meshes[instances[i].mesh].numTriangles; }, A.order);
     A.inst.assign(count, CrInstance{});
-    A.back.resize((size_t)CR_BACK_DOUBLES * count);
+    A.proof.resize((size_t)CR_PROOF_F4 * 4 * count);
     A.worldView.resize(16ull * count);
     A.world.resize(16ull * count);
     A.seg.clear();
@@ -284,7 +296,7 @@ cr_status assemble(cr_context* ctx, const cr_instance* instances, uint32_t count
         float* wv = &A.worldView[16ull * r];
         mat4_mul(view, in.world, wv);  // CuRast_render.h:409
         ci.flip = det3_glm(wv) < 0.0f ? 1u : 0u;
-        back_face_data(wv, &A.back[(size_t)CR_BACK_DOUBLES * r]);
+        proof_data(wv, m.box, &A.proof[(size_t)CR_PROOF_F4 * 4 * r]);
         memcpy(&A.world[16ull * r], in.world, 64);
         // CuRast_render.h:425-433: consecutive instances of one mesh form a segment
         if (A.seg.empty() || A.seg.back().positions != m.positions || A.seg.back().indices != m.indices ||
@@ -301,7 +313,8 @@ cr_status assemble(cr_context* ctx, const cr_instance* instances, uint32_t count
             s.itemBoxes = m.itemBoxes;
             s.itemCones = m.itemCones;
             s.itemSlices = m.itemSlices;
-            s.subBoxes = m.subBoxes;
+            s.subObbs = m.subObbs;
+            s.itemObbs = m.itemObbs;
             s.localLists = m.localLists;
             s.localCounts = m.localCounts;
             s.groupBoxes = m.groupBoxes;
@@ -384,30 +397,31 @@ void ensure_bins(cr_context* ctx, uint64_t tiles) {
 cr_status launch_mesh_boxes(cr_context* ctx, MeshRec& m) {
     const size_t ib = align_up((size_t)((m.numTriangles + CR_BATCH - 1) / CR_BATCH) * 24, 256);
     const size_t cb = align_up((size_t)((m.numVertices + CR_VCHUNK - 1) / CR_VCHUNK) * 24, 256);
-    const size_t sb = align_up((size_t)((m.numTriangles + CR_SUB - 1) / CR_SUB) * 24, 256);
     const uint64_t nItems = (m.numTriangles + CR_BATCH - 1) / CR_BATCH;
     const uint64_t nChunks = (m.numVertices + CR_VCHUNK - 1) / CR_VCHUNK;
     const size_t gb = align_up((size_t)((nItems + CR_GROUP - 1) / CR_GROUP) * 24, 256);
     const size_t cgb = align_up((size_t)((nChunks + CR_GROUP - 1) / CR_GROUP) * 24, 256);
     const size_t icb = align_up((size_t)nItems * CR_CONE_FLOATS * 4, 256);
     const size_t isb = align_up((size_t)nItems * 32, 256);
+    const size_t ob = align_up((size_t)nItems * CR_OBB_F4 * 16, 256);
     if (!m.itemBoxes) {
-        cr_status s = ctx->dev_alloc((void**)&m.itemBoxes, ib + cb + sb + gb + cgb + icb + isb + 256, "mesh boxes");
+        const size_t bytes = ib + cb + gb + cgb + icb + isb + ob + 256;
+        cr_status s = ctx->dev_alloc((void**)&m.itemBoxes, bytes, "mesh boxes");
         if (s) return s;
         m.chunkBoxes = (float*)((char*)m.itemBoxes + ib);
-        m.subBoxes = (float*)((char*)m.itemBoxes + ib + cb);
-        m.groupBoxes = (float*)((char*)m.itemBoxes + ib + cb + sb);
-        m.chunkGroupBoxes = (float*)((char*)m.itemBoxes + ib + cb + sb + gb);
-        m.itemCones = (float*)((char*)m.itemBoxes + ib + cb + sb + gb + cgb);
-        m.itemSlices = (uint4*)((char*)m.itemBoxes + ib + cb + sb + gb + cgb + icb);
-        m.boxBytes = ib + cb + sb + gb + cgb + icb + isb + 256;
+        m.groupBoxes = (float*)((char*)m.itemBoxes + ib + cb);
+        m.chunkGroupBoxes = (float*)((char*)m.itemBoxes + ib + cb + gb);
+        m.itemCones = (float*)((char*)m.itemBoxes + ib + cb + gb + cgb);
+        m.itemSlices = (uint4*)((char*)m.itemBoxes + ib + cb + gb + cgb + icb);
+        m.itemObbs = (float4*)((char*)m.itemBoxes + ib + cb + gb + cgb + icb + isb);
+        m.boxBytes = bytes;
     }
-    m.meshBox = (float*)((char*)m.itemBoxes + ib + cb + sb + gb + cgb + icb + isb);
+    m.meshBox = (float*)((char*)m.itemBoxes + ib + cb + gb + cgb + icb + isb + ob);
     m.dCodec = (CrCodec*)((char*)m.meshBox + 64);
     CR_CUDA(cudaMemcpy(m.dCodec, &m.codec, sizeof(CrCodec), cudaMemcpyHostToDevice), "mesh codec");
     if (cr_launch_mesh_boxes(m.indices, m.positions, m.compressed ? m.dCodec : nullptr, m.numTriangles,
-                             m.numVertices, m.itemBoxes, m.chunkBoxes, m.subBoxes, m.meshBox, m.groupBoxes,
-                             m.chunkGroupBoxes, m.itemCones, m.itemSlices, 0))
+                             m.numVertices, m.itemBoxes, m.chunkBoxes, m.meshBox, m.groupBoxes, m.chunkGroupBoxes,
+                             m.itemCones, m.itemSlices, m.itemObbs, 0))
         return fail(CR_ERR_CUDA, "mesh box launch: %s", cudaGetErrorString(cudaGetLastError()));
     return CR_OK;
 }
@@ -421,6 +435,12 @@ cr_status build_mesh_boxes(cr_context* ctx, MeshRec& m) {
     if (cr_status s = launch_mesh_boxes(ctx, m)) return s;
     CR_CUDA(cudaDeviceSynchronize(), "mesh boxes");
     return read_mesh_box(m);
+}
+
+static void free_sub_obbs(cr_context* ctx, MeshRec& m) {
+    ctx->dev_free(m.subObbs, m.subBytes);
+    m.subObbs = nullptr;
+    m.subBytes = 0;
 }
 
 // Per-item vertex lists of an indexed mesh, built once on first use (a
@@ -449,6 +469,24 @@ void ensure_local_lists(cr_context* ctx, MeshRec& m) {
     }
 }
 
+// The oriented sub-boxes of a mesh that box-culled frames draw, built once on
+// first use (absent after a failure: the frame then draws every triangle of
+// its listed items, with the same output).
+void ensure_sub_obbs(cr_context* ctx, MeshRec& m) {
+    if (m.subTried || m.numTriangles == 0) return;
+    m.subTried = true;
+    const size_t bytes = (size_t)((m.numTriangles + CR_SUB - 1) / CR_SUB) * CR_OBB_F4 * 16;
+    if (ctx->dev_alloc((void**)&m.subObbs, bytes, "oriented sub-boxes") != CR_OK) {
+        cr_internal_set_error("");
+        m.subObbs = nullptr;
+        return;
+    }
+    m.subBytes = bytes;
+    if (cr_launch_sub_obbs(m.indices, m.positions, m.compressed ? m.dCodec : nullptr, m.numTriangles, m.subObbs, 0) ||
+        cudaDeviceSynchronize() != cudaSuccess)
+        free_sub_obbs(ctx, m);
+}
+
 void ensure_local_lists_for(cr_context* ctx, const cr_instance* instances, uint32_t count) {
     for (uint32_t i = 0; i < count; i++) {
         const uint32_t m = instances[i].mesh;
@@ -464,8 +502,8 @@ cr_status upload_frame(cr_context* ctx, const Assembled& A, cudaStream_t stream,
     const size_t oWV = align_up(oInst + n * sizeof(CrInstance), 256);
     const size_t oW = align_up(oWV + n * 64, 256);
     const size_t oSeg = align_up(oW + n * 64, 256);
-    const size_t oBack = align_up(oSeg + m * sizeof(CrSegment), 256);
-    const size_t total = align_up(oBack + n * CR_BACK_DOUBLES * 8, 256);
+    const size_t oProof = align_up(oSeg + m * sizeof(CrSegment), 256);
+    const size_t total = align_up(oProof + n * CR_PROOF_F4 * 16, 256);
     // the previous frame's copy must have left the staging buffer
     CR_CUDA(cudaEventSynchronize(ctx->frameCopied), "frame staging");
     if (total > ctx->hFrameCap) {
@@ -490,7 +528,7 @@ cr_status upload_frame(cr_context* ctx, const Assembled& A, cudaStream_t stream,
     memcpy(h + oWV, A.worldView.data(), n * 64);
     memcpy(h + oW, A.world.data(), n * 64);
     memcpy(h + oSeg, A.seg.data(), m * sizeof(CrSegment));
-    memcpy(h + oBack, A.back.data(), n * CR_BACK_DOUBLES * 8);
+    memcpy(h + oProof, A.proof.data(), n * CR_PROOF_F4 * 16);
     CR_CUDA(cudaMemcpyAsync(ctx->dFrame, h, total, cudaMemcpyHostToDevice, stream), "frame table upload");
     CR_CUDA(cudaEventRecord(ctx->frameCopied, stream), "frame event");
     char* d = (char*)ctx->dFrame;
@@ -498,7 +536,7 @@ cr_status upload_frame(cr_context* ctx, const Assembled& A, cudaStream_t stream,
     fp.world_view = (const float4*)(d + oWV);
     fp.world = (const float4*)(d + oW);
     fp.segments = (const CrSegment*)(d + oSeg);
-    fp.instBack = (const double*)(d + oBack);
+    fp.instProof = (const float4*)(d + oProof);
     fp.numInstances = (uint32_t)n;
     fp.numSegments = (uint32_t)m;
     fp.numItems = A.numItems;
@@ -739,6 +777,7 @@ cr_status cr_destroy(cr_context* ctx) {
         }
         if (m.itemBoxes) cudaFree(m.itemBoxes);
         if (m.localLists) cudaFree(m.localLists);
+        if (m.subObbs) cudaFree(m.subObbs);
     }
     if (ctx->itemList) cudaFree(ctx->itemList);
     if (ctx->outcodes) cudaFree(ctx->outcodes);
@@ -1093,6 +1132,7 @@ cr_status cr_mesh_destroy(cr_context* ctx, uint32_t mesh) {
     if (m.owned) free_mesh_arrays(ctx, m);
     ctx->dev_free(m.itemBoxes, m.boxBytes);
     ctx->dev_free(m.localLists, m.localBytes);
+    ctx->dev_free(m.subObbs, m.subBytes);
     m = MeshRec{};
     return CR_OK;
 }
@@ -1107,6 +1147,8 @@ cr_status cr_mesh_refresh(cr_context* ctx, uint32_t mesh) {
     m.localCounts = nullptr;
     m.localBytes = 0;
     m.localTried = false;
+    free_sub_obbs(ctx, m);  // likewise
+    m.subTried = false;
     return build_mesh_boxes(ctx, m);
 }
 
@@ -1218,7 +1260,7 @@ cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_
     if (boxes && !direct && !refMath && !(flags & kRenderResolveOnly))
         for (uint32_t i = 0; i < count; i++) {
             const uint32_t m = instances[i].mesh;
-            if (m < ctx->meshes.size() && ctx->meshes[m].live) ensure_local_lists(ctx, ctx->meshes[m]);
+            if (m < ctx->meshes.size() && ctx->meshes[m].live) ensure_sub_obbs(ctx, ctx->meshes[m]);
         }
 
     Assembled A;

@@ -43,7 +43,7 @@ struct MeshRec {
     // hierarchical-cull boxes (library-owned, also for borrowed meshes)
     float* itemBoxes = nullptr;   // per CR_BATCH triangles
     float* chunkBoxes = nullptr;  // per CR_VCHUNK vertices
-    float* subBoxes = nullptr;    // per CR_SUB triangles
+    float4* itemObbs = nullptr;   // per item, CR_OBB_F4
     float* groupBoxes = nullptr;  // per CR_GROUP item boxes
     float* chunkGroupBoxes = nullptr;  // per CR_GROUP chunk boxes
     float* itemCones = nullptr;   // per CR_BATCH triangles: CR_CONE_FLOATS normal cone
@@ -60,6 +60,11 @@ struct MeshRec {
     uint32_t* localCounts = nullptr;
     size_t localBytes = 0;
     bool localTried = false;
+    // oriented sub-boxes of box-culled frames (CR_OBB_F4 per CR_SUB triangles),
+    // built on first use
+    float4* subObbs = nullptr;
+    size_t subBytes = 0;
+    bool subTried = false;
 };
 
 void mat4_mul(const float* a, const float* b, float* out);  // glm order
@@ -102,7 +107,7 @@ struct Assembled {
     std::vector<float> worldView;   // 16 per instance
     std::vector<float> world;       // 16 per instance
     std::vector<CrSegment> seg;
-    std::vector<double> back;       // CR_BACK_DOUBLES per instance (back-face proof)
+    std::vector<float> proof;       // CR_PROOF_F4 float4 per instance (item proofs)
     uint64_t totalTriangles = 0;
     uint64_t numItems = 0;
     uint64_t outBytes = 0;     // vertex-pass record slots of all instances
@@ -224,6 +229,8 @@ void free_mesh_arrays(cr_context* ctx, MeshRec& m);
 cr_status ensure_records(cr_context* ctx, uint64_t bytes);
 // Builds a mesh's per-item vertex lists on first use (absent on failure).
 void ensure_local_lists(cr_context* ctx, MeshRec& m);
+// Builds a mesh's oriented sub-boxes on first use (absent on failure).
+void ensure_sub_obbs(cr_context* ctx, MeshRec& m);
 // Vertex lists for every mesh of an instance list (batched frames).
 void ensure_local_lists_for(cr_context* ctx, const cr_instance* instances, uint32_t count);
 

@@ -127,7 +127,8 @@ struct alignas(16) CrSegment {
     uint32_t flags;             // bit 0: index array 16-byte aligned (TMA tiles)
     uint64_t itemBase;          // first stage-1 work item of this segment
     const float* itemBoxes;     // per CR_BATCH triangles: box of their vertices (or nullptr)
-    const float* subBoxes;      // per CR_SUB triangles: box of their vertices (or nullptr)
+    const float4* subObbs;      // per CR_SUB triangles, CR_OBB_F4: oriented box of their
+                                // vertices (box-culled frames; or nullptr)
     const uint8_t* localLists;  // per item, CR_LOCAL_BYTES (or nullptr)
     const uint32_t* localCounts;  // per item, distinct vertices or CR_LOCAL_NONE
     CrCodec codec;              // compressed meshes (flags bit 0 is then clear)
@@ -136,8 +137,14 @@ struct alignas(16) CrSegment {
     const float* itemCones;     // per item, CR_CONE_FLOATS: its triangles' normal cone (or nullptr)
     const uint4* itemSlices;    // per item, two: the vertex-pass slices its vertices lie in
                                 // (CR_VSLICE; or nullptr)
+    const float4* itemObbs;     // per item, CR_OBB_F4: oriented box of its vertices (or nullptr)
+    uint64_t pad;
 };
-static_assert(sizeof(CrSegment) == 144, "CrSegment layout");
+static_assert(sizeof(CrSegment) == 160, "CrSegment layout");
+// An oriented box, twelve floats: the centre c, then three axes A_j; it holds
+// every vertex p of its triangles as p = c + sum t_j A_j with |t_j| <= 1 in exact
+// arithmetic (NaN: a non-finite vertex, proves nothing).
+#define CR_OBB_F4 3
 // Per-item normal cone (object space), for the back-face proof of the frame
 // cull: axis m (float xyz, unit length within 2^-23), cosT (every triangle's
 // unit normal u has u . m / |m| >= cosT; below -1: no cone), nMin (every
@@ -145,10 +152,14 @@ static_assert(sizeof(CrSegment) == 144, "CrSegment layout");
 // |pc - pa| <= edge), sinT >= sqrt(1 - cosT^2), and r >= half the diagonal of
 // the item's box.
 #define CR_CONE_FLOATS 8
-// Per-instance data of the back-face proof (CrFrameParams::instBack, doubles):
-// the camera in object space (e = -R^-1 t, 3), |det R| (0: no proof), the
-// Frobenius norm of R, max_i sum_j |R_ij|, max_i |t_i|, and |e|.
-#define CR_BACK_DOUBLES 8
+// Per-instance data of the item proofs (CrFrameParams::instProof, float4), from
+// the world-view matrix [R | t]:
+//   [0] the camera in object space e = -R^-1 t, |e|
+//   [1] |det R| rounded down (0: no back-face proof), and rounded up: the
+//       Frobenius norm of R, max_i sum_j |R_ij|, max_i |t_i|
+//   [2] rounded up, for x, y, z: sum_j |R_ij| max|p_j| + |t_i| over the mesh's
+//       box (infinite where it is not finite: no sample-miss proof)
+#define CR_PROOF_F4 3
 
 struct alignas(16) CrTile {     // HugeTriangle, HostDeviceInterface.h:254-259
     int32_t instance;           // instance | view << 26 (view 0 in single-view frames)
@@ -270,9 +281,8 @@ struct CrFrameParams {
     // counted in counters[CR_CTR_SURVIVORS], at most s1Cap
     uint64_t* s1List;
     uint64_t s1Cap;
-    // CR_BACK_DOUBLES per instance for the item cull's back-face proof, or
-    // nullptr (no proof)
-    const double* instBack;
+    // CR_PROOF_F4 per instance for the item proofs, or nullptr (no proofs)
+    const float4* instProof;
     // record-culled frames: per vertex-pass slice (CrInstance::vchunkBase *
     // CR_VCHUNK / CR_VSLICE + slice), needStamp when a drawn item uses one of
     // its vertices (k_stamp, from CrSegment::itemSlices, after the item cull);
@@ -383,16 +393,18 @@ int cr_launch_ref_raster(const CrFrameParams& p, void* stream);
 int cr_launch_ref_raster_nofma(const CrFrameParams& p, void* stream);
 
 // Mesh preparation (meshprep.cu): the box of the vertices of every CR_BATCH
-// and every CR_SUB consecutive triangles and of every CR_VCHUNK consecutive
-// vertices (a box
+// consecutive triangles and of every CR_VCHUNK consecutive vertices (a box
 // with a non-finite position is NaN and culls nothing).
 // `codec`: device copy of a compressed mesh's codec, or nullptr.
 // itemCones: per item CR_CONE_FLOATS (or nullptr); itemSlices: per item two
 // uint4 (CrSegment::itemSlices, or nullptr).
 int cr_launch_mesh_boxes(const uint32_t* indices, const float* positions, const CrCodec* codec,
                          uint32_t numTriangles, uint32_t numVertices, float* itemBoxes, float* chunkBoxes,
-                         float* subBoxes, float* meshBox, float* groupBoxes, float* chunkGroupBoxes,
-                         float* itemCones, uint4* itemSlices, void* stream);
+                         float* meshBox, float* groupBoxes, float* chunkGroupBoxes, float* itemCones,
+                         uint4* itemSlices, float4* itemObbs, void* stream);
+// The oriented box (CR_OBB_F4) of every CR_SUB consecutive triangles.
+int cr_launch_sub_obbs(const uint32_t* indices, const float* positions, const CrCodec* codec, uint32_t numTriangles,
+                       float4* subObbs, void* stream);
 // Per-item vertex lists of an indexed mesh (see CR_LOCAL_BYTES).
 int cr_launch_local_lists(const uint32_t* indices, const CrCodec* codec, uint32_t numTriangles, uint8_t* lists,
                           uint32_t* counts, void* stream);

@@ -3,8 +3,8 @@
 //
 //   item boxes   one per CR_BATCH (128) consecutive triangles: the box of
 //                every vertex those triangles reference (a stage-1 work item)
-//   sub-boxes    one per CR_SUB (16) consecutive triangles, for the sample-miss
-//                proof of box_misses_samples
+//   oriented     one per item and (box-culled frames) per CR_SUB (16) consecutive
+//   boxes        triangles, for the sample-miss proof of obb_misses_samples
 //   chunk boxes  one per CR_VCHUNK (1024) consecutive vertices (a vertex-pass
 //                chunk)
 //   group boxes  one per CR_GROUP (32) consecutive item boxes and one per 32
@@ -234,35 +234,167 @@ __global__ void __launch_bounds__(256) k_item_cones(const uint32_t* idx, const f
     }
 }
 
-// Half a warp per sub-box: lane t of the half is its triangle t.
-__global__ void __launch_bounds__(256) k_sub_boxes(const uint32_t* idx, const float* pos, const CrCodec* codec,
-                                                   uint32_t nT, float* boxes) {
-    const int lane = threadIdx.x & 31;
+// The oriented box (CR_OBB_F4) of the vertices of LANES * R consecutive
+// triangles, R per lane: 32 x 4 for an item, 16 x 1 for a sub-box.  Axes: the sum of the unit normals, and the
+// principal direction of the vertices across it (mesh items are mostly thin
+// strips of a surface, whose object-space boxes are loose: on the 1M-triangle
+// displaced sphere 26 % of the items of a random instance survive the
+// sample-miss proof with axis-aligned boxes, 17 % with these), or the object's
+// axes where that box has the smaller surface.  Extents are measured in
+// double along the double axes.
+//
+// The stored floats contain the exact box: rounding the centre and the axes
+// moves a point of it by at most 2^-23 (|c| + h0 + h1 + h2) in any direction,
+// and each half extent is enlarged by 2^-20 of itself plus 2^-21 of that sum.
+template <int LANES, int R>
+__global__ void __launch_bounds__(256) k_obbs(const uint32_t* idx, const float* pos, const CrCodec* codec, uint32_t nT,
+                                              float4* obbs) {
+    constexpr uint32_t T = LANES * R;
+    const int lane = threadIdx.x & 31, gl = lane & (LANES - 1);
     const GeomRef g = geom_from(pos, idx, codec);
-    const int half = lane >> 4, hl = lane & 15;
-    static_assert(CR_SUB == 16, "half-warp per sub-box");
-    const uint32_t nSub = (nT + CR_SUB - 1) / CR_SUB;
-    const uint32_t nPairs = (nSub + 1) / 2;
-    for (uint32_t b = blockIdx.x * 8 + (threadIdx.x >> 5); b < nPairs; b += gridDim.x * 8) {
-        const uint32_t sb = 2 * b + half;
-        float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-        bool bad = false;
-        const uint32_t t = sb * CR_SUB + hl;
-        if (sb < nSub && t < nT)
-            for (int k = 0; k < 3; ++k) {
-                extend(lo, hi, bad, g, geom_index(g, 3ull * t + k));
-            }
+    const uint32_t nGroups = (nT + T - 1) / T;
+    const uint32_t perBlock = 256 / LANES;
+    auto sum = [](float v) {
 #pragma unroll
-        for (int d = 8; d >= 1; d >>= 1)
+        for (int d = LANES / 2; d >= 1; d >>= 1) v += __shfl_xor_sync(FULL, v, d);
+        return v;
+    };
+    auto least = [](double v) {
+#pragma unroll
+        for (int d = LANES / 2; d >= 1; d >>= 1) v = fmin(v, __shfl_xor_sync(FULL, v, d));
+        return v;
+    };
+    // whole warps loop together: groups past the end hold no triangle
+    for (uint32_t b0 = blockIdx.x * perBlock; b0 < nGroups; b0 += gridDim.x * perBlock) {
+        const uint32_t b = b0 + threadIdx.x / LANES;
+        float q[R][3][3];
+        bool live[R];
+        bool bad = false;
+        float nx = 0.0f, ny = 0.0f, nz = 0.0f;
+        double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const uint64_t t = (uint64_t)b * T + r * LANES + gl;
+            live[r] = t < nT;
+            if (!live[r]) continue;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                geom_pos(g, geom_index(g, 3ull * t + k), q[r][k][0], q[r][k][1], q[r][k][2]);
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    bad |= !isfinite(q[r][k][j]);
+                    lo[j] = fmin(lo[j], (double)q[r][k][j]);
+                    hi[j] = fmax(hi[j], (double)q[r][k][j]);
+                }
+            }
+            const float u0 = q[r][1][0] - q[r][0][0], u1 = q[r][1][1] - q[r][0][1], u2 = q[r][1][2] - q[r][0][2];
+            const float v0 = q[r][2][0] - q[r][0][0], v1 = q[r][2][1] - q[r][0][1], v2 = q[r][2][2] - q[r][0][2];
+            const float x = u1 * v2 - u2 * v1, y = u2 * v0 - u0 * v2, z = u0 * v1 - u1 * v0;
+            const float l2 = x * x + y * y + z * z;
+            if (l2 > 0.0f && l2 < INFINITY) {
+                const float s = rsqrtf(l2);
+                nx += x * s, ny += y * s, nz += z * s;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            lo[j] = least(lo[j]);
+            hi[j] = -least(-hi[j]);
+        }
+        nx = sum(nx), ny = sum(ny), nz = sum(nz);
+        // any frame will do for the containment; a good one for tightness
+        double m[3] = {nx, ny, nz};
+        double ml = sqrt(m[0] * m[0] + m[1] * m[1] + m[2] * m[2]);
+        if (!(ml > 1e-6)) m[0] = m[1] = 0.0, m[2] = ml = 1.0;
+        m[0] /= ml, m[1] /= ml, m[2] /= ml;
+        // b1, b2: a basis of the plane across m
+        double b1[3];
+        if (fabs(m[0]) < 0.6) b1[0] = 0.0, b1[1] = m[2], b1[2] = -m[1];
+        else b1[0] = -m[2], b1[1] = 0.0, b1[2] = m[0];
+        const double bl = 1.0 / sqrt(b1[0] * b1[0] + b1[1] * b1[1] + b1[2] * b1[2]);
+        b1[0] *= bl, b1[1] *= bl, b1[2] *= bl;
+        const double b2[3] = {m[1] * b1[2] - m[2] * b1[1], m[2] * b1[0] - m[0] * b1[2], m[0] * b1[1] - m[1] * b1[0]};
+        const double mid[3] = {0.5 * (lo[0] + hi[0]), 0.5 * (lo[1] + hi[1]), 0.5 * (lo[2] + hi[2])};
+        const float scale = (float)(1.0 / (fmax(hi[0] - lo[0], fmax(hi[1] - lo[1], hi[2] - lo[2])) + 1e-300));
+        float n = 0.0f, sx = 0.0f, sy = 0.0f, xx = 0.0f, xy = 0.0f, yy = 0.0f;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if (!live[r]) continue;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const double d[3] = {q[r][k][0] - mid[0], q[r][k][1] - mid[1], q[r][k][2] - mid[2]};
+                const float x = (float)(d[0] * b1[0] + d[1] * b1[1] + d[2] * b1[2]) * scale;
+                const float y = (float)(d[0] * b2[0] + d[1] * b2[1] + d[2] * b2[2]) * scale;
+                n += 1.0f, sx += x, sy += y, xx += x * x, xy += x * y, yy += y * y;
+            }
+        }
+        n = sum(n), sx = sum(sx), sy = sum(sy), xx = sum(xx), xy = sum(xy), yy = sum(yy);
+        const float in = 1.0f / fmaxf(n, 1.0f);
+        float th = 0.5f * atan2f(2.0f * (xy - sx * sy * in), (xx - sx * sx * in) - (yy - sy * sy * in));
+        if (!isfinite(th)) th = 0.0f;
+        double ct = cosf(th), sn = sinf(th);
+        const double cl = 1.0 / sqrt(ct * ct + sn * sn);
+        ct *= cl, sn *= cl;
+        double ax[3][3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            ax[0][j] = ct * b1[j] + sn * b2[j];
+            ax[1][j] = ct * b2[j] - sn * b1[j];
+            ax[2][j] = m[j];
+        }
+        double pl[3] = {INFINITY, INFINITY, INFINITY}, ph[3] = {-INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if (!live[r]) continue;
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    const double x = q[r][k][0] * ax[j][0] + q[r][k][1] * ax[j][1] + q[r][k][2] * ax[j][2];
+                    pl[j] = fmin(pl[j], x);
+                    ph[j] = fmax(ph[j], x);
+                }
+        }
+        double h[3], a[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            pl[j] = least(pl[j]);
+            ph[j] = -least(-ph[j]);
+            h[j] = 0.5 * (ph[j] - pl[j]);
+            a[j] = 0.5 * (hi[j] - lo[j]);
+        }
+        double c[3];
+        if (a[0] * a[1] + a[1] * a[2] + a[2] * a[0] <= h[0] * h[1] + h[1] * h[2] + h[2] * h[0]) {
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
-                lo[j] = fminf(lo[j], __shfl_xor_sync(FULL, lo[j], d));
-                hi[j] = fmaxf(hi[j], __shfl_xor_sync(FULL, hi[j], d));
+                c[j] = mid[j];
+                h[j] = a[j];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) ax[j][k] = j == k ? 1.0 : 0.0;
             }
-        const unsigned anyBad = __ballot_sync(FULL, bad);
-        bad = (anyBad >> (16 * half)) & 0xffffu;
-        if (sb < nSub && hl < 6)
-            boxes[6ull * sb + hl] = bad ? __int_as_float(0x7fffffff) : (hl < 3 ? lo[hl] : hi[hl - 3]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                c[k] = 0.5 * ((pl[0] + ph[0]) * ax[0][k] + (pl[1] + ph[1]) * ax[1][k] + (pl[2] + ph[2]) * ax[2][k]);
+        }
+        const unsigned badM = __ballot_sync(FULL, bad);
+        const bool anyBad = ((badM >> (lane & ~(LANES - 1))) & (LANES == 32 ? FULL : (1u << (LANES & 31)) - 1u)) != 0u;
+        const double slack = 4.76837158203125e-07 *  // 2^-21
+                                 (fmax(fabs(c[0]), fmax(fabs(c[1]), fabs(c[2]))) + h[0] + h[1] + h[2]) +
+                             1e-37;
+        if (gl == 0 && b < nGroups) {
+            float o[12];
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                o[j] = anyBad ? __int_as_float(0x7fffffff) : (float)c[j];
+                const double hj = h[j] * 1.00000095367431640625 + slack;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) o[3 + 3 * j + k] = (float)(ax[j][k] * hj);
+            }
+#pragma unroll
+            for (int j = 0; j < CR_OBB_F4; ++j)
+                obbs[(uint64_t)CR_OBB_F4 * b + j] = make_float4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+        }
     }
 }
 
@@ -438,19 +570,27 @@ int cr_launch_local_lists(const uint32_t* indices, const CrCodec* codec, uint32_
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
+int cr_launch_sub_obbs(const uint32_t* indices, const float* positions, const CrCodec* codec, uint32_t numTriangles,
+                       float4* subObbs, void* stream) {
+    const uint32_t blocks = ((numTriangles + CR_SUB - 1) / CR_SUB + 15) / 16;
+    if (!blocks) return 0;
+    k_obbs<CR_SUB, 1><<<blocks < 148 * 16 ? blocks : 148 * 16, 256, 0, (cudaStream_t)stream>>>(
+        indices, positions, codec, numTriangles, subObbs);
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
 int cr_launch_mesh_boxes(const uint32_t* indices, const float* positions, const CrCodec* codec,
                          uint32_t numTriangles, uint32_t numVertices, float* itemBoxes, float* chunkBoxes,
-                         float* subBoxes, float* meshBox, float* groupBoxes, float* chunkGroupBoxes,
-                         float* itemCones, uint4* itemSlices, void* stream) {
+                         float* meshBox, float* groupBoxes, float* chunkGroupBoxes, float* itemCones,
+                         uint4* itemSlices, float4* itemObbs, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     const uint32_t nItems = (numTriangles + CR_BATCH - 1) / CR_BATCH;
     const uint32_t nChunks = (numVertices + CR_VCHUNK - 1) / CR_VCHUNK;
     if (nItems) k_item_boxes<<<(nItems + 7) / 8 < 148 * 16 ? (nItems + 7) / 8 : 148 * 16, 256, 0, st>>>(
         indices, positions, codec, numTriangles, itemBoxes);
-    const uint32_t nPairs = ((numTriangles + CR_SUB - 1) / CR_SUB + 1) / 2;
-    if (nPairs && subBoxes)
-        k_sub_boxes<<<(nPairs + 7) / 8 < 148 * 16 ? (nPairs + 7) / 8 : 148 * 16, 256, 0, st>>>(
-            indices, positions, codec, numTriangles, subBoxes);
+    if (nItems && itemObbs)
+        k_obbs<32, 4><<<(nItems + 7) / 8 < 148 * 16 ? (nItems + 7) / 8 : 148 * 16, 256, 0, st>>>(
+            indices, positions, codec, numTriangles, itemObbs);
     if (nChunks) k_chunk_boxes<<<(nChunks + 7) / 8 < 148 * 16 ? (nChunks + 7) / 8 : 148 * 16, 256, 0, st>>>(
         positions, codec, numVertices, chunkBoxes);
     const uint32_t nGroups = (nItems + CR_GROUP - 1) / CR_GROUP;

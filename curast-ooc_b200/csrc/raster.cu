@@ -154,8 +154,8 @@ __global__ void __launch_bounds__(THREADS, VX_MIN_BLOCKS) k_vertex(const CrFrame
 //                 cone, tv.cu:168-188), or whose box is wholly behind or
 //                 beyond one side, has every triangle of the item culled by
 //                 the reference's own tests (tv.cu:110-119); so has one whose
-//                 box provably misses every sample (box_misses_samples,
-//                 tv.cu:153-158).  Items with a surviving instance are
+//                 oriented box provably misses every sample
+//                 (obb_misses_samples, tv.cu:153-158).  Items with a surviving instance are
 //                 appended (warp-aggregated) with the mask of those instances.
 // Skipping what the boxes prove cannot change the visbuffer; the two levels
 // let a frame whose camera sees a small part of a large mesh classify a box
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(THREADS, 3) k_cull(const CrFrameParams p) {
     }
     if (!p.itemList) return;
     // items of the listed units, a lane per item
-    const double invW = 1.0 / (double)p.W, invH = 1.0 / (double)p.H;
+    const float Wf = (float)p.W, Hf = (float)p.H;
     const uint64_t nUnits = min((uint64_t)p.counters[CR_CTR_UNITS], p.numUnits);
     for (uint64_t k = gw; k < nUnits; k += nw) {
         const uint2 e = __ldg(&p.unitList[k]);
@@ -337,30 +337,39 @@ __global__ void __launch_bounds__(THREADS, 3) k_cull(const CrFrameParams p) {
         uint32_t mask = 0;
         if (valid) {
             const float* boxes = ldg_ptr(&sg->itemBoxes);
-            const float* cones = p.instBack ? ldg_ptr(&sg->itemCones) : nullptr;
+            const float4* cones = p.instProof ? reinterpret_cast<const float4*>(ldg_ptr(&sg->itemCones)) : nullptr;
+            const float4* obbs = p.instProof ? ldg_ptr(&sg->itemObbs) : nullptr;
             if (!boxes) {
                 mask = alive | (insideU << 16);
             } else {
                 float blo[3], bhi[3];
                 load_box(boxes + 6ull * batch, blo, bhi);
+                const V3 mid = {0.5f * (blo[0] + bhi[0]), 0.5f * (blo[1] + bhi[1]), 0.5f * (blo[2] + bhi[2])};
+                float4 c0 = make_float4(0.0f, 0.0f, 0.0f, -2.0f), c1 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (cones) {
+                    c0 = __ldg(cones + 2ull * batch);
+                    c1 = __ldg(cones + 2ull * batch + 1);
+                }
+                Obb ob;
+                if (obbs) ob = load_obb(obbs + (uint64_t)CR_OBB_F4 * batch);
                 for (uint32_t rest = alive; rest; rest &= rest - 1) {
                     const uint32_t slot = __ffs(rest) - 1;
                     const uint32_t inst = ib + slot;
-                    // every triangle of the item faces away from the camera
-                    if (cones && item_back_facing(p.instBack + (uint64_t)CR_BACK_DOUBLES * inst,
-                                                  cones + (uint64_t)CR_CONE_FLOATS * batch, blo, bhi))
-                        continue;
-                    const Mat M = load_mat(p.world_view + 4ull * inst);
                     bool inside = ((insideU >> slot) & 1u) != 0u;
+                    if (p.instProof) {
+                        const Proof P = load_proof(p, inst);
+                        // every triangle of the item faces away from the camera
+                        if (item_back_facing(P, c0, c1, mid)) continue;
+                        // the sample-miss proof of the whole item (for every
+                        // record mode: it culls items of sub-pixel triangles
+                        // before their indices are read)
+                        if (obbs && obb_misses_samples(P, fa, p.f, Wf, Hf, ob)) continue;
+                    }
                     if (!inside) {
-                        const uint32_t c = classify_box(M, fa, p.f, blo, bhi);
+                        const uint32_t c = classify_box(load_mat(p.world_view + 4ull * inst), fa, p.f, blo, bhi);
                         if (c & CR_OC_MASK) continue;
                         inside = (c & CH_INSIDE) != 0u;
                     }
-                    // the sample-miss proof of the whole item box (for every
-                    // record mode: it culls items of sub-pixel triangles before
-                    // their indices are read)
-                    if (box_misses_samples(M, fa, p.f, p.W, p.H, invW, invH, blo, bhi)) continue;
                     // bit 16 + slot: every vertex of the item is in front of
                     // the camera and inside every side (no chunk it touches
                     // can have been classified culled)
@@ -514,25 +523,17 @@ __device__ __forceinline__ void gather_culls(const CrFrameParams& p, uint32_t in
 }
 
 // What the ring slot of an item holds: its index tile (a full 128-triangle
-// tile of a 16-byte aligned index array), in box-culled frames its vertex-list
-// block when it has one, or nothing (tails and non-indexed meshes, read
-// directly).
+// tile of a 16-byte aligned index array) or nothing (tails and non-indexed
+// meshes, read directly).
 struct TileSrc {
     const void* src;
     uint32_t bytes;
-    bool local;
 };
 
-template <bool BOXES>
-__device__ __forceinline__ TileSrc tile_source(const CrSegment* sg, uint32_t batch, bool allowLocal) {
-    if (BOXES && allowLocal) {
-        const uint32_t* lc = ldg_ptr(&sg->localCounts);
-        if (lc && __ldg(lc + batch) <= CR_LOCAL_MAX)
-            return TileSrc{ldg_ptr(&sg->localLists) + (uint64_t)batch * CR_LOCAL_BYTES, CR_LOCAL_BYTES, true};
-    }
+__device__ __forceinline__ TileSrc tile_source(const CrSegment* sg, uint32_t batch) {
     if (item_uses_tma(sg, batch))
-        return TileSrc{ldg_ptr(&sg->indices) + (uint64_t)batch * (CR_BATCH * 3), CR_BATCH * 12, false};
-    return TileSrc{nullptr, 0, false};
+        return TileSrc{ldg_ptr(&sg->indices) + (uint64_t)batch * (CR_BATCH * 3), CR_BATCH * 12};
+    return TileSrc{nullptr, 0};
 }
 
 // Warp-aggregated append of one stage-1 triangle per set lane to the
@@ -594,7 +595,7 @@ __global__ void __launch_bounds__(WARPS * 32, S1C_MIN_BLOCKS) k_s1cull(const CrF
         const uint64_t pk = gw + (uint64_t)s * nw;
         if (pk >= nItems) break;
         const Item it = decode_item(p, item_at(pk));
-        const TileSrc ts = tile_source<false>(p.segments + it.seg, it.batch, false);
+        const TileSrc ts = tile_source(p.segments + it.seg, it.batch);
         if (ts.src) {
             pending |= 1u << s;
             // failure-detection test hook: the first copy is never issued, so
@@ -651,7 +652,7 @@ __global__ void __launch_bounds__(WARPS * 32, S1C_MIN_BLOCKS) k_s1cull(const CrF
             const uint64_t npk = pk + (uint64_t)STAGES * nw;
             if (npk < nItems) {
                 const Item nt = decode_item(p, item_at(npk));
-                const TileSrc ns = tile_source<false>(p.segments + nt.seg, nt.batch, false);
+                const TileSrc ns = tile_source(p.segments + nt.seg, nt.batch);
                 if (ns.src) {
                     pending |= bit;
                     if (lane == 0) {
@@ -767,19 +768,19 @@ __global__ void __launch_bounds__(WARPS * 32) k_s1raster(const CrFrameParams p) 
 }
 
 // Box-culled frames (some mesh drawn more than once: no per-vertex records).
-// Persistent warps over the work items; per item a warp waits for the
-// item's vertex-list block (or its index tile) in the TMA ring, then per
-// instance decides which of its triangles can be culled without positions,
-// queues the others across the item's instances in a per-warp ring and runs
-// the reference's full per-triangle path (stage1_triangle) on them 32 at a
-// time.
-//   vertex list   the item's distinct vertices (at most 256) get cell
-//                 records in shared memory per instance, the same records
-//                 the vertex pass would write; each triangle reads its three
-//                 from there
-//   no list       sub-box proofs of the sample-miss cull, one per
-//                 (instance, 16 triangles), spread over the lanes
-// Nontrivial triangles are appended with one atomic per warp (ballot / popc).
+// Persistent warps over the work items; per item a warp waits for the item's
+// index tile in the TMA ring while it proves, for every live instance and
+// every CR_SUB triangles of the item (a lane per pair), that their oriented box
+// misses every sample; the triangles of the other pairs run through the
+// reference's full path (stage1_triangle), two pairs at a time.  Nontrivial
+// triangles are appended with one atomic per warp (ballot / popc).
+//
+// Issue-bound.  Small instances of dense meshes are the frames that come here,
+// and almost every triangle in them misses every sample: of the 128 triangles of
+// a listed (item, instance) pair of 3000 x 1M-triangle spheres about 40 are left
+// by the sub-box proofs (3 of 8 boxes, 22 issue slots a pair), where cell records of
+// the item's 160 distinct vertices cost about 900 slots a pair.  Stage 1 of that
+// frame (with the oriented item boxes) went from 8.66 to 4.68 ms.
 #ifndef CR_S1_BOXES_MIN_BLOCKS
 #define CR_S1_BOXES_MIN_BLOCKS 3
 #endif
@@ -789,17 +790,12 @@ template <int WARPS, bool PACKED>
 __global__ void __launch_bounds__(WARPS * 32, CR_S1_BOXES_MIN_BLOCKS) k_stage1(const CrFrameParams p) {
     pdl_enter();
     constexpr int STAGES = 2;
-    static_assert(CR_LOCAL_BYTES <= CR_BATCH * 12, "a vertex-list block fits a ring slot");
     __shared__ __align__(128) uint32_t s_idx[WARPS][STAGES][CR_BATCH * 3];
     __shared__ __align__(8) uint64_t s_bar[WARPS][STAGES];
-    __shared__ uint16_t s_ring[WARPS][S1_RING];
-    __shared__ __align__(16) uint32_t s_rec[WARPS][CR_LOCAL_MAX];
     const int lane = threadIdx.x & 31;
     const int w = threadIdx.x >> 5;
     const uint64_t gw = (uint64_t)blockIdx.x * WARPS + w;
     const uint64_t nw = (uint64_t)gridDim.x * WARPS;
-    // shared-memory cell records hold 12-bit pixel cells
-    const bool lists = p.W <= 4096 && p.H <= 4096;
 
     if (lane == 0) {
         for (int s = 0; s < STAGES; ++s) mbar_init(&s_bar[w][s], 1);
@@ -817,7 +813,7 @@ __global__ void __launch_bounds__(WARPS * 32, CR_S1_BOXES_MIN_BLOCKS) k_stage1(c
         const uint64_t pk = gw + (uint64_t)s * nw;
         if (pk >= nItems) break;
         const Item it = decode_item(p, item_at(pk));
-        const TileSrc ts = tile_source<true>(p.segments + it.seg, it.batch, lists);
+        const TileSrc ts = tile_source(p.segments + it.seg, it.batch);
         if (ts.src) {
             pending |= 1u << s;
             const bool drop = (p.debugFlags & 1u) && gw == 0 && s == 0;
@@ -826,9 +822,8 @@ __global__ void __launch_bounds__(WARPS * 32, CR_S1_BOXES_MIN_BLOCKS) k_stage1(c
     }
     __syncwarp();
 
-    const float fa = p.f / p.aspect;
+    const Target tg = target_of(p);
     const float Wf = (float)p.W, Hf = (float)p.H;
-    const float Wm1 = (float)(p.W - 1), Hm1 = (float)(p.H - 1);
     uint32_t parity = 0;
     uint32_t k = 0;
     for (uint64_t pk = gw; pk < nItems; pk += nw, ++k) {
@@ -840,10 +835,36 @@ __global__ void __launch_bounds__(WARPS * 32, CR_S1_BOXES_MIN_BLOCKS) k_stage1(c
         const CrSegment* sg = p.segments + it.seg;
         const uint32_t numTri = __ldg(&sg->numTriangles);
         const GeomRef geo = geom_of_t<PACKED>(sg);
-        const TileSrc ts = tile_source<true>(sg, it.batch, lists);
-        const bool tma = ts.src != nullptr;
-        const bool local = ts.local;
+        const bool tma = tile_source(sg, it.batch).src != nullptr;
         const uint32_t tri0 = it.batch * CR_BATCH;
+        const uint32_t first = __ldg(&sg->firstInstance);
+        const uint32_t ib = first + it.chunk * CR_INST_CHUNK;
+        const uint32_t ie = min(ib + CR_INST_CHUNK, first + __ldg(&sg->instanceCount));
+        const uint32_t alive = imask & ((1u << (ie - ib)) - 1u);
+        // lane k: the slot of the k-th surviving instance
+        const uint32_t slotOf = lane < __popc(alive) ? __fns(alive, 0, lane + 1) : 0u;
+        // bit 8 (k % 4) + b of subw[k / 4] is set unless sub-box b of the k-th
+        // surviving instance is proven to miss every sample (or is empty)
+        uint32_t subw[4];
+        {
+            const float4* obbs = p.instProof ? ldg_ptr(&sg->subObbs) : nullptr;
+            const int nsub = (int)min((uint32_t)(CR_BATCH / CR_SUB), (numTri - tri0 + CR_SUB - 1) / CR_SUB);
+            const int pairs = __popc(alive) * (CR_BATCH / CR_SUB);
+            Obb ob;
+            if (obbs && (lane & 7) < nsub)
+                ob = load_obb(obbs + CR_OBB_F4 * ((uint64_t)it.batch * (CR_BATCH / CR_SUB) + (lane & 7)));
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                subw[t] = 0;
+                if (t * 32 >= pairs) continue;
+                const int j = t * 32 + lane;
+                const uint32_t inst = ib + __shfl_sync(FULL, slotOf, (j >> 3) & 31);
+                bool keep = j < pairs && (j & 7) < nsub;
+                if (keep && obbs) keep = !obb_misses_samples(load_proof(p, inst), tg.fa, p.f, Wf, Hf, ob);
+                subw[t] = __ballot_sync(FULL, keep);
+            }
+        }
+        static_assert(CR_BATCH / CR_SUB == 8 && CR_INST_CHUNK <= 16, "8 sub-boxes x 16 instances in 4 ballots");
         if (tma) {
             const bool ok =
                 __all_sync(FULL, mbar_wait_bounded(&s_bar[w][slot], (parity & bit) ? 1u : 0u, p.waitTimeoutNs));
@@ -857,134 +878,41 @@ __global__ void __launch_bounds__(WARPS * 32, CR_S1_BOXES_MIN_BLOCKS) k_stage1(c
         const uint32_t* tile = s_idx[w][slot];
         // vertex index of corner c of the triangle at tile position pos
         auto index_of = [&](uint32_t pos, int c) -> uint32_t {
-            if (local) return tile[(tile[CR_LOCAL_MAX + pos] >> (8 * c)) & 0xffu];
             if (tma) return tile[3 * pos + c];
             return geom_index(geo, 3ull * (tri0 + pos) + c);
         };
-        bool act[S1_R];
-#pragma unroll
-        for (int r = 0; r < S1_R; ++r) act[r] = tri0 + r * 32 + lane < numTri;
-
-        const uint32_t first = __ldg(&sg->firstInstance);
-        const uint32_t count = __ldg(&sg->instanceCount);
-        const uint32_t ib = first + it.chunk * CR_INST_CHUNK;
-        const uint32_t ie = min(ib + CR_INST_CHUNK, first + count);
-        const uint32_t alive = imask & ((1u << (ie - ib)) - 1u);
-        // items without a vertex list: sub-box proofs of the sample-miss cull
-        // for every (surviving instance, sub-box) pair, spread over the lanes;
-        // bit 8 k + b of subw[k / 4] is set unless sub-box b of the k-th
-        // surviving instance is proven to miss every sample
-        uint32_t subw[4] = {~0u, ~0u, ~0u, ~0u};
-        if (!local) {
-            const float* sbx = ldg_ptr(&sg->subBoxes);
-            const int nsub = (int)min((uint32_t)(CR_BATCH / CR_SUB), (numTri - tri0 + CR_SUB - 1) / CR_SUB);
-            const int pairs = __popc(alive) * (CR_BATCH / CR_SUB);
-            if (sbx) {
+        // the sub-boxes that are left, two at a time across the item's
+        // instances: half a warp each, a triangle per lane
 #pragma unroll 1
-                for (int t = 0; t < 4; ++t) {
-                    if (t * 32 >= pairs) break;
-                    const int j = t * 32 + lane;
-                    bool keep = true;
-                    if (j < pairs && (j & 7) < nsub) {
-                        const uint32_t islot = __fns(alive, 0, (j >> 3) + 1);
-                        const float* bx = sbx + 6ull * ((uint64_t)it.batch * (CR_BATCH / CR_SUB) + (j & 7));
-                        const float blo[3] = {__ldg(bx), __ldg(bx + 1), __ldg(bx + 2)};
-                        const float bhi[3] = {__ldg(bx + 3), __ldg(bx + 4), __ldg(bx + 5)};
-                        keep = !box_misses_samples(load_mat(p.world_view + 4ull * (ib + islot)), fa, p.f, p.W, p.H,
-                                                   1.0 / (double)p.W, 1.0 / (double)p.H, blo, bhi);
-                    }
-                    subw[t] = __ballot_sync(FULL, keep);
-                }
-            }
-        }
-        static_assert(CR_BATCH / CR_SUB == 8 && CR_INST_CHUNK <= 16, "8 sub-boxes x 16 instances in 4 ballots");
-        const uint32_t nLocal = local ? __ldg(ldg_ptr(&sg->localCounts) + it.batch) : 0u;
-        // Triangles no record or proof culls, queued across the item's
-        // instances as (instance slot << 8 | tile position) in a per-warp ring
-        // and run through the reference's full path 32 at a time.
-        uint16_t* ring = s_ring[w];
-        uint32_t qh = 0, qt = 0;  // ring head / tail (warp-uniform)
-        // evaluates queued triangles 32 at a time (all: down to an empty ring)
-        auto drain = [&](bool all) {
-            while (qt - qh >= 32u || (all && qt > qh)) {
-                const uint32_t j = qh + lane;
+        for (int t = 0; t < 4; ++t) {
+            uint32_t rest = t == 0 ? subw[0] : t == 1 ? subw[1] : t == 2 ? subw[2] : subw[3];
+            while (rest) {
+                const uint32_t b0 = (uint32_t)__ffs(rest) - 1;
+                rest &= rest - 1;
+                const uint32_t b1 = rest ? (uint32_t)__ffs(rest) - 1 : 32u;
+                rest &= rest - 1;
+                const uint32_t b = lane < 16 ? b0 : b1;  // pair 32 t + b: instance rank, sub-box
+                const uint32_t inst = ib + __shfl_sync(FULL, slotOf, (t * 4 + (int)(b >> 3)) & 31);
+                const uint32_t tp = CR_SUB * (b & 7u) + (uint32_t)(lane & 15);
+                const uint32_t tri = tri0 + tp;
                 int res = S1_CULL;
-                uint32_t tri = 0, inst = 0;
-                if (j < qt) {
-                    const uint32_t e = ring[j & (S1_RING - 1)];
-                    const uint32_t tp = e & 0xffu;
-                    inst = ib + (e >> 8);
-                    tri = tri0 + tp;
+                if (b < 32u && tri < numTri) {
                     const V3 pa = pos_of(geo, index_of(tp, 0));
                     const V3 pb = pos_of(geo, index_of(tp, 1));
                     const V3 pc = pos_of(geo, index_of(tp, 2));
-                    res = stage1_triangle(target_of(p), fa, load_mat(p.world_view + 4ull * inst),
+                    res = stage1_triangle(tg, tg.fa, load_mat(p.world_view + 4ull * inst),
                                           __ldg(&p.instances[inst].flip), pa, pb, pc,
                                           __ldg(&p.instances[inst].cum) + tri);
                 }
-                qh = min(qh + 32u, qt);
                 append_nontrivial(p, res == S1_QUEUE, inst, tri);
-                __syncwarp();
             }
-        };
-        int rank = 0;
-        for (uint32_t inst = ib; inst < ie; ++inst) {
-            if (!((alive >> (inst - ib)) & 1u)) continue;  // its box proved every triangle culled
-            const int kk = rank++;
-            bool culledR[S1_R];
-            if (local) {
-                // cell records of the item's distinct vertices for this
-                // instance; an instance whose mesh box is inside the frustum
-                // has the outcode 0 at every vertex
-                const Mat M = load_mat(p.world_view + 4ull * inst);
-                const bool inside = (__ldg(&p.instances[inst].meshClass) & CR_MESH_INSIDE) != 0u;
-                uint32_t* rec = s_rec[w];
-                if (inside) {
-                    for (uint32_t v = lane; v < nLocal; v += 64) {
-                        const uint32_t v2 = v + 32;
-                        const uint32_t r0 = vertex_cell32<false>(M, pos_of(geo, tile[v]), fa, p.f, Wf, Hf, Wm1, Hm1);
-                        const uint32_t r1 = v2 < nLocal ? vertex_cell32<false>(M, pos_of(geo, tile[v2]), fa, p.f, Wf,
-                                                                               Hf, Wm1, Hm1)
-                                                        : 0u;
-                        rec[v] = r0;
-                        if (v2 < nLocal) rec[v2] = r1;
-                    }
-                } else {
-                    for (uint32_t v = lane; v < nLocal; v += 32)
-                        rec[v] = vertex_cell32<true>(M, pos_of(geo, tile[v]), fa, p.f, Wf, Hf, Wm1, Hm1);
-                }
-                __syncwarp();
-                const uint32_t* cw = tile + CR_LOCAL_MAX;  // corner words
-#pragma unroll
-                for (int r = 0; r < S1_R; ++r) {
-                    const uint32_t c = cw[r * 32 + lane];
-                    culledR[r] = !act[r] || cell32_culled(rec[c & 0xffu], rec[(c >> 8) & 0xffu], rec[(c >> 16) & 0xffu]);
-                }
-            } else {
-                const uint32_t w4 = (kk >> 2) == 0 ? subw[0] : (kk >> 2) == 1 ? subw[1] : (kk >> 2) == 2 ? subw[2] : subw[3];
-                const uint32_t sm = (w4 >> (8 * (kk & 3))) & 0xffu;
-#pragma unroll
-                for (int r = 0; r < S1_R; ++r) culledR[r] = !((sm >> (2 * r + (lane >> 4))) & 1u);
-            }
-            // queue the others
-#pragma unroll
-            for (int r = 0; r < S1_R; ++r) {
-                const bool keep = act[r] && !culledR[r];
-                const unsigned m = __ballot_sync(FULL, keep);
-                if (keep) ring[(qt + __popc(m & ((1u << lane) - 1u))) & (S1_RING - 1)] =
-                    (uint16_t)(((inst - ib) << 8) | (uint32_t)(r * 32 + lane));
-                qt += __popc(m);
-            }
-            __syncwarp();
-            drain(false);
         }
-        drain(true);
         __syncwarp();
         {  // every read of this slot is done: refill it with the item STAGES ahead
             const uint64_t npk = pk + (uint64_t)STAGES * nw;
             if (npk < nItems) {
                 const Item nt = decode_item(p, item_at(npk));
-                const TileSrc ns = tile_source<true>(p.segments + nt.seg, nt.batch, lists);
+                const TileSrc ns = tile_source(p.segments + nt.seg, nt.batch);
                 if (ns.src) {
                     pending |= bit;
                     if (lane == 0) {

@@ -594,117 +594,86 @@ __device__ __forceinline__ uint32_t classify_box(const Mat& M, float fa, float f
                           make_float4(M.c0.z, M.c1.z, M.c2.z, M.c3.z), fa, f, lo, hi);
 }
 
-// Corner c (bit j: hi on axis j) of an affine form: base + the steps of set bits.
-__device__ __forceinline__ double corner_of(double base, const double st[3], int c) {
-    double q = base;
-    if (c & 1) q += st[0];
-    if (c & 2) q += st[1];
-    if (c & 4) q += st[2];
-    return q;
+// An instance's item-proof data (CR_PROOF_F4) and its matrix rows.
+struct Proof {
+    float4 rx, ry, rz;  // rows of [R | t]
+    float4 eye, det, S;
+};
+
+__device__ __forceinline__ Proof load_proof(const CrFrameParams& p, uint32_t inst) {
+    const Mat M = load_mat(p.world_view + 4ull * inst);
+    const float4* q = p.instProof + (uint64_t)CR_PROOF_F4 * inst;
+    return Proof{make_float4(M.c0.x, M.c1.x, M.c2.x, M.c3.x), make_float4(M.c0.y, M.c1.y, M.c2.y, M.c3.y),
+                 make_float4(M.c0.z, M.c1.z, M.c2.z, M.c3.z), __ldg(q), __ldg(q + 1), __ldg(q + 2)};
 }
 
-// One screen axis of box_misses_samples: true if every vertex of the box has
-// a float screen coordinate strictly inside (k, k + 1) for one integer k >= 0.
-// The corner numerators are F (bn + st_n) (F = fa, or f) and the depths
-// -(bz + st_z), summed in double; SX = |F| S_x (or S_y) and SZ = S_z scale the
-// rounding: EX = 2^-19 SX and ED bound the float evaluation error of X and d
-// at any vertex of the box; Dmin > 4 ED is the smallest depth.
+struct Obb {
+    V3 c, a0, a1, a2;
+};
+
+__device__ __forceinline__ Obb load_obb(const float4* o) {
+    const float4 x = __ldg(o), y = __ldg(o + 1), z = __ldg(o + 2);
+    return Obb{{x.x, x.y, x.z}, {x.w, y.x, y.y}, {y.z, y.w, z.x}, {z.y, z.z, z.w}};
+}
+
+__device__ __forceinline__ float row_dir(const float4 r, const V3 a) {
+    return __fmaf_rn(r.x, a.x, __fmaf_rn(r.y, a.y, r.z * a.z));
+}
+
+__device__ __forceinline__ float row_pos(const float4 r, const V3 c) {
+    return __fmaf_rn(r.x, c.x, __fmaf_rn(r.y, c.y, __fmaf_rn(r.z, c.z, r.w)));
+}
+
+// One screen axis of obb_misses_samples: true if every point of the box has
+// a stage-1 screen coordinate strictly inside (k, k + 1) for one integer
+// k >= 0.  F = fa (or f), row the x (or y) row, S its bound, size W (or H); dz
+// and g are the centre's depth and the depth steps of the axes, iD >= 1 / the
+// least depth.
 //
-// The exact coordinate s(p) = W ((X / D) / 2 + 1/2) - 1/2 is an increasing
-// function of X / D, a linear-fractional function with D > 0 on the box, so
-// its extremes over the box are at corners.  Stage 1 evaluates it as
-// fl(fl(fl(fl(X^ / d^) * 0.5 + 0.5) * W) - 0.5); with |X / D| <= R its error is
-// below Es = W/2 En + 3 2^-24 W (R/2 + 1/2) + 2^-25, En = (EX + R ED) /
-// (Dmin - ED) + 2^-24 (R + En); invD >= 1 / (Dmin - ED).  Each corner is checked against the bounds
-// k + Es, k + 1 - Es by cross-multiplication (D > 0), with a tolerance above
-// the double rounding of the corner sums and of the check.  k >= 0: for
-// k = -1 the bounding box's clamp to 0 makes floor(min_x) = 0 and the cull
-// fails; for k >= W - 1 the clamp of max_x to W - 1 keeps max_x < k + 1 and
-// the cull holds.
-__device__ __forceinline__ bool axis_misses_samples(double F, double bn, const double stn[3], double bz,
-                                                    const double stz[3], double invD, double ED, double SX, double SZ,
-                                                    double Wd, double invW) {
-    const double EX = SX * 1.9073486328125e-06;  // 2^-19
-    // k from corner 0 (any estimate will do: the corner checks prove the rest)
-    const float s0 = (float)Wd * ((float)(F * bn) * __frcp_rn((float)-bz) * 0.5f + 0.5f) - 0.5f;
-    if (!(s0 >= 0.0f && s0 < 1e9f)) return false;  // also NaN
-    const double k = (double)floorf(s0);
-    // |X / D| <= R on the interval the checks below allow; invW is within
-    // 2^-52 of 1 / W, far inside the slack of Es
-    const double R = fmax(fabs(2.0 * ((k + 0.5) * invW) - 1.0), fabs(2.0 * ((k + 1.5) * invW) - 1.0));
-    const double En = (EX + R * ED) * invD + 1.1920928955078125e-07 * (R + 1.0);                  // 2^-23
-    const double Es = 0.5 * Wd * En + 2.384185791015625e-07 * (Wd * (0.5 * R + 0.5) + 1.0) + 1e-6;  // 2^-22
-    if (!(Es < 0.25)) return false;
-    const double alo = 2.0 * ((k + Es + 0.5) * invW) - 1.0;
-    const double ahi = 2.0 * ((k + 1.0 - Es + 0.5) * invW) - 1.0;
-    const double tol0 = SX + R * SZ;
-#pragma unroll 1
-    for (int c = 0; c < 8; ++c) {
-        const double X = F * corner_of(bn, stn, c);
-        const double D = -corner_of(bz, stz, c);
-        const double tol = 2.842170943040401e-14 * ((fabs(X) + R * D) + tol0);  // 2^-45
-        if (!(X - alo * D > tol && ahi * D - X > tol)) return false;
-    }
-    return true;
+// The exact coordinate is s(p) = W ((X / D) / 2 + 1/2) - 1/2.  For any number
+// r0, X / D - r0 = (X - r0 D) / D, and X - r0 D is affine: its centre value plus
+// at most e = sum_j |F g_xj + r0 g_zj| (D = -q.z).  With r0 the float quotient of
+// the centre, everything float about this -- the centre's X, D and quotient, the
+// steps, e -- is off by less than 48u (|F| S + |r0| Sz) in the numerator (u =
+// 2^-24; each row form errs by 3u S per term, and an axis' terms are at most
+// twice S), and stage 1's own X and d of a vertex by 5u of the same, over a d no
+// less than the least depth; 96u is allowed.  Its quotient, and the scale to
+// pixels there and here, round by less than 16u W (|r0| + 2) pixels; 32u is
+// allowed.  k >= 0: for k = -1 the bounding box's clamp to 0 makes floor(min_x)
+// = 0 and the cull fails; for k >= W - 1 the clamp of max_x to W - 1 keeps
+// max_x < k + 1 and the cull holds.  NaN and infinity fail the comparisons.
+__device__ __forceinline__ bool axis_misses_samples(float F, const float4 row, float S, float Sz, const Obb& b, float D0,
+                                                    const float3 gz, float iD, float W) {
+    const float u = 5.9604644775390625e-08f;
+    const float r0 = __fdividef(F * row_pos(row, b.c), D0);
+    const float e = fabsf(__fmaf_rn(r0, gz.x, F * row_dir(row, b.a0))) +
+                    fabsf(__fmaf_rn(r0, gz.y, F * row_dir(row, b.a1))) +
+                    fabsf(__fmaf_rn(r0, gz.z, F * row_dir(row, b.a2)));
+    const float ar = fabsf(r0);
+    const float h = 0.5f * W * ((e + (96.0f * u * (fabsf(F) * S + (ar + 1.0f) * Sz) + 1e-30f)) * iD) +
+                    32.0f * u * W * (ar + 2.0f);
+    const float s0 = W * (0.5f * r0 + 0.5f) - 0.5f;
+    const float lo = s0 - h, hi = s0 + h, k = floorf(lo);
+    return lo > k && k >= 0.0f && hi < k + 1.0f && h < 0.5f;
 }
 
-// True if every vertex p in the object-space box [lo, hi] is, in stage 1's
-// float arithmetic (xform, viewToNDC, ndcToScreen, -0.5: tv.cu:103-134), in
-// front of the camera (depth > 0) and strictly inside one pixel column or one
-// pixel row of samples.  Then every triangle whose vertices lie in the box has
-// isNontrivial false and meets the reference's sample-miss cull (tv.cu:153-158),
-// so it writes nothing.  The float transform of a vertex is within 3 2^-24 S
-// of the exact affine value (S = sum_j |M_j| max|p_j| + |M_3| per row; the
-// bound uses 2^-19 S, which also covers fl(fa q.x)).  Corner values are exact
-// products of floats summed in double.  Non-finite boxes prove nothing.
-// invW, invH: 1 / W and 1 / H in double (any rounding: they only place the
-// bounds the corners are checked against).
-__device__ bool box_misses_samples(const Mat& M, float fa, float f, int W, int H, double invW, double invH,
-                                   const float lo[3], const float hi[3]) {
-    const double E19 = 1.9073486328125e-06;  // 2^-19
-    const double ax[3] = {M.c0.x, M.c1.x, M.c2.x}, ay[3] = {M.c0.y, M.c1.y, M.c2.y};
-    const double az[3] = {M.c0.z, M.c1.z, M.c2.z};
-    double mabs[3];
-#pragma unroll
-    for (int j = 0; j < 3; ++j) mabs[j] = fmax(fabs((double)lo[j]), fabs((double)hi[j]));
-    const double Sz = (fabs(az[0]) * mabs[0] + fabs(az[1]) * mabs[1]) + (fabs(az[2]) * mabs[2] + fabs((double)M.c3.z));
-    if (!(Sz < 1e30)) return false;
-    double bz = M.c3.z, stz[3];
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-        bz += az[j] * (double)lo[j];
-        stz[j] = az[j] * (double)hi[j] - az[j] * (double)lo[j];
-    }
-    double Dmin = 1e300;
-#pragma unroll
-    for (int c = 0; c < 8; ++c) Dmin = fmin(Dmin, -corner_of(bz, stz, c));
-    const double ED = E19 * Sz + 1e-30;
-    if (!(Dmin > 4.0 * ED && Dmin < 1e30)) return false;  // every vertex in front, with room
-    // an upper bound of 1 / (Dmin - ED): the float reciprocal of the rounded
-    // value is within 2^-22.9 of it; (1 + 2^-20) covers that
-    const double invD = (double)__frcp_rn((float)(Dmin - ED)) * 1.00000095367431640625;
-    {
-        const double Sx =
-            (fabs(ax[0]) * mabs[0] + fabs(ax[1]) * mabs[1]) + (fabs(ax[2]) * mabs[2] + fabs((double)M.c3.x));
-        double bx = M.c3.x, stx[3];
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            bx += ax[j] * (double)lo[j];
-            stx[j] = ax[j] * (double)hi[j] - ax[j] * (double)lo[j];
-        }
-        if (Sx < 1e30 &&
-            axis_misses_samples(fa, bx, stx, bz, stz, invD, ED, fabs((double)fa) * Sx, Sz, (double)W, invW))
-            return true;
-    }
-    const double Sy = (fabs(ay[0]) * mabs[0] + fabs(ay[1]) * mabs[1]) + (fabs(ay[2]) * mabs[2] + fabs((double)M.c3.y));
-    double by = M.c3.y, sty[3];
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-        by += ay[j] * (double)lo[j];
-        sty[j] = ay[j] * (double)hi[j] - ay[j] * (double)lo[j];
-    }
-    return Sy < 1e30 &&
-           axis_misses_samples(f, by, sty, bz, stz, invD, ED, fabs((double)f) * Sy, Sz, (double)H, invH);
+// True if every vertex in the oriented box is, in stage 1's float arithmetic
+// (xform, viewToNDC, ndcToScreen, -0.5: tv.cu:103-134), in front of the camera
+// (depth > 0) and strictly inside one pixel column or one pixel row of
+// samples.  Then every triangle whose vertices lie in the box has isNontrivial
+// false and meets the reference's sample-miss cull (tv.cu:153-158), so it writes
+// nothing.  Single precision with fused products: about 90 instructions a
+// box and instance, no division beyond two reciprocals.
+__device__ __forceinline__ bool obb_misses_samples(const Proof& P, float fa, float f, float W, float H, const Obb& b) {
+    const float u = 5.9604644775390625e-08f;
+    const float3 gz = make_float3(row_dir(P.rz, b.a0), row_dir(P.rz, b.a1), row_dir(P.rz, b.a2));
+    const float D0 = -row_pos(P.rz, b.c);
+    // the least depth, less every rounding of it (here and in stage 1)
+    const float Dmin = (D0 - (fabsf(gz.x) + fabsf(gz.y) + fabsf(gz.z))) - (64.0f * u * P.S.z + 1e-30f);
+    if (!(Dmin > 1e-30f && Dmin < 1e30f)) return false;
+    const float iD = __fdividef(1.0f, Dmin) * 1.00000095367431640625f;
+    return axis_misses_samples(fa, P.rx, P.S.x, P.S.z, b, D0, gz, iD, W) ||
+           axis_misses_samples(f, P.ry, P.S.y, P.S.z, b, D0, gz, iD, H);
 }
 
 // True if every triangle of an item is culled by stage 1's back-face test
@@ -712,51 +681,44 @@ __device__ bool box_misses_samples(const Mat& M, float fa, float f, int W, int H
 // the camera e = -R^-1 t in object space, the exact value of stage 1's
 // res = av . ((bv - av) x (cv - av)) is det R ((pa - e) . n), n the object-space
 // (pb - pa) x (pc - pa); with the mirror flip the test culls when
-// (pa - e) . n >= 0.  From the item's box (centre c, half-diagonal r) and
-// normal cone (axis m, every unit normal within acos cosT of it),
-// (pa - e) . n >= |n| G with G = |c - e| cos(phi + theta) - r, phi the angle
+// (pa - e) . n >= 0.  For a ball (centre c, radius r) that holds the item's
+// vertices and its normal cone (axis m, every unit normal within acos cosT of
+// it), (pa - e) . n >= |n| G with G = |c - e| cos(phi + theta) - r, phi the angle
 // between c - e and m, evaluated without dividing as ((c - e) . m cos theta -
 // |(c - e) x m| sin theta) / |m| with |m| = 1 (the stored unit axis is within
-// 2^-23 of it, a relative error that the 1e-6 slack covers with the double
-// rounding).  The float res differs from the exact one by at most
-// E: the transform's rounding (each view coordinate within gamma_3 T of the
-// exact one, T = sum_j |R_ij| |p_j| + |t_i|), the edge subtractions, the cross
-// and dot products (gamma_2 and gamma_3 of their magnitude bounds), with |av| <=
-// |R|_F (|c - e| + r) and edges <= |R|_F edge; E is doubled.  When
-// |det R| nMin G > E every triangle's float res has the sign that culls it.
-// B: CR_BACK_DOUBLES of the instance; cone: CR_CONE_FLOATS of the item.
-__device__ __noinline__ bool item_back_facing(const double* B, const float* cone, const float lo[3],
-                                                 const float hi[3]) {
-    const double detA = B[3];
-    const double cosT = (double)__ldg(cone + 3);
-    if (!(detA > 0.0) || !(cosT > 0.0)) return false;
-    const double m0 = __ldg(cone), m1 = __ldg(cone + 1), m2 = __ldg(cone + 2);
-    const double sinT = __ldg(cone + 6), r = __ldg(cone + 7);
-    double w[3], P = 0.0;
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-        w[j] = 0.5 * ((double)lo[j] + (double)hi[j]) - B[j];
-        P = fmax(P, fmax(fabs((double)lo[j]), fabs((double)hi[j])));
-    }
-    const double wl = sqrt(w[0] * w[0] + w[1] * w[1] + w[2] * w[2]);
-    if (!(wl > 0.0)) return false;
-    const double dm = w[0] * m0 + w[1] * m1 + w[2] * m2;
-    const double cx = w[1] * m2 - w[2] * m1, cy = w[2] * m0 - w[0] * m2, cz = w[0] * m1 - w[1] * m0;
-    const double cr = sqrt(cx * cx + cy * cy + cz * cz);
-    // rounding of e, the centre and the products in double, and |m| = 1
-    // within 2^-23: far below 1e-6 of the magnitudes involved (B[7] = |e|)
-    const double G = (dm * cosT - cr * sinT) - r - 1e-6 * (wl + r + B[7] + P);
-    if (!(G > 0.0)) return false;
-    const double u = 5.9604644775390625e-08;  // 2^-24
-    const double g2 = 2.0 * u / (1.0 - 2.0 * u), g3 = 3.0 * u / (1.0 - 3.0 * u);
-    const double a = B[4] * (wl + r);                // |av| bound
-    const double L = B[4] * (double)__ldg(cone + 5);  // edge length bound in view space
-    const double Delta = 1.7320508075688774 * g3 * (B[5] * P + B[6]);  // |av - A| bound
-    const double eta = 2.01 * Delta + u * L;         // |fl(bv - av) - (B - A)| bound
-    const double Lp = L + eta;
-    const double E = 2.0 * ((Delta + a * 3.4641016151377548 * g2 + g3 * (a + Delta)) * Lp * Lp * 1.01 +
-                            a * (2.0 * eta * L + eta * eta));
-    return isfinite(E) && detA * (double)__ldg(cone + 4) * G > E;
+// 2^-23 of it).  Evaluated in single precision G is off by less than 20u
+// (|c - e| + |e| + |c|) + 4u r; 64u (3.8e-6) is taken off.  The float res differs from
+// the exact one by at most E: the transform's rounding (each view coordinate within
+// gamma_3 T of the exact one, T = sum_j |R_ij| |p_j| + |t_i|), the edge
+// subtractions, the cross and dot products (gamma_2 and gamma_3 of their
+// magnitude bounds, with |av| <= |R|_F (|c - e| + r) and edges <= |R|_F edge); E
+// is doubled, and its own single-precision sum (all terms positive) is covered by
+// 1.001.  When |det R| nMin G > E every triangle's float res has the sign that
+// culls it (1e-30: products that underflow prove nothing).
+// c0, c1: the item's CR_CONE_FLOATS; mid: the centre of its box, r half its
+// diagonal.
+__device__ __forceinline__ bool item_back_facing(const Proof& P, const float4 c0, const float4 c1, const V3 mid) {
+    const float detA = P.det.x, cosT = c0.w, nMin = c1.x, edge = c1.y, sinT = c1.z, r = c1.w;
+    if (!(detA > 0.0f) || !(cosT > 0.0f)) return false;
+    const V3 w = {mid.x - P.eye.x, mid.y - P.eye.y, mid.z - P.eye.z};
+    const float p = fmaxf(fabsf(mid.x), fmaxf(fabsf(mid.y), fabsf(mid.z))) + r;  // >= max |p_j|
+    const float wl = sqrtf(__fmaf_rn(w.x, w.x, __fmaf_rn(w.y, w.y, w.z * w.z)));
+    const float dm = __fmaf_rn(w.x, c0.x, __fmaf_rn(w.y, c0.y, w.z * c0.z));
+    const float cx = __fmaf_rn(w.y, c0.z, -(w.z * c0.y)), cy = __fmaf_rn(w.z, c0.x, -(w.x * c0.z)),
+                cz = __fmaf_rn(w.x, c0.y, -(w.y * c0.x));
+    const float cr = sqrtf(__fmaf_rn(cx, cx, __fmaf_rn(cy, cy, cz * cz)));
+    const float G = ((dm * cosT - cr * sinT) - r) - 3.814697265625e-06f * (wl + r + P.eye.w + 2.0f * p);
+    if (!(G > 0.0f)) return false;
+    const float u = 5.9604644775390625e-08f;
+    const float g2 = 2.001f * u, g3 = 3.001f * u;
+    const float a = P.det.y * (wl + r) * 1.000001f;  // |av| bound
+    const float L = P.det.y * edge;                  // edge length bound in view space
+    const float Delta = 1.7320509f * g3 * (P.det.z * p + P.det.w);  // |av - A| bound
+    const float eta = 2.01f * Delta + u * L;         // |fl(bv - av) - (B - A)| bound
+    const float Lp = L + eta;
+    const float E = 2.0f * ((Delta + a * 3.4641018f * g2 + g3 * (a + Delta)) * Lp * Lp * 1.01f +
+                            a * (2.0f * eta * L + eta * eta));
+    return detA * nMin * G * 0.999f > E * 1.001f + 1e-30f;
 }
 
 // Cell record of one vertex: the outcode plus stage 1's own screen position

@@ -1,0 +1,200 @@
+"""Soundness of the frame cull's single-precision item proofs (raster_core.cuh
+item_back_facing and obb_misses_samples, with the oriented boxes of meshprep.cu
+k_obbs and the per-instance data of api.cpp proof_data), restated in numpy with
+the same float operations: whenever a proof says an item is culled, every one of
+its triangles (vertices) meets stage 1's float test."""
+import numpy as np
+import pytest
+from test_backface_proof_cpu import back_face_data, det3_glm, item_cone, items, look_at, stage1_backface_culled, xform
+
+F = np.float32
+U = F(2.0 ** -24)
+
+
+def fma(a, b, c):
+    return F(float(a) * float(b) + float(c))
+
+
+def dot_pos(r, c):
+    return fma(r[0], c[0], fma(r[1], c[1], fma(r[2], c[2], r[3])))
+
+
+def dot_dir(r, a):
+    return fma(r[0], a[0], fma(r[1], a[1], F(r[2]) * F(a[2])))
+
+
+def instance_proof(M, lo, hi):
+    """api.cpp proof_data: eye, |eye|; |det|, |R|_F, rowAbs, tAbs; S per row."""
+    e, det, frob, row, t, el = back_face_data(M)
+    R = M.reshape(4, 4).T.astype(np.float64)
+    S = np.abs(R[:3, :3]) @ np.maximum(np.abs(lo), np.abs(hi)).astype(np.float64) + np.abs(R[:3, 3])
+    up = 1 + 1e-6
+    return (e.astype(F), F(el * up), F(det * (1 - 1e-6)), F(frob * up), F(row * up), F(t * up),
+            (S * up).astype(F))
+
+
+def proof_back_facing(M, lo, hi, cone, drop_error=False):
+    e, el, det, frob, row, tabs, _ = instance_proof(M, lo, hi)
+    m, cosT, nMin, edge, sinT, r = [F(x) if np.ndim(x) == 0 else x.astype(F) for x in cone]
+    if not (det > 0 and cosT > 0):
+        return False
+    mid = (F(0.5) * (lo + hi)).astype(F)
+    w = (mid - e).astype(F)
+    p = np.abs(mid).max() + r
+    wl = np.sqrt(fma(w[0], w[0], fma(w[1], w[1], w[2] * w[2])))
+    dm = fma(w[0], m[0], fma(w[1], m[1], w[2] * m[2]))
+    cx, cy, cz = (fma(w[1], m[2], -(w[2] * m[1])), fma(w[2], m[0], -(w[0] * m[2])), fma(w[0], m[1], -(w[1] * m[0])))
+    cr = np.sqrt(fma(cx, cx, fma(cy, cy, cz * cz)))
+    G = ((dm * cosT - cr * sinT) - r) - F(3.814697265625e-06) * (wl + r + el + F(2) * p)
+    if not G > 0:
+        return False
+    g2, g3 = F(2.001) * U, F(3.001) * U
+    a, L = frob * (wl + r) * F(1.000001), frob * edge
+    Delta = F(1.7320509) * g3 * (row * p + tabs)
+    eta = F(2.01) * Delta + U * L
+    Lp = L + eta
+    E = F(2) * ((Delta + a * F(3.4641018) * g2 + g3 * (a + Delta)) * Lp * Lp * F(1.01) +
+                a * (F(2) * eta * L + eta * eta))
+    if drop_error:
+        E = F(0)
+    return bool(det * nMin * G * F(0.999) > E * F(1.001) + F(1e-30))
+
+
+def obb(p):
+    """meshprep.cu k_obbs on an (n, 3) float32 set, with a given frame's axes."""
+    q = p.astype(np.float64)
+    _, _, ax = np.linalg.svd(q - q.mean(0), full_matrices=True)
+    x = q @ ax.T
+    lo, hi = x.min(0), x.max(0)
+    h, c = 0.5 * (hi - lo), (0.5 * (lo + hi)) @ ax
+    slack = 2.0 ** -21 * (np.abs(c).max() + h.sum()) + 1e-37
+    return c.astype(F), [(ax[j] * (h[j] * (1 + 2.0 ** -20) + slack)).astype(F) for j in range(3)]
+
+
+def axis_misses(Fa, row, S, Sz, b, D0, gz, iD, W, margin):
+    r0 = F(Fa * dot_pos(row, b[0])) / D0
+    e = F(0)
+    for j in range(3):
+        e = e + np.abs(fma(r0, gz[j], Fa * dot_dir(row, b[1][j])))
+    ar = np.abs(r0)
+    h = F(0.5) * W * ((e + margin * (F(96) * U * (np.abs(Fa) * S + (ar + F(1)) * Sz) + F(1e-30))) * iD) + \
+        margin * F(32) * U * W * (ar + F(2))
+    s0 = W * (F(0.5) * r0 + F(0.5)) - F(0.5)
+    lo, hi = s0 - h, s0 + h
+    k = np.floor(lo)
+    return bool(lo > k and k >= 0 and hi < k + F(1) and h < F(0.5))
+
+
+def proof_misses(M, fa, f, W, H, b, S, margin=F(1)):
+    rows = M.reshape(4, 4).T.astype(F)
+    gz = [dot_dir(rows[2], a) for a in b[1]]
+    D0 = -dot_pos(rows[2], b[0])
+    Dmin = (D0 - (np.abs(gz[0]) + np.abs(gz[1]) + np.abs(gz[2]))) - margin * (F(64) * U * S[2] + F(1e-30))
+    if not (Dmin > F(1e-30) and Dmin < F(1e30)):
+        return False
+    iD = F(1) / Dmin * F(1.00000095367431640625)
+    return axis_misses(fa, rows[0], S[0], S[2], b, D0, gz, iD, W, margin) or \
+        axis_misses(f, rows[1], S[1], S[2], b, D0, gz, iD, H, margin)
+
+
+def stage1_screen(M, p, fa, f, W, H):
+    """viewToNDC, ndcToScreen, -0.5 of every vertex (float32, stage 1's order), and its depth."""
+    q = xform(M, p)
+    d = -q[:, 2]
+    x = ((fa * q[:, 0]) / d * F(0.5) + F(0.5)) * W - F(0.5)
+    y = ((f * q[:, 1]) / d * F(0.5) + F(0.5)) * H - F(0.5)
+    return x, y, d
+
+
+def missed(x, y, W, H):
+    def axis(s, n):
+        lo, hi = max(s.min(), F(0)), min(s.max(), F(n - 1))
+        return lo > np.floor(lo) and hi < np.floor(lo) + 1
+
+    return axis(x, W) or axis(y, H)
+
+
+def clusters(rng, n, drop):
+    """n proven (or, with the margins dropped, claimed) clusters of vertices that
+    end within a few float spacings of a sample line; the share that is wrong."""
+    wrong = claimed = 0
+    W, H = 1920, 1080
+    f = F(1.7320508)
+    fa = F(f / F(W / H))
+    for _ in range(n):
+        size = 10.0 ** rng.uniform(-5, 0)
+        off = rng.uniform(-1, 1, 3) * rng.choice([0.0, 1.0, 100.0])
+        Rm = np.linalg.qr(rng.normal(size=(3, 3)))[0]
+        # a box's corners and points inside: the box is met by its vertices
+        corner = np.array([[(c >> j) & 1 for j in range(3)] for c in range(8)]) * 2.0 - 1.0
+        p = (np.concatenate([corner, rng.uniform(-1, 1, (8, 3))]) * size * np.array([1.0, 0.3, 0.02])) @ Rm.T + off
+        # a fraction of a pixel wide, its edge next to a sample column, across a row
+        dist = size * 10.0 ** rng.uniform(3.1, 6.0)
+        px, py = rng.integers(1, W - 2), rng.integers(1, H - 2)
+        Vr = np.linalg.qr(rng.normal(size=(3, 3)))[0]
+        v = p.astype(F).astype(np.float64) @ Vr.T
+        t = np.array([0.0, 0.0, -dist]) - v.mean(0)
+        v2 = v + t
+        sx = (fa * v2[:, 0] / -v2[:, 2] * 0.5 + 0.5) * W - 0.5
+        sy = (f * v2[:, 1] / -v2[:, 2] * 0.5 + 0.5) * H - 0.5
+        gap = rng.choice([0.0, 3e-5, 1e-4, 1e-2, 0.02, 0.1])
+        t[0] += (px + gap - sx.min()) / W * 2 / float(fa) * dist
+        t[1] += (py - sy.mean()) / H * 2 / float(f) * dist
+        M = np.eye(4)
+        M[:3, :3], M[:3, 3] = Vr, t
+        M = M.astype(F).T.reshape(16)
+        pts = p.astype(F)
+        S = instance_proof(M, pts.min(0), pts.max(0))[-1]
+        b = obb(pts)
+        if drop:
+            b = (b[0], [(a / (1 + 2.0 ** -20)).astype(F) for a in b[1]])
+        if proof_misses(M, fa, f, F(W), F(H), b, S, F(0) if drop else F(1)):
+            claimed += 1
+            x, y, d = stage1_screen(M, pts, fa, f, F(W), F(H))
+            wrong += not ((d > 0).all() and missed(x, y, W, H))
+    return claimed, wrong
+
+
+def test_sample_miss_proof_is_sound():
+    claimed, wrong = clusters(np.random.default_rng(5), 6000, False)
+    assert claimed > 800 and wrong == 0, (claimed, wrong)
+
+
+def test_sample_miss_margins_matter():
+    claimed, wrong = clusters(np.random.default_rng(5), 6000, True)
+    assert claimed > 800 and wrong > 0, (claimed, wrong)
+
+
+@pytest.mark.parametrize("drop", [False, True])
+def test_back_face_proof_is_sound(drop):
+    rng = np.random.default_rng(12)
+    proved = wrong = 0
+    for pa, pb, pc in items(rng):
+        cone = item_cone(pa, pb, pc)
+        if cone is None:
+            continue
+        allp = np.concatenate([pa, pb, pc])
+        lo, hi = allp.min(0), allp.max(0)
+        centre = 0.5 * (lo.astype(np.float64) + hi)
+        for _ in range(40):
+            m = cone[0] / np.linalg.norm(cone[0])
+            dirn = -m + rng.normal(scale=rng.choice([0.01, 0.3, 1.0]), size=3)
+            eye = centre + dirn / np.linalg.norm(dirn) * rng.uniform(0.05, 200.0)
+            k = int(rng.integers(128))
+            a64 = pa[k].astype(np.float64)
+            nk = np.cross(pb[k].astype(np.float64) - a64, pc[k].astype(np.float64) - a64)
+            if rng.random() < 0.5:  # just behind the plane of one of the item's triangles
+                nk /= np.linalg.norm(nk)
+                inpl = np.cross(nk, rng.normal(size=3))
+                dist = rng.uniform(0.05, 50.0)
+                eye = a64 + inpl / np.linalg.norm(inpl) * dist - nk * dist * rng.choice([1e-8, 1e-6, 1e-5, 1e-4, 1e-3])
+            Wm = np.eye(4)
+            if rng.random() < 0.5:
+                Wm[:3, :3] = np.diag(rng.uniform(0.3, 3.0, 3) * rng.choice([-1, 1], 3))
+            V = look_at(eye, centre + rng.normal(scale=0.5, size=3))
+            M = (V @ Wm).astype(F).T.reshape(16)
+            if proof_back_facing(M, lo, hi, cone, drop):
+                proved += 1
+                wrong += not stage1_backface_culled(M, det3_glm(M) < 0, pa, pb, pc).all()
+    assert proved > 100
+    assert (wrong > 0) if drop else (wrong == 0), (proved, wrong)
