@@ -1387,7 +1387,8 @@ cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_
     mat4_inverse(cam->view, rp.viewI);
     for (int r = 0; r < 3; r++)  // viewI * (0,0,0,1)
         rp.origin[r] = (rp.viewI[0 + r] * 0.0f + rp.viewI[4 + r] * 0.0f) + (rp.viewI[8 + r] * 0.0f + rp.viewI[12 + r] * 1.0f);
-    rp.p00 = cam->proj[0];
+    rp.ip00 = 1.0f / cam->proj[0];
+    rp.ip11 = 1.0f / cam->proj[5];
     rp.p11 = cam->proj[5];
     rp.background = 0xffffffffu;  // HostDeviceInterface.h:37 BACKGROUND_COLOR
     memcpy(rp.view, cam->view, 64);

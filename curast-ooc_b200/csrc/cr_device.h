@@ -325,7 +325,8 @@ struct CrResolveParams {
     int32_t W, H;
     float viewI[16];            // inverse(view), glm::inverse float order
     float origin[3];            // viewI * (0,0,0,1)
-    float p00, p11;             // proj[0][0], proj[1][1]
+    float ip00, ip11;           // 1 / proj[0][0], 1 / proj[1][1] (rounded once)
+    float p11;                  // proj[1][1] (STAGE display)
     uint32_t background;
     uint32_t writeBackground;   // 1: empty pixels get the background
     uint64_t idLo, idHi;        // covered pixels are written only for ids in [idLo, idHi)

@@ -232,7 +232,8 @@ cr_status render_on_device(int32_t device, const cr_noalloc_instance* instances,
     cr_internal_mat4_inverse(cam->view, rp.viewI);
     for (int r = 0; r < 3; r++)
         rp.origin[r] = (rp.viewI[0 + r] * 0.0f + rp.viewI[4 + r] * 0.0f) + (rp.viewI[8 + r] * 0.0f + rp.viewI[12 + r] * 1.0f);
-    rp.p00 = cam->proj[0];
+    rp.ip00 = 1.0f / cam->proj[0];
+    rp.ip11 = 1.0f / cam->proj[5];
     rp.p11 = cam->proj[5];
     rp.background = 0xffffffffu;
     memcpy(rp.view, cam->view, 64);

@@ -68,7 +68,13 @@ __device__ __forceinline__ V3 pos_of(const GeomRef& g, uint32_t v) {
     return r;
 }
 
-__device__ __forceinline__ void resolve_pixel(const CrResolveParams& p, const int x, const int y) {
+// The pixel's coordinates on the image plane (resolve.cu:662-676): a block's
+// columns and rows share them.
+__device__ __forceinline__ float plane_coord(int i, int n) { return 2.0f * ((float)i + 0.5f) / (float)n - 1.0f; }
+
+// u, v: plane_coord of x and y.
+__device__ __forceinline__ void resolve_pixel(const CrResolveParams& p, const int x, const int y, const float u,
+                                              const float v) {
     const int pid = x + p.W * y;
     const uint64_t pixel = __ldcs(reinterpret_cast<const unsigned long long*>(p.fb) + pid);
 
@@ -120,9 +126,7 @@ __device__ __forceinline__ void resolve_pixel(const CrResolveParams& p, const in
             if (p.display == 4) {  // DisplayAttribute::VERTEX_COLORS
                 // computeRayDir, resolve.cu:662-676
                 const V3 origin = {p.origin[0], p.origin[1], p.origin[2]};
-                const float u = 2.0f * ((float)x + 0.5f) / (float)p.W - 1.0f;
-                const float v = 2.0f * ((float)y + 0.5f) / (float)p.H - 1.0f;
-                const V3 rdv = normalize3(V3{1.0f / p.p00 * u, 1.0f / p.p11 * v, -1.0f});
+                const V3 rdv = normalize3(V3{p.ip00 * u, p.ip11 * v, -1.0f});
                 const V3 rayDir = normalize3(sub3(xform_m(p.viewI, rdv), origin));
 
                 // intersectPlane (helpers:318-348) and barycentrics (resolve.cu:790-834)
@@ -210,10 +214,15 @@ __global__ void __launch_bounds__(256) k_resolve(const CrResolveParams p) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (p.hostCounters && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.y == 0 && threadIdx.x < CR_CTR_COUNT)
         p.hostCounters[threadIdx.x] = p.counters[threadIdx.x];
+    __shared__ float s_u[32], s_v[8];
+    const int t = threadIdx.y * 32 + threadIdx.x;
+    if (t < 32) s_u[t] = plane_coord(blockIdx.x * 32 + t, p.W);
+    else if (t < 40) s_v[t - 32] = plane_coord(blockIdx.y * 8 + t - 32, p.H);
+    __syncthreads();
     const int x = blockIdx.x * 32 + threadIdx.x;
     const int y = blockIdx.y * 8 + threadIdx.y;
     if (x >= p.W || y >= p.H) return;
-    resolve_pixel(p, x, y);
+    resolve_pixel(p, x, y, s_u[threadIdx.x], s_v[threadIdx.y]);
 }
 
 // Batched frames: one flat grid of 32x32-pixel tiles over all views (view v
@@ -224,6 +233,7 @@ __global__ void __launch_bounds__(256) k_resolve(const CrResolveParams p) {
 __global__ void __launch_bounds__(256) k_resolve_views(const CrResolveParams base, const CrView* views,
                                                        uint32_t numViews) {
     __shared__ CrResolveParams s_p;
+    __shared__ float s_u[32], s_v[32];
     uint32_t lo = 0, hi = numViews - 1;  // view owning this block
     while (lo < hi) {
         const uint32_t mid = (lo + hi + 1) >> 1;
@@ -243,21 +253,25 @@ __global__ void __launch_bounds__(256) k_resolve_views(const CrResolveParams bas
         s_p.origin[0] = __ldg(&v->origin[0]);
         s_p.origin[1] = __ldg(&v->origin[1]);
         s_p.origin[2] = __ldg(&v->origin[2]);
-        s_p.p00 = __ldg(&v->p00);
+        s_p.ip00 = 1.0f / __ldg(&v->p00);
+        s_p.ip11 = 1.0f / __ldg(&v->p11);
         s_p.p11 = __ldg(&v->p11);
         s_p.idBase = __ldg(&v->idBase);
     }
     if (t < 16) s_p.viewI[t] = __ldg(&v->viewI[t]);
     if (t >= 16 && t < 32) s_p.view[t - 16] = __ldg(&v->view[t - 16]);
-    __syncthreads();
     const uint32_t b = blockIdx.x - __ldg(&v->resolveBlockBase);
     const uint32_t bx = (uint32_t)(W + 31) / 32;
-    const int x = (int)(b % bx) * 32 + threadIdx.x;
+    const int x0 = (int)(b % bx) * 32, y0 = (int)(b / bx) * 32;
+    if (t >= 32 && t < 64) s_u[t - 32] = plane_coord(x0 + t - 32, W);
+    else if (t >= 64 && t < 96) s_v[t - 64] = plane_coord(y0 + t - 64, H);
+    __syncthreads();
+    const int x = x0 + threadIdx.x;
     if (x >= W) return;
 #pragma unroll 1
     for (int k = 0; k < 4; ++k) {
-        const int y = (int)(b / bx) * 32 + threadIdx.y + 8 * k;
-        if (y < H) resolve_pixel(s_p, x, y);
+        const int r = threadIdx.y + 8 * k;
+        if (y0 + r < H) resolve_pixel(s_p, x, y0 + r, s_u[threadIdx.x], s_v[r]);
     }
 }
 
