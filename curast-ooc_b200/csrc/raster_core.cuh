@@ -874,7 +874,21 @@ __device__ __forceinline__ V2 sh_intersect(V2 p1, V2 p2, int e) {
     return V2{p1.x + t * (p2.x - p1.x), value};
 }
 
+// Extends [bmin, bmax] by the triangle clipped to the window.  A triangle wholly
+// inside comes out of the clipper as its own three corners, so its box is taken
+// without the clipper (whose polygon lives in local memory: most of the setup's
+// time where triangles are small on screen).
 __device__ void window_clip(V2 a, V2 b, V2 c, V2& bmin, V2& bmax) {
+    const float lx = fminf(a.x, fminf(b.x, c.x)), hx = fmaxf(a.x, fmaxf(b.x, c.x));
+    const float ly = fminf(a.y, fminf(b.y, c.y)), hy = fmaxf(a.y, fmaxf(b.y, c.y));
+    const bool num = a.x == a.x && b.x == b.x && c.x == c.x && a.y == a.y && b.y == b.y && c.y == c.y;
+    if (num && lx >= -1.0f && hx <= 1.0f && ly >= -1.0f && hy <= 1.0f) {
+        bmin.x = fminf(bmin.x, lx);
+        bmin.y = fminf(bmin.y, ly);
+        bmax.x = fmaxf(bmax.x, hx);
+        bmax.y = fmaxf(bmax.y, hy);
+        return;
+    }
     V2 buf[2][8];
     int cur = 0;
     buf[0][0] = a;
