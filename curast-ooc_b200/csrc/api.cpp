@@ -1195,7 +1195,7 @@ cr_status cr_render(cr_context* ctx, const cr_instance* instances, uint32_t coun
                     uint64_t d_visbuffer, uint64_t d_rgba, uint64_t d_colorbuffer, int32_t display, uint32_t flags,
                     void* stream_) {
     return render_impl(ctx, instances, count, nullptr, cam, d_visbuffer, d_rgba, d_colorbuffer, display, flags,
-                       stream_, 0, ~0ull);
+                       stream_, 0, ~0ull, ResolvePart::Whole, nullptr);
 }
 
 }  // extern "C"
@@ -1214,7 +1214,7 @@ static constexpr uint64_t kDirectBoxes = CR_DIRECT_BOXES;
 cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_t count, const uint64_t* firstIds,
                           const cr_camera* cam, uint64_t d_visbuffer, uint64_t d_rgba, uint64_t d_colorbuffer,
                           int32_t display, uint32_t flags, void* stream_, uint64_t resolveIdLo,
-                          uint64_t resolveIdHi) {
+                          uint64_t resolveIdHi, ResolvePart part, const uint32_t* meshIds) {
     if (!ctx || !cam || (!instances && count)) return fail(CR_ERR_INVALID, "cr_render: NULL argument");
     if (cam->width <= 0 || cam->height <= 0 || (uint64_t)cam->width * cam->height >= (1ull << 31))
         return fail(CR_ERR_INVALID, "cr_render: bad resolution %dx%d", cam->width, cam->height);
@@ -1266,6 +1266,8 @@ cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_
     Assembled A;
     cr_status s = assemble(ctx, instances, count, cam->view, flags, A, firstIds);
     if (s) return s;
+    if (meshIds)
+        for (uint32_t r = 0; r < count; r++) A.inst[r].id = meshIds[A.order[r]];
     float pxPerTriangle = 0.0f;  // screen area the instances' boxes cover per triangle (an estimate)
     {  // whole-mesh classes: fa as the kernels form it (f / aspect in float)
         const float f = cam->proj[5];
@@ -1396,7 +1398,8 @@ cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_
     rp.thrLarge = ctx->cfg.threshold_large;
     rp.idLo = resolveIdLo;
     rp.idHi = resolveIdHi;
-    rp.writeBackground = resolveIdLo == 0 ? 1u : 0u;
+    rp.writeBackground = part == ResolvePart::Later ? 0u : resolveIdLo == 0 ? 1u : 0u;
+    rp.ownOnly = part == ResolvePart::Whole ? 0u : 1u;
     // the resolve, the frame's last kernel, hands the counters to the host
     rp.counters = ctx->counters;
     rp.hostCounters = ctx->hCounters;

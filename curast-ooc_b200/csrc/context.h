@@ -210,12 +210,19 @@ cr_status assemble(cr_context* ctx, const cr_instance* instances, uint32_t count
 // Internal render flag: resolve only (the frame's raster passes are done).
 constexpr uint32_t kRenderResolveOnly = 1u << 31;
 
+// What the resolve of one pass of a multi-pass frame writes: every pixel, or
+// those whose triangle belongs to the pass's own instances (and, in the first
+// pass, the background).
+enum class ResolvePart { Whole, First, Later };
+
 // cr_render with optional explicit first ids; the resolve writes only pixels
 // whose triangle id lies in [resolveIdLo, resolveIdHi) and the background
-// only when resolveIdLo == 0 (multi-pass frames resolve group by group).
+// only when resolveIdLo == 0.  meshIds: the instances' places for the MESH_ID
+// display (null: their places in the list).
 cr_status render_impl(cr_context* ctx, const cr_instance* instances, uint32_t count, const uint64_t* firstIds,
                       const cr_camera* cam, uint64_t d_visbuffer, uint64_t d_rgba, uint64_t d_colorbuffer,
-                      int32_t display, uint32_t flags, void* stream, uint64_t resolveIdLo, uint64_t resolveIdHi);
+                      int32_t display, uint32_t flags, void* stream, uint64_t resolveIdLo, uint64_t resolveIdHi,
+                      ResolvePart part, const uint32_t* meshIds);
 cr_status ensure_queues(cr_context* ctx, uint64_t ntWant, uint64_t hugeWant);
 // (Re)builds a mesh's hierarchical-cull boxes from its current contents.
 cr_status build_mesh_boxes(cr_context* ctx, MeshRec& m);

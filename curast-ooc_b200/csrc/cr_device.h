@@ -330,6 +330,7 @@ struct CrResolveParams {
     uint32_t background;
     uint32_t writeBackground;   // 1: empty pixels get the background
     uint64_t idLo, idHi;        // covered pixels are written only for ids in [idLo, idHi)
+    uint32_t ownOnly;           // 1: and only where the id is a triangle of one of the instances
     float view[16];             // the view matrix (STAGE display)
     uint32_t thrSmall, thrLarge;  // the stage thresholds (STAGE display)
     uint64_t idBase;            // added to a pixel's id to find its instance (batched

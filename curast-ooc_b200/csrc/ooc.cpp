@@ -370,42 +370,71 @@ cr_status cr_ooc_render(cr_ooc* o, const cr_camera* cam, uint64_t d_visbuffer, u
     }
     st.visible_nodes = (uint32_t)order.size();
     st.visible_triangles = sum;
-    // passes of at most numSlots nodes
-    std::vector<std::pair<size_t, size_t>> passes;
-    for (size_t a = 0; a < order.size(); a += o->numSlots) passes.push_back({a, std::min(order.size(), a + o->numSlots)});
-    if (passes.empty()) passes.push_back({0, 0});
+    // passes of at most numSlots nodes, each in draw order.  A frame of several
+    // starts with the nodes that are resident already (the order of the passes is
+    // free: ids are fixed and the visbuffer is a minimum), so that no pass
+    // evicts what a later one would find.
+    // Stage 2 keeps 32 bits of an id (tv.cu:414), so past 2^32 triangles a pixel
+    // may name a node of an earlier pass: such frames resolve after every
+    // raster pass, node groups in draw order.
+    const bool multi = order.size() > o->numSlots;
+    const bool wide = sum > (1ull << 32);
+    std::vector<std::vector<uint32_t>> passes;  // places in `order`
+    if (multi && !wide) {
+        std::vector<uint32_t> first, rest;
+        for (uint32_t k = 0; k < (uint32_t)order.size(); k++) (o->nodes[order[k]].slot >= 0 ? first : rest).push_back(k);
+        const size_t fill = std::min(rest.size(), (size_t)o->numSlots - first.size());
+        first.insert(first.end(), rest.begin(), rest.begin() + fill);
+        std::sort(first.begin(), first.end());
+        passes.push_back(std::move(first));
+        for (size_t a = fill; a < rest.size(); a += o->numSlots)
+            passes.emplace_back(rest.begin() + a, rest.begin() + std::min(rest.size(), a + o->numSlots));
+    } else {
+        for (size_t a = 0; a < order.size(); a += o->numSlots) {
+            passes.emplace_back(std::min(order.size() - a, (size_t)o->numSlots));
+            std::iota(passes.back().begin(), passes.back().end(), (uint32_t)a);
+        }
+        if (passes.empty()) passes.emplace_back();
+    }
     st.passes = (uint32_t)passes.size();
-    const bool multi = passes.size() > 1;
     const bool resolve = !(flags & CR_RENDER_NO_RESOLVE);
-    auto run_pass = [&](size_t p, uint32_t passFlags, uint64_t idLo, uint64_t idHi) -> cr_status {
-        std::vector<uint32_t> nodesP(order.begin() + passes[p].first, order.begin() + passes[p].second);
+    auto run_pass = [&](size_t p, uint32_t passFlags, uint64_t idLo, uint64_t idHi, ResolvePart part) -> cr_status {
+        std::vector<uint32_t> nodesP(passes[p].size());
+        for (size_t k = 0; k < nodesP.size(); k++) nodesP[k] = order[passes[p][k]];
         cr_status ps = make_resident(o, nodesP, stream, st);
         if (ps) return ps;
         std::vector<cr_instance> inst(nodesP.size());
         std::vector<uint64_t> ids(nodesP.size());
+        std::vector<uint32_t> places(nodesP.size());  // MESH_ID: within the cache-sized run of draw order
         for (size_t k = 0; k < nodesP.size(); k++) {
             inst[k].mesh = o->nodes[nodesP[k]].mesh;
             memcpy(inst[k].world, o->nodes[nodesP[k]].desc.world, 64);
-            ids[k] = firstId[passes[p].first + k];
+            ids[k] = firstId[passes[p][k]];
+            places[k] = passes[p][k] % o->numSlots;
         }
         ps = render_impl(o->ctx, inst.data(), (uint32_t)inst.size(), ids.data(), cam, d_visbuffer, d_rgba, 0, display,
-                         passFlags, stream, idLo, idHi);
+                         passFlags, stream, idLo, idHi, part, places.data());
         if (ps) return ps;
         return mark_read(o, nodesP, stream);
     };
-    // raster passes (the first one clears), then -- for several passes -- the
-    // resolve group by group, last group first (it is still resident)
+    // raster passes (the first one clears).  Each pass of several also resolves
+    // the pixels that its own nodes hold by then: a pixel keeps its last
+    // winner's pass's colour, and that winner's geometry is resident in that
+    // pass, where a resolve after all passes would upload the evicted nodes
+    // again.
     const uint32_t keep = flags & (CR_RENDER_SYNC | CR_RENDER_TIMING);
+    const bool late = multi && wide;
     for (size_t p = 0; p < passes.size(); p++) {
-        uint32_t f = keep | (p > 0 ? CR_RENDER_NO_CLEAR : 0u) | ((multi || !resolve) ? CR_RENDER_NO_RESOLVE : 0u);
-        s = run_pass(p, f, 0, ~0ull);
+        uint32_t f = keep | (p > 0 ? CR_RENDER_NO_CLEAR : 0u) | ((late || !resolve) ? CR_RENDER_NO_RESOLVE : 0u);
+        s = run_pass(p, f, 0, ~0ull,
+                     !multi || late ? ResolvePart::Whole : p == 0 ? ResolvePart::First : ResolvePart::Later);
         if (s) return s;
     }
-    if (multi && resolve) {
+    if (late && resolve) {  // last group first (it is still resident)
         for (size_t q = passes.size(); q-- > 0;) {
-            const uint64_t lo = firstId[passes[q].first];
-            const uint64_t hi = q + 1 < passes.size() ? firstId[passes[q + 1].first] : ~0ull;
-            s = run_pass(q, (flags & CR_RENDER_SYNC) | kRenderResolveOnly, lo, hi);
+            const uint64_t lo = firstId[passes[q].front()];
+            const uint64_t hi = q + 1 < passes.size() ? firstId[passes[q + 1].front()] : ~0ull;
+            s = run_pass(q, (flags & CR_RENDER_SYNC) | kRenderResolveOnly, lo, hi, ResolvePart::Whole);
             if (s) return s;
         }
     }

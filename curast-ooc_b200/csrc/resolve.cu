@@ -102,6 +102,8 @@ __device__ __forceinline__ void resolve_pixel(const CrResolveParams& p, const ui
         }
         const CrInstance* I = p.instances + lo;
         const uint32_t nT = __ldg(&I->numTriangles);
+        // a pass of several: the pixel's triangle is another pass's
+        if (p.ownOnly && (tid < __ldg(&I->cum) || tid - __ldg(&I->cum) >= nT)) return;
         uint32_t tri = (uint32_t)(tid - __ldg(&I->cum));
         tri = min(tri, nT - 1u);
         const uint32_t* colors = ldg_ptr(&I->colors);

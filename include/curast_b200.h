@@ -437,8 +437,8 @@ uint32_t cr_scene_class(uint64_t triangles, uint64_t pixels, uint32_t num_views)
  * one frame in the reference's order (triangle count descending, then node
  * index; src/CuRast_render.h:316-345), ids being the prefix sum over the
  * selected nodes.  A selection larger than the cache is drawn in several
- * passes into the same visbuffer with the same ids, then resolved group by
- * group, so the output does not depend on the budget. */
+ * passes into the same visbuffer with the same ids, resolved pass by
+ * pass, so the output does not depend on the budget. */
 #define CR_OOC_MAX_NODE_TRIANGLES 65536u
 
 typedef struct cr_ooc_node {
