@@ -372,24 +372,33 @@ cr_status ensure_queues(cr_context* ctx, uint64_t ntWant, uint64_t hugeWant) {
     return CR_OK;
 }
 
-// The chain heads of the binned stage 3 for a frame of `tiles` screen tiles;
-// without memory for them the frame takes the unbinned stage 3.
+// The chain heads, entry counts and unit list of the binned stage 3 for a frame
+// of `tiles` screen tiles and the current stage-3 queue; without memory for
+// them the frame takes the unbinned stage 3.
 void ensure_bins(cr_context* ctx, uint64_t tiles) {
-    if (tiles <= ctx->binTiles) return;
+    // a unit per tile and per CR_BIN_PART further entries
+    const uint64_t units = tiles + ctx->hugeCap / CR_BIN_PART;
+    if (tiles <= ctx->binTiles && units <= ctx->binUnitCap) return;
     if (cudaDeviceSynchronize() != cudaSuccess) return;
-    const size_t bytes = tiles * CR_BIN_CHAINS * 8;
-    ctx->dev_free(ctx->binHeads, ctx->binTiles * CR_BIN_CHAINS * 8);
+    tiles = std::max(tiles, ctx->binTiles);
+    const size_t hb = tiles * CR_BIN_CHAINS * 8, cb = align_up(tiles * 4, 256), ub = units * sizeof(uint2);
+    ctx->dev_free(ctx->binHeads, ctx->binBytes);
     ctx->binHeads = nullptr;
-    ctx->binTiles = 0;
+    ctx->binTiles = ctx->binUnitCap = 0;
+    ctx->binBytes = 0;
     void* heads = nullptr;
-    if (ctx->dev_alloc(&heads, bytes, "stage-3 bins") != CR_OK) return;
-    if (cudaMemset(heads, 0, bytes) != cudaSuccess) {
+    if (ctx->dev_alloc(&heads, hb + cb + ub, "stage-3 bins") != CR_OK) return;
+    if (cudaMemset(heads, 0, hb + cb) != cudaSuccess) {
         cudaGetLastError();
-        ctx->dev_free(heads, bytes);
+        ctx->dev_free(heads, hb + cb + ub);
         return;
     }
     ctx->binHeads = (unsigned long long*)heads;
+    ctx->binCounts = (uint32_t*)((char*)heads + hb);
+    ctx->binUnits = (uint2*)((char*)heads + hb + cb);
     ctx->binTiles = tiles;
+    ctx->binUnitCap = units;
+    ctx->binBytes = hb + cb + ub;
     ctx->binStamp = 0;
 }
 
@@ -1412,17 +1421,21 @@ cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_
                               (uint64_t)((cam->height + CR_TILE_SIZE - 1) / CR_TILE_SIZE);
     const bool bins = !refMath && count > 0 && !(flags & kRenderResolveOnly) && ctx->cfg.memory_budget == 0 &&
                       cam->width <= 8192 && cam->height <= 8192;
-    if (bins) ensure_bins(ctx, binTiles);
     fp.binTilesX = (uint32_t)((cam->width + CR_TILE_SIZE - 1) / CR_TILE_SIZE);
     fp.binTilesY = (uint32_t)((cam->height + CR_TILE_SIZE - 1) / CR_TILE_SIZE);
 
     auto issue = [&](cudaEvent_t* tev, cudaEvent_t rasterEnd) -> cr_status {
-        if (bins && ctx->binHeads && ctx->hugeCap < 0xffffffffull) {
+        fp.binHeads = nullptr;
+        if (bins && ctx->hugeCap < 0xffffffffull) ensure_bins(ctx, binTiles);  // the queue may have grown
+        if (bins && ctx->hugeCap < 0xffffffffull && ctx->binHeads) {
             if (++ctx->binStamp == 0) {  // the stamps wrapped: empty every chain
                 CR_CUDA(cudaMemsetAsync(ctx->binHeads, 0, ctx->binTiles * CR_BIN_CHAINS * 8, stream), "stage-3 bins");
                 ctx->binStamp = 1;
             }
             fp.binHeads = ctx->binHeads;
+            fp.binCounts = ctx->binCounts;
+            fp.binUnits = ctx->binUnits;
+            fp.binUnitCap = (uint32_t)ctx->binUnitCap;
             fp.binStamp = ctx->binStamp;
         }
         fp.ntList = ctx->ntList;
@@ -1445,7 +1458,9 @@ cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_
         const bool raster = !(flags & kRenderResolveOnly);
         if ((flags & CR_RENDER_NO_CLEAR) || !raster) {
             CR_CUDA(cudaMemsetAsync(ctx->counters, 0, CR_CTR_COUNT * sizeof(unsigned long long), stream), "counters");
-        } else if (cr_launch_clear(fp.fb, numPixels, ctx->counters, stream)) {
+            if (fp.binHeads) CR_CUDA(cudaMemsetAsync(ctx->binCounts, 0, binTiles * 4, stream), "stage-3 bins");
+        } else if (cr_launch_clear(fp.fb, numPixels, ctx->counters, stream, fp.binHeads ? ctx->binCounts : nullptr,
+                                   (uint32_t)binTiles)) {
             return fail(CR_ERR_CUDA, "clear launch: %s", cudaGetErrorString(cudaGetLastError()));
         }
         CR_CUDA(mark(1), "event");

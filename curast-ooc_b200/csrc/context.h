@@ -165,8 +165,13 @@ struct cr_context {
     uint64_t s1Cap = 0;
     CrTile* hugeList = nullptr;
     uint64_t hugeCap = 0;
-    unsigned long long* binHeads = nullptr;   // chain heads of the binned stage 3, binTiles tiles
-    uint64_t binTiles = 0;
+    // binned stage 3, one allocation: chain heads and entry counts of binTiles
+    // tiles, binUnitCap units
+    unsigned long long* binHeads = nullptr;
+    uint32_t* binCounts = nullptr;
+    uint2* binUnits = nullptr;
+    uint64_t binTiles = 0, binUnitCap = 0;
+    size_t binBytes = 0;
     uint32_t binStamp = 0;                    // the last issued frame's stamp (0 is never issued)
     unsigned long long* counters = nullptr;
     unsigned long long* hCounters = nullptr;  // pinned

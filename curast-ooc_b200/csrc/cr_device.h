@@ -42,7 +42,8 @@
 #define CR_CTR_UNITS 7          // item groups the group cull leaves for the item cull
 #define CR_CTR_CGROUPS 8        // chunk groups the group cull leaves for the chunk cull
 #define CR_CTR_VSLICES 9        // slices the vertex pass evaluated (frames with slice stamps)
-#define CR_CTR_S3UNIT 10        // quadrants of screen tiles taken by k_stage3_bins
+#define CR_CTR_S3UNIT 10        // units taken by k_stage3_bins
+#define CR_CTR_BINUNITS 11      // units of the binned stage 3
 #define CR_CTR_COUNT 16
 
 // Compressed geometry (the reference's IX_PU16 meshes, CMesh fields
@@ -169,6 +170,9 @@ struct alignas(16) CrTile {     // HugeTriangle, HostDeviceInterface.h:254-259
 };
 // Binned stage 3: chains per 64x64 screen tile, each a list of queue entries.
 #define CR_BIN_CHAINS 128
+#ifndef CR_BIN_PART
+#define CR_BIN_PART 512         // a tile's entries per unit of work
+#endif
 
 // Stage-2 queue entry: (view << 58) | (instance << 32) | triangle; single-view
 // frames use view 0, i.e. the reference's packing (tv.cu:192-197).
@@ -301,6 +305,9 @@ struct CrFrameParams {
     // CR_BIN_CHAINS chain heads, (stamp << 32) | first queue entry; a head of
     // another stamp is an empty chain, so no frame clears them
     unsigned long long* binHeads;
+    uint32_t* binCounts;        // entries per screen tile (cleared with the visbuffer)
+    uint2* binUnits;            // {tile, its unit's number}, counted in counters[CR_CTR_BINUNITS]
+    uint32_t binUnitCap;
     uint32_t binStamp;
     uint32_t binTilesX, binTilesY;
 };
@@ -379,7 +386,9 @@ struct CrLaunchShape {
 };
 
 int cr_query_launch_shape(int device, CrLaunchShape* out);
-int cr_launch_clear(uint64_t* fb, uint64_t numPixels, unsigned long long* counters, void* stream);
+// binCounts: numTiles entry counts of the binned stage 3, cleared too (or nullptr).
+int cr_launch_clear(uint64_t* fb, uint64_t numPixels, unsigned long long* counters, void* stream,
+                    uint32_t* binCounts = nullptr, uint32_t numTiles = 0);
 int cr_launch_vertex(const CrFrameParams& p, const CrLaunchShape& s, void* stream);
 int cr_launch_stage1(const CrFrameParams& p, const CrLaunchShape& s, void* stream);
 int cr_launch_stage2(const CrFrameParams& p, const CrLaunchShape& s, void* stream);

@@ -25,8 +25,10 @@
 //            (the reference: lane 0 sets up while 31 lanes wait), then per
 //            triangle rows are narrowed to the columns that can pass and
 //            packed across the lanes.               reference: tv.cu:388-563
-//   stage 3  a warp per 64x64 tile or band of its rows (the reference: one
-//            64-thread block per tile), rows narrowed likewise.
+//   stage 3  k_stage3_bins: a block per quadrant of a screen tile and run of its
+//            triangles (stage3_bins.cuh), or k_stage3: a warp per (triangle,
+//            64x64 tile) or band of its rows (the reference: one 64-thread block
+//            per tile), rows narrowed likewise.
 //                                                   reference: tv.cu:568-745
 #include <cuda_runtime.h>
 #include <algorithm>
@@ -948,7 +950,8 @@ __global__ void __launch_bounds__(WARPS * 32, CR_S1_BOXES_MIN_BLOCKS) k_stage1(c
 
 // resolve.cu:213-232 (0xFFFFFFF0'00000000 per pixel), 16-byte stores; block 0
 // also resets the frame's counters.
-__global__ void __launch_bounds__(256) k_clear(uint64_t* fb, uint64_t n, unsigned long long* counters) {
+__global__ void __launch_bounds__(256) k_clear(uint64_t* fb, uint64_t n, unsigned long long* counters,
+                                               uint32_t* binCounts, uint32_t numTiles) {
     // launched the ordinary way (it overwrites what the previous frame's
     // resolve reads); lets the frame cull be scheduled early
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -957,6 +960,7 @@ __global__ void __launch_bounds__(256) k_clear(uint64_t* fb, uint64_t n, unsigne
     const uint64_t n2 = n / 2;
     ulonglong2* v = reinterpret_cast<ulonglong2*>(fb);
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < numTiles; i += stride) binCounts[i] = 0u;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n2; i += stride)
         v[i] = make_ulonglong2(clearv, clearv);
     if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) fb[n - 1] = clearv;
@@ -1027,10 +1031,11 @@ int launch_pdl(Kernel kernel, unsigned grid, unsigned block, void* stream, const
 }
 }  // namespace
 
-int cr_launch_clear(uint64_t* fb, uint64_t numPixels, unsigned long long* counters, void* stream) {
+int cr_launch_clear(uint64_t* fb, uint64_t numPixels, unsigned long long* counters, void* stream, uint32_t* binCounts,
+                    uint32_t numTiles) {
     const uint64_t want = (numPixels / 2 + 255) / 256;
     const unsigned grid = (unsigned)(want < 1 ? 1 : (want > 148 * 16 ? 148 * 16 : want));
-    k_clear<<<grid, 256, 0, (cudaStream_t)stream>>>(fb, numPixels, counters);
+    k_clear<<<grid, 256, 0, (cudaStream_t)stream>>>(fb, numPixels, counters, binCounts, binCounts ? numTiles : 0u);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -1095,9 +1100,7 @@ int cr_launch_stage2(const CrFrameParams& p, const CrLaunchShape& s, void* strea
 
 int cr_launch_stage3(const CrFrameParams& p, const CrLaunchShape& s, void* stream) {
     if (p.binHeads) {
-        const uint64_t units = 4ull * p.binTilesX * p.binTilesY;
-        return launch_pdl(k_stage3_bins, (unsigned)std::min<uint64_t>(units, (uint64_t)s.stage3BinBlocks), B3_THREADS,
-                          stream, p);
+        return launch_pdl(k_stage3_bins, (unsigned)s.stage3BinBlocks, B3_THREADS, stream, p);
     }
     return launch_pdl(k_stage3<S3_WARPS, false>, (unsigned)s.stage3Blocks, S3_WARPS * 32, stream, p);
 }

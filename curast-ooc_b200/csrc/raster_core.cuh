@@ -1267,10 +1267,16 @@ __device__ __forceinline__ void stage2_run(const CrFrameParams& p) {
                             const uint64_t tile = (uint64_t)t.tile_y * p.binTilesX + (uint32_t)t.tile_x;
                             t.tile_x = -1;
                             if (in) {  // always: a triangle's box is clamped to the screen
+                                const uint32_t pos = atomicAdd(&p.binCounts[tile], 1u);
                                 const unsigned long long prev = atomicExch(
-                                    &p.binHeads[tile * CR_BIN_CHAINS + (slot & (CR_BIN_CHAINS - 1))],
+                                    &p.binHeads[tile * CR_BIN_CHAINS + (pos & (CR_BIN_CHAINS - 1))],
                                     ((unsigned long long)p.binStamp << 32) | slot);
                                 if ((uint32_t)(prev >> 32) == p.binStamp) t.tile_x = (int32_t)(uint32_t)prev;
+                                if (pos % CR_BIN_PART == 0) {
+                                    const unsigned long long un = atomicAdd(&p.counters[CR_CTR_BINUNITS], 1ull);
+                                    if (un < p.binUnitCap)
+                                        p.binUnits[un] = make_uint2((uint32_t)tile, pos / CR_BIN_PART);
+                                }
                             }
                         }
                         p.hugeList[slot] = t;

@@ -6,17 +6,16 @@
 // lies in front of it.  What bounds that is the work on hidden fragments: in
 // a frame of 375K tiles over 510 screen tiles a pixel is traced hundreds of
 // times.  Here stage 2 links each queued tile into one of CR_BIN_CHAINS
-// chains of its screen tile, and a block takes a quadrant (32x32 pixels) of
-// one screen tile with all of its triangles:
-//   * the words live in shared memory (a warp owns 16x8 pixels), loaded once
-//     and merged into the visbuffer by at most one atomic minimum per pixel:
+// chains of its screen tile and starts a unit of work for every CR_BIN_PART of a
+// tile's entries; a block takes a unit -- an even share of one screen tile's
+// chains, over one quadrant of the tile -- a warp per region of 16x8 pixels:
+//   * a region's words live in shared memory, loaded once and merged into the visbuffer by at most one atomic minimum per pixel:
 //     the word kept is the minimum of the same candidates;
 //   * the pixel's ray (two divisions, a square root) is formed once per pixel
 //     instead of once per fragment: it does not depend on the triangle;
-//   * a triangle is first tested against the warp's 16x8 pixels, 32 triangles
-//     at a time (a lane per triangle): dropped where no pixel can pass
-//     intersect_mt, or where no word it could write is below the words
-//     already there (bin_rejects);
+//   * a triangle is first tested against the region, 32 triangles at a time (a
+//     lane per triangle): dropped where no pixel can pass intersect_mt, or
+//     where no word it could write is below the words already there (bin_test);
 //   * four triangles that are left find their eight rows' spans at once (a
 //     lane per row, bin_row_span, in float), and the spans' pixels are packed
 //     across the lanes; where they fill most of the region the warp steps
@@ -24,12 +23,13 @@
 // Every fragment left runs the float test of k_stage3 unchanged, so the
 // visbuffer is the same bit for bit.
 // Measured (B200, stage 3): 60K-triangle soup at 1917x1083 (375K tiles) 4.90 ->
-// 0.29 ms; 2M-triangle compressed heightfield at 2560x1440 (348K) 0.85 -> 0.40; 1M
-// heightfield at 1080p (26.6K) 0.117 -> 0.086.  Three blocks per SM (79 registers);
-// four spill (heightfield 0.097, compressed 0.43).  The pixels' words in registers
-// and a quarter of a region per step, without row spans, cost slivers more
-// (heightfield 0.156, compressed 0.75, soup 0.23); taking the next unit's ticket
-// while working on one made the tail longer (heightfield 0.102, compressed 0.55).
+// 0.275 ms; 2M-triangle compressed heightfield at 2560x1440 (348K) 0.85 -> 0.300; 1M
+// heightfield at 1080p (26.6K) 0.117 -> 0.054.  One unit per quadrant whatever the
+// length of the tile's list left a tail of a few long lists (0.29, 0.40, 0.086: 24 % of
+// the warps active, 4.5 warps per issue at a barrier); a unit's four quadrants one
+// after the other in one block, its triangles set up once, made short queues serial
+// (0.29, 0.46, 0.076; 60 tiles of a planet frame 0.025 instead of 0.010).  The pixels'
+// words in registers, without row spans, cost slivers more (0.23, 0.75, 0.156).
 #pragma once
 #include "raster_core.cuh"
 
@@ -46,8 +46,8 @@ constexpr int B3_W = 16, B3_H = 8;  // a warp's pixels
 #ifndef B3_DENSE
 #define B3_DENSE 80
 #endif
-constexpr int B3_BATCH = 2 * CR_BIN_CHAINS;  // triangles set up per round: two links of every chain
-static_assert(B3_BATCH == B3_THREADS, "a thread sets up one triangle of a round");
+constexpr int B3_BATCH = 256;  // triangles set up per round
+static_assert(B3_BATCH >= CR_BIN_CHAINS && B3_BATCH <= B3_THREADS, "a link of every chain fits a round, a thread per triangle");
 
 // A pixel column passes intersect_mt for a triangle only if (see S3Prune) with
 // d = (rx, ry, -1) the unnormalised ray, s the sign of T = e2 . (tvec x e1),
@@ -101,19 +101,19 @@ __device__ __forceinline__ float corner_max(const float (*t)[B3_BATCH], int row,
     return (fmaxf(nx * x0, nx * x1) + fmaxf(ny * y0, ny * y1)) - nz;
 }
 
-// True if triangle j of the round cannot change a pixel of the region:
-// zmax is the greatest high half of the region's words.
-__device__ __forceinline__ bool bin_rejects(const float (*t)[B3_BATCH], int j, float x0, float x1, float y0, float y1,
-                                            uint32_t zmax) {
+// Whether triangle j of the round can hit a pixel of the region, and the least
+// high half of a word that it can write there (0: no bound): a word's high
+// half is (depth bits & ~7) << 1 | four id bits.
+__device__ __forceinline__ bool bin_test(const float (*t)[B3_BATCH], int j, float x0, float x1, float y0, float y1,
+                                         uint32_t& zlow) {
     const float mD = t[BT_MD][j], mU = t[BT_MU][j], mV = t[BT_MV][j];
     const float D = corner_max(t, BT_N1, j, x0, x1, y0, y1);
     const float U = corner_max(t, BT_N2, j, x0, x1, y0, y1);
     const float V = corner_max(t, BT_Q, j, x0, x1, y0, y1);
     const float K = corner_max(t, BT_K, j, x0, x1, y0, y1);
-    if (D < -mD || U < -mU || V < -mV || K < -(mD + mU + mV)) return true;
-    // the high half of a word is (depth bits & ~7) << 1 | four id bits
     const uint32_t low = __float_as_uint(__fdividef(t[BT_T][j], D + mD));
-    return low > 0x0da24260u && low <= 0x7f800000u && ((low & 0x7ffffff8u) << 1) > zmax;  // zlow > 1e-30, not NaN
+    zlow = low > 0x0da24260u && low <= 0x7f800000u ? (low & 0x7ffffff8u) << 1 : 0u;  // above 1e-30, not NaN
+    return !(D < -mD || U < -mU || V < -mV || K < -(mD + mU + mV));
 }
 
 // Columns [lo, lo + len) of a region row that can pass: column c of the row
@@ -232,7 +232,8 @@ __global__ void __launch_bounds__(B3_THREADS, B3_MINB) k_stage3_bins(const CrFra
     __shared__ uint8_t s_ring[B3_WARPS][64];
     __shared__ uint32_t s_unit, s_n;
     const uint64_t count = min((uint64_t)p.counters[CR_CTR_HUGE], p.hugeCap);
-    if (count == 0) return;
+    const uint64_t units = 4ull * min((uint64_t)p.counters[CR_CTR_BINUNITS], (uint64_t)p.binUnitCap);
+    if (units == 0) return;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const Target tg = target_of(p);
     const float Wf = (float)tg.W, Hf = (float)tg.H;
@@ -244,44 +245,48 @@ __global__ void __launch_bounds__(B3_THREADS, B3_MINB) k_stage3_bins(const CrFra
     const float Dn = 1.0f + fabsf(ifa) * um + fabsf(iff) * vm;
     const float A = 2.0f * ifa / Wf;  // the ray's x step per column
     const int numPixels = tg.W * tg.H;
-    const uint32_t units = 4u * tilesX * tilesY;
     unsigned long long* const word = s_word[w];
     uint8_t* const ring = s_ring[w];
+    // the reference's per-pixel ray (tv.cu:690-705)
+    auto ray_x = [&](int px) { return ifa * (2.0f * ((float)px + 0.5f) / Wf - 1.0f); };
+    auto ray_y = [&](int py) { return iff * (2.0f * ((float)py + 0.5f) / Hf - 1.0f); };
     while (true) {
         // taken only when the block is free for it: the units differ widely
         if (tid == 0) s_unit = (uint32_t)atomicAdd(&p.counters[CR_CTR_S3UNIT], 1ull);
         __syncthreads();
         const uint32_t unit = s_unit;
         if (unit >= units) return;
-        const uint32_t tile = unit >> 2;
-        // each of the first CR_BIN_CHAINS threads follows one chain
+        const uint2 un = p.binUnits[unit >> 2];
+        const uint32_t tile = un.x;
+        // this unit's chains: those of its number, modulo the tile's units
+        const uint32_t parts =
+            min((p.binCounts[tile] + CR_BIN_PART - 1) / (uint32_t)CR_BIN_PART, (uint32_t)CR_BIN_CHAINS);
         uint32_t cur = 0xffffffffu;
-        if (tid < CR_BIN_CHAINS) {
+        if (tid < CR_BIN_CHAINS && un.y < parts && tid % parts == un.y) {
             const unsigned long long h = p.binHeads[(uint64_t)tile * CR_BIN_CHAINS + tid];
             if ((uint32_t)(h >> 32) == p.binStamp) cur = (uint32_t)h;
         }
-        if (!__syncthreads_or(cur != 0xffffffffu)) continue;
-        // the chain's next entry is loaded ahead of its use, while the warp
-        // reads its pixels or works on a round
+        // the chain's next entry is loaded ahead of its use
         CrTile ahead = {};
         if (cur < p.hugeCap) ahead = p.hugeList[cur];
+        // this warp's region of the quadrant
         const int x0 = (int)(tile % tilesX) * CR_TILE_SIZE + (int)(unit & 1u) * 32 + (w & 1) * B3_W;
         const int y0 = (int)(tile / tilesX) * CR_TILE_SIZE + (int)((unit >> 1) & 1u) * 32 + (w >> 1) * B3_H;
-        // the reference's per-pixel ray (tv.cu:690-705)
-        auto ray_x = [&](int px) { return ifa * (2.0f * ((float)px + 0.5f) / Wf - 1.0f); };
-        auto ray_y = [&](int py) { return iff * (2.0f * ((float)py + 0.5f) / Hf - 1.0f); };
+        const float wx0 = ray_x(x0), wx1 = ray_x(x0 + B3_W - 1);
+        const float wy0 = ray_y(y0), wy1 = ray_y(y0 + B3_H - 1);
         // pixel lane + 32 m of the region, rows of 16: column lane & 15, row
-        // (lane >> 4) + 2 m.  Columns past the right edge wrap into the next
-        // row, as the reference's pixel index does; rows past the end are not
-        // written (their word 0 is never undercut).
+        // (lane >> 4) + 2 m.  Columns past the right edge wrap into the next row,
+        // as the reference's pixel index does; rows past the end are not written
+        // (their word 0 is never undercut).
         const int pid0 = x0 + (lane & 15) + tg.W * (y0 + (lane >> 4));
         const float myDx = ray_x(x0 + (lane & 15));
         if (lane < B3_W) s_dx[w][lane] = myDx;
         if (lane < B3_H) s_dy[w][lane] = ray_y(y0 + lane);
+        __syncwarp();
         uint32_t zw = 0;  // the greatest high half of the region's words
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
-            const V3 d = {myDx, ray_y(y0 + (lane >> 4) + 2 * m), -1.0f};
+            const V3 d = {myDx, s_dy[w][(lane >> 4) + 2 * m], -1.0f};
             s_inv[w][lane + 32 * m] = 1.0f / sqrtf(dot3(d, d));
             const int pid = pid0 + 2 * m * tg.W;
             const uint64_t v = pid < numPixels ? p.fb[pid] : 0ull;
@@ -290,15 +295,15 @@ __global__ void __launch_bounds__(B3_THREADS, B3_MINB) k_stage3_bins(const CrFra
         }
         zw = __reduce_max_sync(FULL, zw);
         __syncwarp();
-        const float wx0 = s_dx[w][0], wx1 = s_dx[w][B3_W - 1], wy0 = s_dy[w][0], wy1 = s_dy[w][B3_H - 1];
         const float rowY = s_dy[w][lane & 7];
-        // two links of every chain per round; a chain holds each entry once,
-        // so no walk is longer than the queue
+        bool touched = false;
+        // a chain holds each entry once, so no walk is longer than the queue
         for (uint64_t walked = 0; walked <= count; ++walked) {
             if (tid == 0) s_n = 0;
-            __syncthreads();
-#pragma unroll
-            for (int step = 0; step < 2; ++step) {
+            int live = __syncthreads_count(cur < p.hugeCap);
+            if (live == 0) break;
+            // links of the live chains, while another of each fits
+            for (int n = 0; live > 0 && n + live <= B3_BATCH;) {
                 const bool on = cur < p.hugeCap;  // 0xffffffff: the chain's end
                 const unsigned mk = __ballot_sync(FULL, on);
                 uint32_t b = 0;
@@ -309,8 +314,9 @@ __global__ void __launch_bounds__(B3_THREADS, B3_MINB) k_stage3_bins(const CrFra
                     cur = (uint32_t)ahead.tile_x;  // the next entry of the chain
                     if (cur < p.hugeCap) ahead = p.hugeList[cur];
                 }
+                n += live;
+                live = __syncthreads_count(cur < p.hugeCap);
             }
-            __syncthreads();
             const int n = (int)s_n;
             if (tid < n) {
                 CrTile e;
@@ -370,6 +376,7 @@ __global__ void __launch_bounds__(B3_THREADS, B3_MINB) k_stage3_bins(const CrFra
                 }
                 qh += (uint32_t)k4;
                 if (__any_sync(FULL, changed)) {
+                    touched = true;
                     __syncwarp();
                     uint32_t z = 0;
 #pragma unroll
@@ -379,23 +386,25 @@ __global__ void __launch_bounds__(B3_THREADS, B3_MINB) k_stage3_bins(const CrFra
                 __syncwarp();
             };
             for (int base = 0; base < n; base += 32) {
-                const int j0 = base + lane;
-                const bool keep = j0 < n && !bin_rejects(s_t, j0, wx0, wx1, wy0, wy1, zw);
+                const int j = base + lane;
+                uint32_t zlow = 0;
+                const bool keep = j < n && bin_test(s_t, j, wx0, wx1, wy0, wy1, zlow) && zlow <= zw;
                 const unsigned mask = __ballot_sync(FULL, keep);
-                if (keep) ring[(qt + __popc(mask & ((1u << lane) - 1u))) & 63u] = (uint8_t)j0;
+                if (keep) ring[(qt + __popc(mask & ((1u << lane) - 1u))) & 63u] = (uint8_t)j;
                 qt += (uint32_t)__popc(mask);
                 __syncwarp();
                 while (qt - qh >= 4u) four();
             }
             if (qt != qh) four();
-            if (!__syncthreads_or(cur < p.hugeCap)) break;
         }
+        if (touched)
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            const int pid = pid0 + 2 * m * tg.W;
-            const uint64_t v = word[lane + 32 * m];
-            if (pid < numPixels && v < p.fb[pid]) fb_min(p.fb, (uint32_t)pid, v);
-        }
+            for (int m = 0; m < 4; ++m) {
+                const int pid = pid0 + 2 * m * tg.W;
+                const uint64_t v = word[lane + 32 * m];
+                if (pid < numPixels && v < p.fb[pid]) fb_min(p.fb, (uint32_t)pid, v);
+            }
+        __syncwarp();
     }
 }
 
