@@ -315,8 +315,7 @@ cr_status assemble(cr_context* ctx, const cr_instance* instances, uint32_t count
             s.itemSlices = m.itemSlices;
             s.subObbs = m.subObbs;
             s.itemObbs = m.itemObbs;
-            s.localLists = m.localLists;
-            s.localCounts = m.localCounts;
+            s.subCones = m.subCones;
             s.groupBoxes = m.groupBoxes;
             A.seg.push_back(s);
         }
@@ -448,58 +447,58 @@ cr_status build_mesh_boxes(cr_context* ctx, MeshRec& m) {
 
 static void free_sub_obbs(cr_context* ctx, MeshRec& m) {
     ctx->dev_free(m.subObbs, m.subBytes);
-    m.subObbs = nullptr;
+    m.subObbs = m.subCones = nullptr;
     m.subBytes = 0;
 }
 
-// Per-item vertex lists of an indexed mesh, built once on first use (a
-// budget or allocation failure leaves them absent: the frame then draws
-// without them, with the same output).
-void ensure_local_lists(cr_context* ctx, MeshRec& m) {
-    if (m.localTried || !m.indices || m.numTriangles == 0) return;
-    m.localTried = true;
-    const size_t nItems = (m.numTriangles + CR_BATCH - 1) / CR_BATCH;
-    const size_t lb = align_up(nItems * CR_LOCAL_BYTES, 256);
-    const size_t bytes = lb + align_up(nItems * 4, 256);
-    if (ctx->dev_alloc((void**)&m.localLists, bytes, "vertex lists") != CR_OK) {
-        cr_internal_set_error("");
-        m.localLists = nullptr;
-        return;
-    }
-    m.localCounts = (uint32_t*)(m.localLists + lb);
-    m.localBytes = bytes;
-    if (cr_launch_local_lists(m.indices, m.compressed ? m.dCodec : nullptr, m.numTriangles, m.localLists,
-                              m.localCounts, 0) ||
-        cudaDeviceSynchronize() != cudaSuccess) {
-        ctx->dev_free(m.localLists, m.localBytes);
-        m.localLists = nullptr;
-        m.localCounts = nullptr;
-        m.localBytes = 0;
-    }
-}
-
-// The oriented sub-boxes of a mesh that box-culled frames draw, built once on
-// first use (absent after a failure: the frame then draws every triangle of
+// The oriented sub-boxes of a mesh that box-culled or batched frames draw,
+// built once on first use (absent after a failure: the frame then draws every triangle of
 // its listed items, with the same output).
 void ensure_sub_obbs(cr_context* ctx, MeshRec& m) {
     if (m.subTried || m.numTriangles == 0) return;
     m.subTried = true;
-    const size_t bytes = (size_t)((m.numTriangles + CR_SUB - 1) / CR_SUB) * CR_OBB_F4 * 16;
+    const size_t n = (m.numTriangles + CR_SUB - 1) / CR_SUB, ob = n * CR_OBB_F4 * 16;
+    const size_t bytes = ob + n * CR_CONE_FLOATS * 4;
     if (ctx->dev_alloc((void**)&m.subObbs, bytes, "oriented sub-boxes") != CR_OK) {
         cr_internal_set_error("");
         m.subObbs = nullptr;
         return;
     }
     m.subBytes = bytes;
-    if (cr_launch_sub_obbs(m.indices, m.positions, m.compressed ? m.dCodec : nullptr, m.numTriangles, m.subObbs, 0) ||
+    m.subCones = (float4*)((char*)m.subObbs + ob);
+    if (cr_launch_sub_obbs(m.indices, m.positions, m.compressed ? m.dCodec : nullptr, m.numTriangles, m.subObbs,
+                           (float*)m.subCones, 0) ||
         cudaDeviceSynchronize() != cudaSuccess)
         free_sub_obbs(ctx, m);
 }
 
-void ensure_local_lists_for(cr_context* ctx, const cr_instance* instances, uint32_t count) {
+// Whether every mesh of the frame has its sub-boxes, or can get them and leave
+// as much device memory again and a gigabyte (a frame that would not be
+// box-culled otherwise has none to lose for them).
+bool sub_obbs_fit(cr_context* ctx, const cr_instance* instances, uint32_t count) {
+    size_t need = 0;
+    for (uint32_t i = 0; i < count; i++) {
+        if (instances[i].mesh >= ctx->meshes.size()) return false;
+        const MeshRec& m = ctx->meshes[instances[i].mesh];
+        if (!m.live || !m.itemObbs || m.subDeclined || (m.subTried && !m.subObbs)) return false;
+        if (!m.subObbs) need += (size_t)((m.numTriangles + CR_SUB - 1) / CR_SUB) * (CR_OBB_F4 * 16 + CR_CONE_FLOATS * 4);
+    }
+    if (need == 0) return true;
+    size_t freeBytes = 0, total = 0;
+    const bool fits = ctx->cfg.memory_budget == 0 && cudaMemGetInfo(&freeBytes, &total) == cudaSuccess &&
+                      freeBytes > 2 * need + (1ull << 30);
+    if (!fits)
+        for (uint32_t i = 0; i < count; i++) {
+            MeshRec& m = ctx->meshes[instances[i].mesh];
+            if (!m.subObbs) m.subDeclined = true;  // not asked again every frame
+        }
+    return fits;
+}
+
+void ensure_sub_obbs_for(cr_context* ctx, const cr_instance* instances, uint32_t count) {
     for (uint32_t i = 0; i < count; i++) {
         const uint32_t m = instances[i].mesh;
-        if (m < ctx->meshes.size() && ctx->meshes[m].live) ensure_local_lists(ctx, ctx->meshes[m]);
+        if (m < ctx->meshes.size() && ctx->meshes[m].live) ensure_sub_obbs(ctx, ctx->meshes[m]);
     }
 }
 
@@ -597,8 +596,10 @@ void read_counters(cr_context* ctx) {
     ctx->last.vertex_slices_evaluated =
         !ctx->last.vertex_chunks ? 0 : ctx->lastStamps ? c[CR_CTR_VSLICES] : c[CR_CTR_CHUNKS] * (CR_VCHUNK / CR_VSLICE);
     ctx->last.stage1_survivors = c[CR_CTR_SURVIVORS];
-    if (ctx->lastDirect) {  // nothing culled ahead of the per-triangle path
+    if (ctx->lastDirect) {  // nothing culled ahead of the per-triangle path: every vertex evaluated there
         ctx->last.work_items_drawn = ctx->last.work_items;
+        ctx->last.vertex_chunks_evaluated = ctx->last.vertex_chunks;
+        ctx->last.vertex_slices_evaluated = ctx->last.vertex_chunks ? ctx->lastDirectSlices : 0;
         ctx->last.stage1_survivors = ctx->lastDirect;
     }
 }
@@ -785,7 +786,6 @@ cr_status cr_destroy(cr_context* ctx) {
             }
         }
         if (m.itemBoxes) cudaFree(m.itemBoxes);
-        if (m.localLists) cudaFree(m.localLists);
         if (m.subObbs) cudaFree(m.subObbs);
     }
     if (ctx->itemList) cudaFree(ctx->itemList);
@@ -1140,7 +1140,6 @@ cr_status cr_mesh_destroy(cr_context* ctx, uint32_t mesh) {
     cudaDeviceSynchronize();
     if (m.owned) free_mesh_arrays(ctx, m);
     ctx->dev_free(m.itemBoxes, m.boxBytes);
-    ctx->dev_free(m.localLists, m.localBytes);
     ctx->dev_free(m.subObbs, m.subBytes);
     m = MeshRec{};
     return CR_OK;
@@ -1151,13 +1150,10 @@ cr_status cr_mesh_refresh(cr_context* ctx, uint32_t mesh) {
     CR_CUDA(cudaSetDevice(ctx->device), "cudaSetDevice");
     CR_CUDA(cudaDeviceSynchronize(), "mesh refresh");
     MeshRec& m = ctx->meshes[mesh];
-    ctx->dev_free(m.localLists, m.localBytes);  // rebuilt on next use
-    m.localLists = nullptr;
-    m.localCounts = nullptr;
-    m.localBytes = 0;
-    m.localTried = false;
-    free_sub_obbs(ctx, m);  // likewise
-    m.subTried = false;
+    // in place: a captured plan may read them
+    if (m.subObbs && cr_launch_sub_obbs(m.indices, m.positions, m.compressed ? m.dCodec : nullptr, m.numTriangles,
+                                        m.subObbs, (float*)m.subCones, 0))
+        return fail(CR_ERR_CUDA, "sub-box launch: %s", cudaGetErrorString(cudaGetLastError()));
     return build_mesh_boxes(ctx, m);
 }
 
@@ -1210,15 +1206,12 @@ cr_status cr_render(cr_context* ctx, const cr_instance* instances, uint32_t coun
 }  // extern "C"
 
 // Frames of at most this many triangles take every triangle straight through
-// the per-triangle path (CrFrameParams::direct).
-#ifndef CR_DIRECT_RECORDS
-#define CR_DIRECT_RECORDS (1ull << 17)
-#endif
-#ifndef CR_DIRECT_BOXES
-#define CR_DIRECT_BOXES (4ull << 20)
-#endif
-static constexpr uint64_t kDirectRecords = CR_DIRECT_RECORDS;
-static constexpr uint64_t kDirectBoxes = CR_DIRECT_BOXES;
+// the per-triangle path (CrFrameParams::direct).  Below it the five kernels that
+// decide which triangles not to draw cost more than drawing them: planets of
+// sub-pixel triangles at 1280x720, culled / direct: 200K 95.7 / 71.3 us, 1M 110 / 85, 4M
+// 119 / 111, 8M 126 / 159 (seen whole: 61 / 35, 75 / 48, 93 / 87, 113 / 146); instances, 30 x
+// 1,000 136 / 28, 300 x 5,000 172 / 79, 100 x 50,000 91 / 101, 10 x 1M 62 / 154.
+static constexpr uint64_t kDirectLimit = 4ull << 20;
 
 cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_t count, const uint64_t* firstIds,
                           const cr_camera* cam, uint64_t d_visbuffer, uint64_t d_rgba, uint64_t d_colorbuffer,
@@ -1235,7 +1228,7 @@ cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_
 
     // what stage 1 culls from: one outcode byte or one 8-byte cell record per
     // (instance, vertex), or (no records) box proofs of the sample-miss cull
-    // and per-item vertex lists; the choice changes speed only, never the output
+    // on oriented boxes and single triangles; the choice changes speed only, never the output
     const uint32_t rec = ctx->cfg.cull_records;
     // the reference build's arithmetic: no records, no culling proofs
     const bool refMath = (flags & (CR_RENDER_REF_MATH | CR_RENDER_REF_MATH_NO_FMA)) != 0;
@@ -1256,21 +1249,19 @@ cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_
         cellMode = CR_REC_OUTCODES;  // cells hold 16-bit coordinates
     else if (cellMode == CR_REC_CELLS && cam->width <= 4096 && cam->height <= 4096)
         cellMode = CR_REC_CELLS32;  // 12-bit coordinates fit: half the record bytes
-    const bool boxes = cellMode == CR_REC_BOXES;
+    // the failure-detection hook drops an index-tile copy, which box-culled
+    // frames do not make
+    if (ctx->cfg.debug_flags && cellMode == CR_REC_BOXES && !refMath)
+        cellMode = cam->width <= 4096 && cam->height <= 4096 ? CR_REC_CELLS32 : CR_REC_OUTCODES;
+    bool boxes = cellMode == CR_REC_BOXES;
     uint64_t triangles = 0;
     for (uint32_t i = 0; i < count; i++)
         if (instances[i].mesh < ctx->meshes.size()) triangles += ctx->meshes[instances[i].mesh].numTriangles;
-    const uint64_t directLimit = boxes ? kDirectBoxes : kDirectRecords;
     // explicit ids may have gaps, a forced record mode is kept, and the
     // failure-detection hook drops a copy that the direct path does not make
     const bool mayDirect = rec == CR_CULL_AUTO && !refMath && !firstIds && count > 0 && triangles > 0 &&
                            !(flags & kRenderResolveOnly) && ctx->cfg.debug_flags == 0;
-    bool direct = mayDirect && triangles <= directLimit;
-    if (boxes && !direct && !refMath && !(flags & kRenderResolveOnly))
-        for (uint32_t i = 0; i < count; i++) {
-            const uint32_t m = instances[i].mesh;
-            if (m < ctx->meshes.size() && ctx->meshes[m].live) ensure_sub_obbs(ctx, ctx->meshes[m]);
-        }
+    bool direct = mayDirect && triangles <= kDirectLimit;
 
     Assembled A;
     cr_status s = assemble(ctx, instances, count, cam->view, flags, A, firstIds);
@@ -1292,6 +1283,24 @@ cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_
         }
         if (tris > 0.0) pxPerTriangle = (float)(area / tris);
         if (mayDirect && !boxes && inside && pxPerTriangle >= 0.5f) direct = true;
+    }
+    // Frames of mostly sub-pixel triangles are box-culled too, where their meshes'
+    // oriented sub-boxes exist or find room: stage 1's tests of 16 triangles and of
+    // single ones need no per-vertex records.  400M planet at 1080p, vertex pass and
+    // stage 1 from records / cull and stage 1 from boxes: from its surface 203 / 164 us, seen
+    // whole 1,130 / 625.  Frames whose triangles cover half a pixel and more keep the records
+    // and their warp-wide raster.
+    if (mayDirect && !direct && !boxes && pxPerTriangle < 0.5f && sub_obbs_fit(ctx, instances, count)) {
+        boxes = true;
+        cellMode = CR_REC_BOXES;
+    }
+    if (boxes && !direct && !refMath && !(flags & kRenderResolveOnly)) {
+        ensure_sub_obbs_for(ctx, instances, count);
+        for (CrSegment& sg : A.seg) {
+            const MeshRec& m = ctx->meshes[instances[A.order[sg.firstInstance]].mesh];
+            sg.subObbs = m.subObbs;
+            sg.subCones = m.subCones;
+        }
     }
     // frame tables, queues and counters are shared by consecutive frames,
     // which may be issued on different streams
@@ -1370,6 +1379,9 @@ cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_
     ctx->lastStamps = stamps;
     fp.direct = direct ? A.totalTriangles : 0;
     ctx->lastDirect = fp.direct;
+    ctx->lastDirectSlices = 0;
+    for (const CrInstance& I : A.inst) ctx->lastDirectSlices += (I.numVertices + CR_VSLICE - 1) / CR_VSLICE;
+    const uint64_t directChunks = direct && !boxes ? A.numVChunks : 0;
     if (boxes || direct) {  // no vertex pass: no chunks to classify or evaluate
         fp.chunkList = nullptr;
         fp.chunkClass = nullptr;
@@ -1498,7 +1510,7 @@ cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_
     };
     const bool culled = fp.itemList && !refMath && !(flags & kRenderResolveOnly);
     return run_frame(ctx, flags, stream, count, A.totalTriangles, issue, culled ? A.numItems : 0,
-                     culled ? fp.numVChunks : 0);
+                     culled ? fp.numVChunks + directChunks : 0);
 }
 
 extern "C" {

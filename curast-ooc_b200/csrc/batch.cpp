@@ -48,16 +48,17 @@ TableLayout layout_of(size_t n, size_t m, size_t V) {
 // One device allocation per batched frame holds the vertex pass's records
 // and the frame cull's outputs.
 struct CullLayout {
-    size_t oChunkMasks, oUniform, oChunkList, oItems, total;
+    size_t oChunkMasks, oUniform, oChunkList, oItems, oProof, total;
 };
 
-CullLayout cull_layout(const Assembled& A) {
+CullLayout cull_layout(const Assembled& A, size_t V) {
     CullLayout L;
     L.oChunkMasks = align_up(A.outBytes * sizeof(CrViewMasks), 256);
     L.oUniform = align_up(L.oChunkMasks + A.numVChunks * sizeof(CrViewMasks), 256);
     L.oChunkList = align_up(L.oUniform + A.numVChunks, 256);
     L.oItems = align_up(L.oChunkList + A.numVChunks * 4, 256);
-    L.total = align_up(L.oItems + A.numItems * sizeof(CrItemViews), 256) + 256;
+    L.oProof = align_up(L.oItems + A.numItems * sizeof(CrItemViews), 256);
+    L.total = align_up(L.oProof + V * A.inst.size() * 32, 256) + 256;
     return L;
 }
 
@@ -69,11 +70,17 @@ void bind_cull(const Assembled& A, const CullLayout& L, void* base, CrFrameParam
     fp.chunkList = (uint32_t*)(b + L.oChunkList);
     fp.itemViews = (CrItemViews*)(b + L.oItems);
     fp.itemCap = A.numItems;
+    fp.viewProof = (float4*)(b + L.oProof);
+    fp.instProof = fp.viewProof;
 }
 
-// Vertex-list stage 1 (k_stage1_views_lists; no vertex pass) for views whose
-// pixel cells fit the 12-bit cell records.
-void use_lists(const BatchTables& B, CrFrameParams& fp) {
+// Stage 1 from oriented sub-boxes (k_stage1_views_boxes; no vertex pass) for
+// views of at most 4096 pixels a side (in larger ones a box's rounding margin
+// nears a pixel).  Its form for half a window pixel and more per triangle: the
+// crossing lies between 0.2, where testing triangles first is 3 % faster, and 0.9,
+// where it is 13 % slower (figures at the kernel).
+void use_boxes(const BatchTables& B, uint64_t triangles, CrFrameParams& fp) {
+    fp.coopRaster = 2.0 * (double)B.sumPixels >= (double)triangles * (double)B.views.size() ? 1u : 0u;
     if (B.maxW > 4096 || B.maxH > 4096) return;
     fp.cellMode = CR_REC_BOXES;
     fp.chunkList = nullptr;
@@ -306,7 +313,7 @@ cr_status render_batch(cr_context* ctx, const cr_instance* instances, uint32_t c
     cr_status s = check_views(views, nv, flags);
     if (s) return s;
     CR_CUDA(cudaSetDevice(ctx->device), "cudaSetDevice");
-    ensure_local_lists_for(ctx, instances, count);
+    ensure_sub_obbs_for(ctx, instances, count);
     Assembled A;
     s = sets ? assemble(ctx, instances, count, views[0].camera.view, flags | CR_RENDER_KEEP_ORDER, A,
                         sets->firstIds.data())
@@ -321,7 +328,7 @@ cr_status render_batch(cr_context* ctx, const cr_instance* instances, uint32_t c
         if (s) return s;
     }
     CR_CUDA(cudaStreamWaitEvent(stream, ctx->frameDone, 0), "stream wait");
-    const CullLayout CL = cull_layout(A);
+    const CullLayout CL = cull_layout(A, nv);
     s = ensure_records(ctx, CL.total);
     if (s) return s;
 
@@ -353,7 +360,7 @@ cr_status render_batch(cr_context* ctx, const cr_instance* instances, uint32_t c
     bind_tables(A, B, L, (char*)ctx->dFrame, fp, rp);
     base_params(ctx, display, fp, rp);
     bind_cull(A, CL, ctx->outcodes, fp);
-    use_lists(B, fp);
+    use_boxes(B, A.totalTriangles, fp);
     fp.counters = ctx->counters;
     auto issue = [&](cudaEvent_t* tev, cudaEvent_t rasterEnd) -> cr_status {
         fp.ntList = ctx->ntList;
@@ -375,7 +382,7 @@ cr_status cr::scratch_issue(cr_context* ctx, BatchScratch& S, const cr_instance*
                             const cr_view* views, uint32_t nv, int32_t display, uint32_t flags, cudaStream_t stream) {
     cr_status s = check_views(views, nv, flags);
     if (s) return s;
-    ensure_local_lists_for(ctx, instances, count);
+    ensure_sub_obbs_for(ctx, instances, count);
     Assembled A;
     s = assemble(ctx, instances, count, views[0].camera.view, flags, A);
     if (s) return s;
@@ -398,7 +405,7 @@ cr_status cr::scratch_issue(cr_context* ctx, BatchScratch& S, const cr_instance*
         cap = want;
         return CR_OK;
     };
-    const CullLayout CL = cull_layout(A);
+    const CullLayout CL = cull_layout(A, nv);
     if ((s = grow(&S.dTable, S.dTableCap, L.total * 2, "slot table")) ||
         (s = grow(&S.records, S.recordCap, CL.total, "slot records")))
         return s;
@@ -422,7 +429,7 @@ cr_status cr::scratch_issue(cr_context* ctx, BatchScratch& S, const cr_instance*
     bind_tables(A, B, L, (char*)S.dTable, fp, rp);
     base_params(ctx, display, fp, rp);
     bind_cull(A, CL, S.records, fp);
-    use_lists(B, fp);
+    use_boxes(B, A.totalTriangles, fp);
     fp.counters = S.counters;
     fp.ntList = S.ntList;
     fp.ntCap = S.ntCap;
@@ -561,7 +568,7 @@ cr_status cr_batch_plan_create(cr_context* ctx, const cr_instance* instances, ui
     p->flags = flags;
     p->instances.assign(instances, instances + count);
     p->views.assign(views, views + num_views);
-    ensure_local_lists_for(ctx, instances, count);
+    ensure_sub_obbs_for(ctx, instances, count);
     s = assemble(ctx, instances, count, views[0].camera.view, flags, p->A);
     if (s) {
         delete p;
@@ -587,7 +594,7 @@ cr_status cr_batch_plan_create(cr_context* ctx, const cr_instance* instances, ui
         huNeed = ctx->last.huge_tiles + ctx->last.huge_tiles / 2 + 65536;
     }
     p->L = layout_of(p->A.inst.size(), p->A.seg.size(), num_views);
-    p->recordBytes = cull_layout(p->A).total;
+    p->recordBytes = cull_layout(p->A, num_views).total;
     if ((s = ctx->dev_alloc(&p->dTable, p->L.total, "plan table")) ||
         (s = ctx->dev_alloc(&p->records, p->recordBytes, "plan records"))) {
         plan_free(p);
@@ -622,8 +629,8 @@ cr_status cr_batch_plan_create(cr_context* ctx, const cr_instance* instances, ui
     CrResolveParams rp{};
     bind_tables(p->A, p->B, p->L, (char*)p->dTable, fp, rp);
     base_params(ctx, display, fp, rp);
-    bind_cull(p->A, cull_layout(p->A), p->records, fp);
-    use_lists(p->B, fp);
+    bind_cull(p->A, cull_layout(p->A, num_views), p->records, fp);
+    use_boxes(p->B, p->A.totalTriangles, fp);
     fp.counters = p->counters;
     fp.ntList = p->ntList;
     fp.ntCap = p->ntCap;

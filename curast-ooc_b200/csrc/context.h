@@ -55,16 +55,13 @@ struct MeshRec {
     bool compressed = false;
     CrCodec codec{};
     CrCodec* dCodec = nullptr;    // device copy, inside the box allocation
-    // per-item vertex lists, built on first use in a box-culled frame
-    uint8_t* localLists = nullptr;
-    uint32_t* localCounts = nullptr;
-    size_t localBytes = 0;
-    bool localTried = false;
-    // oriented sub-boxes of box-culled frames (CR_OBB_F4 per CR_SUB triangles),
+    // oriented sub-boxes of box-culled and batched frames (CR_OBB_F4 per CR_SUB triangles),
     // built on first use
     float4* subObbs = nullptr;
+    float4* subCones = nullptr;   // CR_CONE_FLOATS each, in the same allocation
     size_t subBytes = 0;
     bool subTried = false;
+    bool subDeclined = false;     // no room for them when a frame would have liked them
 };
 
 void mat4_mul(const float* a, const float* b, float* out);  // glm order
@@ -156,6 +153,7 @@ struct cr_context {
                                     // frame a drawn item used one of its vertices
     uint32_t needStamp = 0;         // the last frame's stamp (0 is never issued)
     uint64_t lastDirect = 0;        // triangles of the last frame if it took the direct path, else 0
+    uint64_t lastDirectSlices = 0;  // its vertices in slices of CR_VSLICE
     bool lastStamps = false;        // the last frame's vertex pass evaluated stamped slices only
     uint64_t lastNontrivial = 0;    // stage-2 queue entries of the last frame whose counters were read
     bool countersPublished = false; // the frame being issued has its resolve copy the counters
@@ -239,12 +237,11 @@ cr_status read_mesh_box(MeshRec& m);
 void free_mesh_arrays(cr_context* ctx, MeshRec& m);
 // Grows the per-vertex record buffer to at least `bytes`.
 cr_status ensure_records(cr_context* ctx, uint64_t bytes);
-// Builds a mesh's per-item vertex lists on first use (absent on failure).
-void ensure_local_lists(cr_context* ctx, MeshRec& m);
 // Builds a mesh's oriented sub-boxes on first use (absent on failure).
 void ensure_sub_obbs(cr_context* ctx, MeshRec& m);
-// Vertex lists for every mesh of an instance list (batched frames).
-void ensure_local_lists_for(cr_context* ctx, const cr_instance* instances, uint32_t count);
+bool sub_obbs_fit(cr_context* ctx, const cr_instance* instances, uint32_t count);
+// Sub-boxes for every mesh of an instance list (batched frames).
+void ensure_sub_obbs_for(cr_context* ctx, const cr_instance* instances, uint32_t count);
 
 // Issues one frame.  issue(tev, rasterEnd) enqueues the stages on `stream`
 // with the context's current queues, recording tev[0..6] around them when

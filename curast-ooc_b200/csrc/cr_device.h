@@ -17,18 +17,6 @@
 #define CR_BATCH 128            // triangles per stage-1 warp item (4 per lane)
 #define CR_INST_CHUNK 16        // instances per stage-1 warp item
 #define CR_SUB 16               // triangles per sub-box (CR_BATCH / CR_SUB per item)
-// Per-item vertex lists (CR_REC_BOXES frames): for each item, the sorted
-// distinct vertices its triangles reference (at most CR_LOCAL_MAX) and each
-// triangle's three positions in that list, in one CR_LOCAL_BYTES block:
-//   uint32_t vertex[CR_LOCAL_MAX]    bytes    0 .. 1023
-//   uint32_t corners[CR_BATCH]       bytes 1024 .. 1535, list positions of
-//                                    corners 0, 1, 2 in bytes 0, 1, 2
-// and, per item, the number of distinct vertices (CR_LOCAL_NONE: more than
-// CR_LOCAL_MAX, or a non-indexed mesh; the item is drawn without a list).
-#define CR_LOCAL_MAX 256
-#define CR_LOCAL_BYTES 1536
-#define CR_LOCAL_NONE 0xffffffffu
-
 // counters[] slots
 #define CR_CTR_NONTRIVIAL 0     // entries appended to the stage-2 queue
 #define CR_CTR_HUGE 1           // tiles appended to the stage-3 queue
@@ -130,8 +118,6 @@ struct alignas(16) CrSegment {
     const float* itemBoxes;     // per CR_BATCH triangles: box of their vertices (or nullptr)
     const float4* subObbs;      // per CR_SUB triangles, CR_OBB_F4: oriented box of their
                                 // vertices (box-culled frames; or nullptr)
-    const uint8_t* localLists;  // per item, CR_LOCAL_BYTES (or nullptr)
-    const uint32_t* localCounts;  // per item, distinct vertices or CR_LOCAL_NONE
     CrCodec codec;              // compressed meshes (flags bit 0 is then clear)
     const float* groupBoxes;    // per CR_GROUP item boxes: their union (or nullptr)
     uint64_t unitBase;          // first group-cull unit (item group x instance chunk)
@@ -139,6 +125,7 @@ struct alignas(16) CrSegment {
     const uint4* itemSlices;    // per item, two: the vertex-pass slices its vertices lie in
                                 // (CR_VSLICE; or nullptr)
     const float4* itemObbs;     // per item, CR_OBB_F4: oriented box of its vertices (or nullptr)
+    const float4* subCones;     // per CR_SUB triangles, CR_CONE_FLOATS (with subObbs)
     uint64_t pad;
 };
 static_assert(sizeof(CrSegment) == 160, "CrSegment layout");
@@ -285,8 +272,10 @@ struct CrFrameParams {
     // counted in counters[CR_CTR_SURVIVORS], at most s1Cap
     uint64_t* s1List;
     uint64_t s1Cap;
-    // CR_PROOF_F4 per instance for the item proofs, or nullptr (no proofs)
+    // CR_PROOF_F4 per instance for the item proofs, or nullptr (no proofs);
+    // batched frames: the first two of them per (view, instance), view-major
     const float4* instProof;
+    float4* viewProof;          // where k_view_proofs writes those
     // record-culled frames: per vertex-pass slice (CrInstance::vchunkBase *
     // CR_VCHUNK / CR_VSLICE + slice), needStamp when a drawn item uses one of
     // its vertices (k_stamp, from CrSegment::itemSlices, after the item cull);
@@ -383,6 +372,7 @@ struct CrLaunchShape {
     int stage2DenseBlocks;      // k_stage2_dense
     int s1RasterOwnBlocks;      // k_s1raster, each lane its own tiny raster
     int stage3BinBlocks;        // k_stage3_bins
+    int s1DirectBlocks;         // k_s1direct
 };
 
 int cr_query_launch_shape(int device, CrLaunchShape* out);
@@ -413,12 +403,10 @@ int cr_launch_mesh_boxes(const uint32_t* indices, const float* positions, const 
                          uint32_t numTriangles, uint32_t numVertices, float* itemBoxes, float* chunkBoxes,
                          float* meshBox, float* groupBoxes, float* chunkGroupBoxes, float* itemCones,
                          uint4* itemSlices, float4* itemObbs, void* stream);
-// The oriented box (CR_OBB_F4) of every CR_SUB consecutive triangles.
+// The oriented box (CR_OBB_F4) and normal cone (CR_CONE_FLOATS) of every CR_SUB
+// consecutive triangles.
 int cr_launch_sub_obbs(const uint32_t* indices, const float* positions, const CrCodec* codec, uint32_t numTriangles,
-                       float4* subObbs, void* stream);
-// Per-item vertex lists of an indexed mesh (see CR_LOCAL_BYTES).
-int cr_launch_local_lists(const uint32_t* indices, const CrCodec* codec, uint32_t numTriangles, uint8_t* lists,
-                          uint32_t* counts, void* stream);
+                       float4* subObbs, float* subCones, void* stream);
 
 // Batched (multi-view) frame: one launch per stage over all views.  Grid
 // sizes are chosen by the host (defaults from occupancy, or tuned).

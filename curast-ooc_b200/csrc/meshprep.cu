@@ -133,29 +133,34 @@ __global__ void __launch_bounds__(256) k_item_slices(const uint32_t* idx, const 
     }
 }
 
-// One warp per item: the normal cone of its triangles (CR_CONE_FLOATS, see
-// cr_device.h), computed in double from the float positions.  The axis is the
+// The normal cone of LANES * R consecutive triangles (CR_CONE_FLOATS, see
+// cr_device.h; 32 x 4: an item, 16 x 1: a sub-box), computed in double from the float positions.  The axis is the
 // sum of the unit normals, normalised and rounded to float; cosT is the least
 // cosine between a unit normal and that float axis, lowered by 1e-9 (far
 // above the double rounding of the computation) and rounded down to float;
 // nMin is rounded down, edge, sinT (from the stored cosT) and r (half the
 // diagonal of the box of the item's vertices) up.  A zero-area or non-finite
 // triangle, or a cone wider than acos(0.05), gives cosT = -2 (no proof).
-__global__ void __launch_bounds__(256) k_item_cones(const uint32_t* idx, const float* pos, const CrCodec* codec,
+template <int LANES, int R>
+__global__ void __launch_bounds__(256) k_cones(const uint32_t* idx, const float* pos, const CrCodec* codec,
                                                     uint32_t nT, float* cones) {
-    const int lane = threadIdx.x & 31;
+    constexpr uint32_t T = LANES * R;
+    const int lane = threadIdx.x & (LANES - 1);
     const GeomRef g = geom_from(pos, idx, codec);
-    const uint32_t nItems = (nT + CR_BATCH - 1) / CR_BATCH;
-    for (uint32_t b = blockIdx.x * 8 + (threadIdx.x >> 5); b < nItems; b += gridDim.x * 8) {
-        double n[CR_BATCH / 32][3];
-        double len[CR_BATCH / 32];
-        bool live[CR_BATCH / 32];
+    const uint32_t nItems = (nT + T - 1) / T;
+    const uint32_t perBlock = 256 / LANES;
+    // whole warps loop together: groups past the end hold no triangle
+    for (uint32_t b0 = blockIdx.x * perBlock; b0 < nItems; b0 += gridDim.x * perBlock) {
+        const uint32_t b = b0 + threadIdx.x / LANES;
+        double n[R][3];
+        double len[R];
+        bool live[R];
         double sx = 0.0, sy = 0.0, sz = 0.0, nMin = INFINITY, edge = 0.0;
         float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
         bool bad = false;
 #pragma unroll
-        for (int r = 0; r < CR_BATCH / 32; ++r) {
-            const uint32_t t = b * CR_BATCH + r * 32 + lane;
+        for (int r = 0; r < R; ++r) {
+            const uint64_t t = (uint64_t)b * T + r * LANES + lane;
             live[r] = t < nT;
             len[r] = 1.0;
             n[r][0] = n[r][1] = n[r][2] = 0.0;
@@ -185,7 +190,7 @@ __global__ void __launch_bounds__(256) k_item_cones(const uint32_t* idx, const f
             }
         }
 #pragma unroll
-        for (int d = 16; d >= 1; d >>= 1) {
+        for (int d = LANES / 2; d >= 1; d >>= 1) {
             sx += __shfl_xor_sync(FULL, sx, d);
             sy += __shfl_xor_sync(FULL, sy, d);
             sz += __shfl_xor_sync(FULL, sz, d);
@@ -197,7 +202,8 @@ __global__ void __launch_bounds__(256) k_item_cones(const uint32_t* idx, const f
                 hi[j] = fmaxf(hi[j], __shfl_xor_sync(FULL, hi[j], d));
             }
         }
-        bad = __any_sync(FULL, bad);
+        const unsigned badM = __ballot_sync(FULL, bad);
+        bad = ((badM >> (threadIdx.x & 31 & ~(LANES - 1))) & (LANES == 32 ? FULL : (1u << (LANES & 31)) - 1u)) != 0u;
         // the axis as stored (float, normalised in double first), renormalised
         // in double as the cone's cosine is measured
         const double sl = sqrt(sx * sx + sy * sy + sz * sz);
@@ -205,11 +211,11 @@ __global__ void __launch_bounds__(256) k_item_cones(const uint32_t* idx, const f
         const double ml = sqrt((double)mx * mx + (double)my * my + (double)mz * mz);
         double cosT = INFINITY;
 #pragma unroll
-        for (int r = 0; r < CR_BATCH / 32; ++r)
+        for (int r = 0; r < R; ++r)
             if (live[r] && len[r] > 0.0)
                 cosT = fmin(cosT, (n[r][0] * mx + n[r][1] * my + n[r][2] * mz) / (len[r] * ml));
 #pragma unroll
-        for (int d = 16; d >= 1; d >>= 1) cosT = fmin(cosT, __shfl_xor_sync(FULL, cosT, d));
+        for (int d = LANES / 2; d >= 1; d >>= 1) cosT = fmin(cosT, __shfl_xor_sync(FULL, cosT, d));
         cosT -= 1e-9;
         if (bad || !(sl > 0.0) || !isfinite(sl) || !(ml > 0.0) || !isfinite(ml) || !(cosT > 0.05)) cosT = -2.0;
         const float cosTf = __double2float_rd(cosT);
@@ -219,7 +225,7 @@ __global__ void __launch_bounds__(256) k_item_cones(const uint32_t* idx, const f
             const double h = 0.5 * ((double)hi[j] - (double)lo[j]);
             r2 += h * h;
         }
-        if (lane < CR_CONE_FLOATS) {
+        if (lane < CR_CONE_FLOATS && b < nItems) {
             float v;
             if (lane == 0) v = mx;
             else if (lane == 1) v = my;
@@ -240,12 +246,15 @@ __global__ void __launch_bounds__(256) k_item_cones(const uint32_t* idx, const f
 // strips of a surface, whose object-space boxes are loose: on the 1M-triangle
 // displaced sphere 26 % of the items of a random instance survive the
 // sample-miss proof with axis-aligned boxes, 17 % with these), or the object's
-// axes where that box has the smaller surface.  Extents are measured in
-// double along the double axes.
+// axes where that box has the smaller surface.  All in single precision.
 //
-// The stored floats contain the exact box: rounding the centre and the axes
-// moves a point of it by at most 2^-23 (|c| + h0 + h1 + h2) in any direction,
-// and each half extent is enlarged by 2^-20 of itself plus 2^-21 of that sum.
+// Containment.  The axes are orthonormal within 2^-21 and the extents measured
+// along them (differences from the middle of the object-space box, 2^-24 of the
+// coordinates each, and three products) are off by less than 2^-22 (M + H), M the
+// largest coordinate and H the sum of the half extents; solving p = c + sum t_j A_j
+// against nearly orthonormal axes and rounding c and A move a point by less than
+// 2^-20 H + 2^-23 M.  Each half extent is enlarged by 2^-19 of itself, 2^-18 H and
+// 2^-20 M.
 template <int LANES, int R>
 __global__ void __launch_bounds__(256) k_obbs(const uint32_t* idx, const float* pos, const CrCodec* codec, uint32_t nT,
                                               float4* obbs) {
@@ -259,9 +268,9 @@ __global__ void __launch_bounds__(256) k_obbs(const uint32_t* idx, const float* 
         for (int d = LANES / 2; d >= 1; d >>= 1) v += __shfl_xor_sync(FULL, v, d);
         return v;
     };
-    auto least = [](double v) {
+    auto least = [](float v) {
 #pragma unroll
-        for (int d = LANES / 2; d >= 1; d >>= 1) v = fmin(v, __shfl_xor_sync(FULL, v, d));
+        for (int d = LANES / 2; d >= 1; d >>= 1) v = fminf(v, __shfl_xor_sync(FULL, v, d));
         return v;
     };
     // whole warps loop together: groups past the end hold no triangle
@@ -271,7 +280,7 @@ __global__ void __launch_bounds__(256) k_obbs(const uint32_t* idx, const float* 
         bool live[R];
         bool bad = false;
         float nx = 0.0f, ny = 0.0f, nz = 0.0f;
-        double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+        float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const uint64_t t = (uint64_t)b * T + r * LANES + gl;
@@ -283,8 +292,8 @@ __global__ void __launch_bounds__(256) k_obbs(const uint32_t* idx, const float* 
 #pragma unroll
                 for (int j = 0; j < 3; ++j) {
                     bad |= !isfinite(q[r][k][j]);
-                    lo[j] = fmin(lo[j], (double)q[r][k][j]);
-                    hi[j] = fmax(hi[j], (double)q[r][k][j]);
+                    lo[j] = fminf(lo[j], q[r][k][j]);
+                    hi[j] = fmaxf(hi[j], q[r][k][j]);
                 }
             }
             const float u0 = q[r][1][0] - q[r][0][0], u1 = q[r][1][1] - q[r][0][1], u2 = q[r][1][2] - q[r][0][2];
@@ -302,29 +311,30 @@ __global__ void __launch_bounds__(256) k_obbs(const uint32_t* idx, const float* 
             hi[j] = -least(-hi[j]);
         }
         nx = sum(nx), ny = sum(ny), nz = sum(nz);
-        // any frame will do for the containment; a good one for tightness
-        double m[3] = {nx, ny, nz};
-        double ml = sqrt(m[0] * m[0] + m[1] * m[1] + m[2] * m[2]);
-        if (!(ml > 1e-6)) m[0] = m[1] = 0.0, m[2] = ml = 1.0;
-        m[0] /= ml, m[1] /= ml, m[2] /= ml;
-        // b1, b2: a basis of the plane across m
-        double b1[3];
-        if (fabs(m[0]) < 0.6) b1[0] = 0.0, b1[1] = m[2], b1[2] = -m[1];
-        else b1[0] = -m[2], b1[1] = 0.0, b1[2] = m[0];
-        const double bl = 1.0 / sqrt(b1[0] * b1[0] + b1[1] * b1[1] + b1[2] * b1[2]);
+        // an orthonormal frame m, b1, b2 (any will do for the containment, a good
+        // one for tightness)
+        float m[3] = {nx, ny, nz};
+        const float ml2 = m[0] * m[0] + m[1] * m[1] + m[2] * m[2];
+        if (!(ml2 > 1e-12f && ml2 < INFINITY)) m[0] = m[1] = 0.0f, m[2] = 1.0f;
+        const float im = 1.0f / sqrtf(m[0] * m[0] + m[1] * m[1] + m[2] * m[2]);
+        m[0] *= im, m[1] *= im, m[2] *= im;
+        float b1[3];
+        if (fabsf(m[0]) < 0.6f) b1[0] = 0.0f, b1[1] = m[2], b1[2] = -m[1];
+        else b1[0] = -m[2], b1[1] = 0.0f, b1[2] = m[0];
+        const float bl = 1.0f / sqrtf(b1[0] * b1[0] + b1[1] * b1[1] + b1[2] * b1[2]);
         b1[0] *= bl, b1[1] *= bl, b1[2] *= bl;
-        const double b2[3] = {m[1] * b1[2] - m[2] * b1[1], m[2] * b1[0] - m[0] * b1[2], m[0] * b1[1] - m[1] * b1[0]};
-        const double mid[3] = {0.5 * (lo[0] + hi[0]), 0.5 * (lo[1] + hi[1]), 0.5 * (lo[2] + hi[2])};
-        const float scale = (float)(1.0 / (fmax(hi[0] - lo[0], fmax(hi[1] - lo[1], hi[2] - lo[2])) + 1e-300));
+        const float b2[3] = {m[1] * b1[2] - m[2] * b1[1], m[2] * b1[0] - m[0] * b1[2], m[0] * b1[1] - m[1] * b1[0]};
+        const float mid[3] = {0.5f * (lo[0] + hi[0]), 0.5f * (lo[1] + hi[1]), 0.5f * (lo[2] + hi[2])};
+        const float scale = 1.0f / (fmaxf(hi[0] - lo[0], fmaxf(hi[1] - lo[1], hi[2] - lo[2])) + 1e-30f);
         float n = 0.0f, sx = 0.0f, sy = 0.0f, xx = 0.0f, xy = 0.0f, yy = 0.0f;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             if (!live[r]) continue;
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                const double d[3] = {q[r][k][0] - mid[0], q[r][k][1] - mid[1], q[r][k][2] - mid[2]};
-                const float x = (float)(d[0] * b1[0] + d[1] * b1[1] + d[2] * b1[2]) * scale;
-                const float y = (float)(d[0] * b2[0] + d[1] * b2[1] + d[2] * b2[2]) * scale;
+                const float d[3] = {q[r][k][0] - mid[0], q[r][k][1] - mid[1], q[r][k][2] - mid[2]};
+                const float x = (d[0] * b1[0] + d[1] * b1[1] + d[2] * b1[2]) * scale;
+                const float y = (d[0] * b2[0] + d[1] * b2[1] + d[2] * b2[2]) * scale;
                 n += 1.0f, sx += x, sy += y, xx += x * x, xy += x * y, yy += y * y;
             }
         }
@@ -332,64 +342,65 @@ __global__ void __launch_bounds__(256) k_obbs(const uint32_t* idx, const float* 
         const float in = 1.0f / fmaxf(n, 1.0f);
         float th = 0.5f * atan2f(2.0f * (xy - sx * sy * in), (xx - sx * sx * in) - (yy - sy * sy * in));
         if (!isfinite(th)) th = 0.0f;
-        double ct = cosf(th), sn = sinf(th);
-        const double cl = 1.0 / sqrt(ct * ct + sn * sn);
-        ct *= cl, sn *= cl;
-        double ax[3][3];
+        const float ct = cosf(th), sn = sinf(th);
+        float ax[3][3];
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
             ax[0][j] = ct * b1[j] + sn * b2[j];
             ax[1][j] = ct * b2[j] - sn * b1[j];
             ax[2][j] = m[j];
         }
-        double pl[3] = {INFINITY, INFINITY, INFINITY}, ph[3] = {-INFINITY, -INFINITY, -INFINITY};
+        float pl[3] = {INFINITY, INFINITY, INFINITY}, ph[3] = {-INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             if (!live[r]) continue;
 #pragma unroll
-            for (int k = 0; k < 3; ++k)
+            for (int k = 0; k < 3; ++k) {
+                const float d[3] = {q[r][k][0] - mid[0], q[r][k][1] - mid[1], q[r][k][2] - mid[2]};
 #pragma unroll
                 for (int j = 0; j < 3; ++j) {
-                    const double x = q[r][k][0] * ax[j][0] + q[r][k][1] * ax[j][1] + q[r][k][2] * ax[j][2];
-                    pl[j] = fmin(pl[j], x);
-                    ph[j] = fmax(ph[j], x);
+                    const float x = d[0] * ax[j][0] + d[1] * ax[j][1] + d[2] * ax[j][2];
+                    pl[j] = fminf(pl[j], x);
+                    ph[j] = fmaxf(ph[j], x);
                 }
+            }
         }
-        double h[3], a[3];
+        float h[3], a[3];
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
             pl[j] = least(pl[j]);
             ph[j] = -least(-ph[j]);
-            h[j] = 0.5 * (ph[j] - pl[j]);
-            a[j] = 0.5 * (hi[j] - lo[j]);
+            h[j] = 0.5f * (ph[j] - pl[j]);
+            a[j] = 0.5f * (hi[j] - lo[j]);
         }
-        double c[3];
+        float c[3];
         if (a[0] * a[1] + a[1] * a[2] + a[2] * a[0] <= h[0] * h[1] + h[1] * h[2] + h[2] * h[0]) {
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
                 c[j] = mid[j];
                 h[j] = a[j];
 #pragma unroll
-                for (int k = 0; k < 3; ++k) ax[j][k] = j == k ? 1.0 : 0.0;
+                for (int k = 0; k < 3; ++k) ax[j][k] = j == k ? 1.0f : 0.0f;
             }
         } else {
 #pragma unroll
             for (int k = 0; k < 3; ++k)
-                c[k] = 0.5 * ((pl[0] + ph[0]) * ax[0][k] + (pl[1] + ph[1]) * ax[1][k] + (pl[2] + ph[2]) * ax[2][k]);
+                c[k] = mid[k] +
+                       0.5f * ((pl[0] + ph[0]) * ax[0][k] + (pl[1] + ph[1]) * ax[1][k] + (pl[2] + ph[2]) * ax[2][k]);
         }
+        const float M = fmaxf(fmaxf(fmaxf(fabsf(lo[0]), fabsf(hi[0])), fmaxf(fabsf(lo[1]), fabsf(hi[1]))),
+                              fmaxf(fabsf(lo[2]), fabsf(hi[2])));
+        const float slack = 3.814697265625e-06f * (h[0] + h[1] + h[2]) + 9.5367431640625e-07f * M + 1e-37f;
         const unsigned badM = __ballot_sync(FULL, bad);
         const bool anyBad = ((badM >> (lane & ~(LANES - 1))) & (LANES == 32 ? FULL : (1u << (LANES & 31)) - 1u)) != 0u;
-        const double slack = 4.76837158203125e-07 *  // 2^-21
-                                 (fmax(fabs(c[0]), fmax(fabs(c[1]), fabs(c[2]))) + h[0] + h[1] + h[2]) +
-                             1e-37;
         if (gl == 0 && b < nGroups) {
             float o[12];
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
-                o[j] = anyBad ? __int_as_float(0x7fffffff) : (float)c[j];
-                const double hj = h[j] * 1.00000095367431640625 + slack;
+                o[j] = anyBad || !(M < 1e18f) ? __int_as_float(0x7fffffff) : c[j];  // huge: sums could overflow
+                const float hj = h[j] * 1.0000019073486328125f + slack;
 #pragma unroll
-                for (int k = 0; k < 3; ++k) o[3 + 3 * j + k] = (float)(ax[j][k] * hj);
+                for (int k = 0; k < 3; ++k) o[3 + 3 * j + k] = ax[j][k] * hj;
             }
 #pragma unroll
             for (int j = 0; j < CR_OBB_F4; ++j)
@@ -481,101 +492,16 @@ __global__ void __launch_bounds__(256) k_mesh_box(const float* itemBoxes, uint32
     }
 }
 
-// One warp per item: the item's 3 CR_BATCH indices are sorted in shared
-// memory (bitonic network over 512 slots, padded with ~0u), the distinct
-// values compacted into the list, and each index replaced by its position in
-// the list (binary search).  Items with more than CR_LOCAL_MAX distinct
-// vertices get CR_LOCAL_NONE.
-constexpr int LL_WARPS = 4;
-__global__ void __launch_bounds__(LL_WARPS * 32) k_local_lists(const uint32_t* idx, const CrCodec* codec, uint32_t nT,
-                                                                uint8_t* lists, uint32_t* counts) {
-    const GeomRef g = geom_from(nullptr, idx, codec);
-    __shared__ uint32_t s_key[LL_WARPS][512];
-    __shared__ uint32_t s_uni[LL_WARPS][512];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    uint32_t* key = s_key[w];
-    uint32_t* uni = s_uni[w];
-    const uint32_t nItems = (nT + CR_BATCH - 1) / CR_BATCH;
-    for (uint32_t b = blockIdx.x * LL_WARPS + w; b < nItems; b += gridDim.x * LL_WARPS) {
-        const uint32_t t0 = b * CR_BATCH;
-        const uint32_t nt = min((uint32_t)CR_BATCH, nT - t0);
-        for (int i = lane; i < 512; i += 32) key[i] = i < 3 * (int)nt ? geom_index(g, 3ull * t0 + i) : ~0u;
-        __syncwarp();
-        for (int k = 2; k <= 512; k <<= 1)
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                for (int i = lane; i < 512; i += 32) {
-                    const int l = i ^ j;
-                    if (l > i) {
-                        const uint32_t a = key[i], c = key[l];
-                        const bool up = (i & k) == 0;
-                        if ((a > c) == up) {
-                            key[i] = c;
-                            key[l] = a;
-                        }
-                    }
-                }
-                __syncwarp();
-            }
-        // distinct values: lane owns slots 16 lane .. 16 lane + 15
-        uint32_t flags = 0;
-        for (int q = 0; q < 16; ++q) {
-            const int i = 16 * lane + q;
-            const uint32_t v = key[i];
-            if (v != ~0u && (i == 0 || key[i - 1] != v)) flags |= 1u << q;
-        }
-        const int mine = __popc(flags);
-        int incl = mine;
-        for (int d = 1; d < 32; d <<= 1) {
-            const int o = __shfl_up_sync(FULL, incl, d);
-            if (lane >= d) incl += o;
-        }
-        const int total = __shfl_sync(FULL, incl, 31);
-        int pos = incl - mine;
-        for (int q = 0; q < 16; ++q)
-            if ((flags >> q) & 1u) uni[pos++] = key[16 * lane + q];
-        __syncwarp();
-        if (lane == 0) counts[b] = total <= CR_LOCAL_MAX ? (uint32_t)total : CR_LOCAL_NONE;
-        if (total > CR_LOCAL_MAX) continue;  // warp-uniform
-        uint8_t* L = lists + (uint64_t)b * CR_LOCAL_BYTES;
-        uint32_t* vl = reinterpret_cast<uint32_t*>(L);
-        for (int i = lane; i < CR_LOCAL_MAX; i += 32) vl[i] = i < total ? uni[i] : 0u;
-        uint32_t* corners = reinterpret_cast<uint32_t*>(L + 1024);
-        for (int t = lane; t < CR_BATCH; t += 32) {
-            uint32_t word = 0;
-            for (int c = 0; c < 3 && t < (int)nt; ++c) {
-                const uint32_t v = geom_index(g, 3ull * (t0 + t) + c);
-                int lo = 0, hi = total - 1;  // uni[lo] == v
-                while (lo < hi) {
-                    const int mid = (lo + hi) >> 1;
-                    if (uni[mid] < v) lo = mid + 1;
-                    else hi = mid;
-                }
-                word |= (uint32_t)lo << (8 * c);
-            }
-            corners[t] = word;
-        }
-        __syncwarp();
-    }
-}
-
 }  // namespace
 
-int cr_launch_local_lists(const uint32_t* indices, const CrCodec* codec, uint32_t numTriangles, uint8_t* lists,
-                          uint32_t* counts, void* stream) {
-    const uint32_t nItems = (numTriangles + CR_BATCH - 1) / CR_BATCH;
-    if (!nItems) return 0;
-    const uint32_t want = (nItems + LL_WARPS - 1) / LL_WARPS;
-    k_local_lists<<<want < 148 * 16 ? want : 148 * 16, LL_WARPS * 32, 0, (cudaStream_t)stream>>>(
-        indices, codec, numTriangles, lists, counts);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
-}
-
 int cr_launch_sub_obbs(const uint32_t* indices, const float* positions, const CrCodec* codec, uint32_t numTriangles,
-                       float4* subObbs, void* stream) {
+                       float4* subObbs, float* subCones, void* stream) {
     const uint32_t blocks = ((numTriangles + CR_SUB - 1) / CR_SUB + 15) / 16;
     if (!blocks) return 0;
     k_obbs<CR_SUB, 1><<<blocks < 148 * 16 ? blocks : 148 * 16, 256, 0, (cudaStream_t)stream>>>(
         indices, positions, codec, numTriangles, subObbs);
+    k_cones<CR_SUB, 1><<<blocks < 148 * 16 ? blocks : 148 * 16, 256, 0, (cudaStream_t)stream>>>(
+        indices, positions, codec, numTriangles, subCones);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -602,7 +528,7 @@ int cr_launch_mesh_boxes(const uint32_t* indices, const float* positions, const 
         k_group_boxes<<<(nCGroups + 7) / 8 < 148 * 16 ? (nCGroups + 7) / 8 : 148 * 16, 256, 0, st>>>(
             chunkBoxes, nChunks, chunkGroupBoxes);
     if (nItems && itemCones)
-        k_item_cones<<<(nItems + 7) / 8 < 148 * 16 ? (nItems + 7) / 8 : 148 * 16, 256, 0, st>>>(
+        k_cones<32, 4><<<(nItems + 7) / 8 < 148 * 16 ? (nItems + 7) / 8 : 148 * 16, 256, 0, st>>>(
             indices, positions, codec, numTriangles, itemCones);
     const uint32_t nSlices = (numVertices + CR_VSLICE - 1) / CR_VSLICE;
     if (nItems && nSlices && itemSlices)

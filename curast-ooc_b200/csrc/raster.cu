@@ -18,9 +18,11 @@
 //            per-warp shared-memory ring signalled by an mbarrier; triangles
 //            whose three records prove them culled stop there) and
 //            k_s1raster (the reference's full path on the survivors, one per
-//            lane).  Box-culled frames: k_stage1 (per-item vertex lists and
-//            shared-memory records per instance).  Nontrivial triangles are
-//            appended with one atomic per warp.     reference: tv.cu:274-384
+//            lane).  Box-culled frames: k_stage1 (oriented boxes of 16
+//            triangles, then a test of single ones) and k_s1raster.  Small
+//            frames: k_s1direct or k_s1raster alone, every triangle.  Nontrivial
+//            triangles are appended with one atomic per warp.
+//                                                   reference: tv.cu:274-384
 //   stage 2  persistent warps; every lane sets up one queued triangle at once
 //            (the reference: lane 0 sets up while 31 lanes wait), then per
 //            triangle rows are narrowed to the columns that can pass and
@@ -117,7 +119,7 @@ __global__ void __launch_bounds__(THREADS, VX_MIN_BLOCKS) k_vertex(const CrFrame
                 if (v >= v1) continue;
                 if (p.cellMode == CR_REC_CELLS32)
                     reinterpret_cast<uint32_t*>(p.outcodes)[outBase + v] =
-                        vertex_cell32<true>(M, q[r], fa, p.f, Wf, Hf, Wm1, Hm1);
+                        vertex_cell32(M, q[r], fa, p.f, Wf, Hf, Wm1, Hm1);
                 else if (p.cellMode == CR_REC_CELLS)
                     reinterpret_cast<uint64_t*>(p.outcodes)[outBase + v] =
                         vertex_cell_record(M, q[r], fa, p.f, Wf, Hf, p.W, p.H);
@@ -339,35 +341,36 @@ __global__ void __launch_bounds__(THREADS, 3) k_cull(const CrFrameParams p) {
         uint32_t mask = 0;
         if (valid) {
             const float* boxes = ldg_ptr(&sg->itemBoxes);
-            const float4* cones = p.instProof ? reinterpret_cast<const float4*>(ldg_ptr(&sg->itemCones)) : nullptr;
             const float4* obbs = p.instProof ? ldg_ptr(&sg->itemObbs) : nullptr;
             if (!boxes) {
                 mask = alive | (insideU << 16);
             } else {
-                float blo[3], bhi[3];
-                load_box(boxes + 6ull * batch, blo, bhi);
-                const V3 mid = {0.5f * (blo[0] + bhi[0]), 0.5f * (blo[1] + bhi[1]), 0.5f * (blo[2] + bhi[2])};
-                float4 c0 = make_float4(0.0f, 0.0f, 0.0f, -2.0f), c1 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                if (cones) {
-                    c0 = __ldg(cones + 2ull * batch);
-                    c1 = __ldg(cones + 2ull * batch + 1);
-                }
+                float4 c0, c1;
                 Obb ob;
-                if (obbs) ob = load_obb(obbs + (uint64_t)CR_OBB_F4 * batch);
+                float radius = 0.0f;
+                if (obbs) {
+                    const float4* cone = reinterpret_cast<const float4*>(ldg_ptr(&sg->itemCones)) + 2ull * batch;
+                    c0 = __ldg(cone);
+                    c1 = __ldg(cone + 1);
+                    ob = load_obb(obbs + (uint64_t)CR_OBB_F4 * batch);
+                    radius = obb_radius(ob);
+                }
                 for (uint32_t rest = alive; rest; rest &= rest - 1) {
                     const uint32_t slot = __ffs(rest) - 1;
                     const uint32_t inst = ib + slot;
                     bool inside = ((insideU >> slot) & 1u) != 0u;
-                    if (p.instProof) {
+                    if (obbs) {
                         const Proof P = load_proof(p, inst);
                         // every triangle of the item faces away from the camera
-                        if (item_back_facing(P, c0, c1, mid)) continue;
+                        if (item_back_facing(P, c0, c1, ob.c, radius)) continue;
                         // the sample-miss proof of the whole item (for every
                         // record mode: it culls items of sub-pixel triangles
                         // before their indices are read)
-                        if (obbs && obb_misses_samples(P, fa, p.f, Wf, Hf, ob)) continue;
+                        if (obb_misses_samples(P, fa, p.f, Wf, Hf, ob)) continue;
                     }
                     if (!inside) {
+                        float blo[3], bhi[3];
+                        load_box(boxes + 6ull * batch, blo, bhi);
                         const uint32_t c = classify_box(load_mat(p.world_view + 4ull * inst), fa, p.f, blo, bhi);
                         if (c & CR_OC_MASK) continue;
                         inside = (c & CH_INSIDE) != 0u;
@@ -718,11 +721,19 @@ __global__ void __launch_bounds__(WARPS * 32, S1C_MIN_BLOCKS) k_s1cull(const CrF
         if (pending & (1u << s)) (void)mbar_wait_bounded(&s_bar[w][s], (parity >> s) & 1u, p.waitTimeoutNs);
 }
 
-// a warp's tiny rasters whose largest has more fragments than this are
-// rasterized across the warp (stage1_coop_raster)
-#ifndef CR_COOP_MIN_FRAGMENTS
-#define CR_COOP_MIN_FRAGMENTS 8
-#endif
+// The instance of triangle j of a direct frame's prefix sum over its instances
+// (CrInstance::cum), j at most a warp past `base`: the search is the warp's, from
+// there a lane steps on.
+__device__ __forceinline__ uint32_t instance_of_triangle(const CrFrameParams& p, uint64_t base, uint64_t j) {
+    uint32_t lo = 0, hi = p.numInstances - 1;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (__ldg(&p.instances[mid].cum) <= base) lo = mid;
+        else hi = mid - 1;
+    }
+    while (lo + 1 < p.numInstances && __ldg(&p.instances[lo + 1].cum) <= j) ++lo;
+    return lo;
+}
 
 // k_s1raster: persistent warps over the survivor list, one triangle per lane:
 // its indices and positions, then the reference's full per-triangle path
@@ -740,20 +751,20 @@ __global__ void __launch_bounds__(WARPS * 32) k_s1raster(const CrFrameParams p) 
     const uint64_t n = DIRECT ? p.direct : min((uint64_t)p.counters[CR_CTR_SURVIVORS], p.s1Cap);
     const Target tg = target_of(p);
     const float fa = tg.fa;
-    for (uint64_t base = gw * 32; base < n; base += nw * 32) {
+    // triangles per warp: 32, fewer where that leaves warps idle and the warp's
+    // raster (COOP) can use the other lanes -- a 4,096-triangle frame in 128 warps
+    // of 32 took them through ten rounds of rows each, 18 us; fewer per warp 10 (stage 1 of that frame
+    // 20.8 -> 12.6 by events)
+    const uint64_t per = COOP ? min((uint64_t)32, max((uint64_t)1, (n + nw - 1) / nw)) : 32;
+    for (uint64_t base = gw * per; base < n; base += nw * per) {
         const uint64_t j = base + lane;
         int res = S1_CULL;
         uint32_t tri = 0, inst = 0;
         S1Raster ras;
         uint64_t rid = 0;
-        if (j < n) {
-            if constexpr (DIRECT) {  // triangle j of the frame's prefix sum over its instances
-                uint32_t hi = p.numInstances - 1;
-                while (inst < hi) {
-                    const uint32_t mid = (inst + hi + 1) >> 1;
-                    if (__ldg(&p.instances[mid].cum) <= j) inst = mid;
-                    else hi = mid - 1;
-                }
+        if (lane < per && j < n) {
+            if constexpr (DIRECT) {
+                inst = instance_of_triangle(p, base, j);
                 tri = (uint32_t)(j - __ldg(&p.instances[inst].cum));
             } else {
                 const uint64_t e = __ldg(p.s1List + j);
@@ -769,183 +780,237 @@ __global__ void __launch_bounds__(WARPS * 32) k_s1raster(const CrFrameParams p) 
             const V3 pb = pos_of(g, i1);
             const V3 pc = pos_of(g, i2);
             rid = __ldg(&I->cum) + tri;
-            res = stage1_triangle<COOP>(tg, fa, load_mat(p.world_view + 4ull * inst), __ldg(&I->flip), pa, pb, pc,
+            res = stage1_triangle<COOP, !DIRECT>(tg, fa, load_mat(p.world_view + 4ull * inst), __ldg(&I->flip), pa, pb, pc,
                                         rid, &ras);
         }
-        if constexpr (COOP) {
-            // the lanes' tiny rasters: spread over the warp when one of them
-            // would hold the others up, else each lane its own
-            const bool mine = res == S1_RASTER;
-            const int frags = mine ? max(ras.size_x, 0) * max(ras.size_y, 0) : 0;
-            if (__reduce_max_sync(FULL, (unsigned)frags) > CR_COOP_MIN_FRAGMENTS)
-                stage1_coop_raster(tg, mine, ras, rid);
-            else if (mine)
-                stage1_own_raster(tg, ras, rid);
-        }
+        if constexpr (COOP) s1_raster_lanes(tg, res, ras, rid);
         append_nontrivial(p, res == S1_QUEUE, inst, tri);
     }
 }
 
+// k_s1direct: direct frames whose triangles are mostly sub-pixel.  Every
+// triangle of every instance, one per lane, through quick_misses; the few it
+// leaves queue in a per-warp ring for the full path, 32 at a time.  A warp takes
+// consecutive triangles, so that its instance (and what the test needs of it)
+// changes rarely.  (300 x 5,121 triangles at 1280x720: every triangle through the
+// full path 35 us, so 26.  A 2M-triangle heightfield of needles at 391x220: each lane
+// its own raster 205 us, the rasters shared over the warp 136; by way of the survivor
+// list and k_s1raster 159.)
+template <int WARPS, bool PACKED>
+__global__ void __launch_bounds__(WARPS * 32, 4) k_s1direct(const CrFrameParams p) {
+    pdl_enter();
+    __shared__ uint64_t s_ring[WARPS][S1_RING];
+    const int lane = threadIdx.x & 31;
+    const uint64_t gw = (uint64_t)blockIdx.x * WARPS + (threadIdx.x >> 5);
+    const uint64_t nw = (uint64_t)gridDim.x * WARPS;
+    const Target tg = target_of(p);
+    const float Wf = (float)p.W, Hf = (float)p.H;
+    uint64_t* const ring = s_ring[threadIdx.x >> 5];
+    uint32_t qh = 0, qt = 0;  // ring head / tail (warp-uniform)
+    const uint64_t share = (p.direct + 32 * nw - 1) / (32 * nw) * 32;
+    const uint64_t end = min(p.direct, (gw + 1) * share);
+    uint32_t inst = gw * share < p.direct ? instance_of_triangle(p, gw * share, gw * share) : 0u;
+    uint32_t of = 0xffffffffu;  // the instance that q, g and cum are of
+    Quick q;
+    GeomRef g;
+    uint64_t cum = 0;
+    for (uint64_t base = gw * share; qh < qt || base < end; base += 32) {
+        if (base < end) {
+            const uint64_t j = base + lane;
+            bool keep = j < end;
+            uint32_t tri = 0;
+            if (keep) {
+                while (inst + 1 < p.numInstances && __ldg(&p.instances[inst + 1].cum) <= j) ++inst;
+                if (inst != of) {
+                    of = inst;
+                    q = make_quick(load_proof(p, inst), tg.fa, p.f, Wf, Hf);
+                    g = geom_of_t<PACKED>(p.instances + inst);
+                    cum = __ldg(&p.instances[inst].cum);
+                }
+                tri = (uint32_t)(j - cum);
+                const V3 pa = pos_of(g, geom_index(g, 3ull * tri + 0));
+                const V3 pb = pos_of(g, geom_index(g, 3ull * tri + 1));
+                const V3 pc = pos_of(g, geom_index(g, 3ull * tri + 2));
+                keep = !quick_misses(q, pa, pb, pc);
+            }
+            const unsigned m = __ballot_sync(FULL, keep);
+            if (keep) ring[(qt + __popc(m & ((1u << lane) - 1u))) & (S1_RING - 1)] = ((uint64_t)inst << 32) | tri;
+            qt += __popc(m);
+            __syncwarp();
+        }
+        if (qt - qh < 32u && base + 32 < end) continue;
+        const uint32_t k = qh + lane;
+        int res = S1_CULL;
+        uint32_t tri = 0, in = 0;
+        S1Raster ras;
+        uint64_t rid = 0;
+        if (k < qt) {
+            const uint64_t e = ring[k & (S1_RING - 1)];
+            in = (uint32_t)(e >> 32);
+            tri = (uint32_t)e;
+            const CrInstance* I = p.instances + in;
+            const GeomRef gk = geom_of_t<PACKED>(I);
+            const V3 pa = pos_of(gk, geom_index(gk, 3ull * tri + 0));
+            const V3 pb = pos_of(gk, geom_index(gk, 3ull * tri + 1));
+            const V3 pc = pos_of(gk, geom_index(gk, 3ull * tri + 2));
+            rid = __ldg(&I->cum) + tri;
+            res = stage1_triangle<true, true>(tg, tg.fa, load_mat(p.world_view + 4ull * in), __ldg(&I->flip), pa, pb, pc,
+                                              rid, &ras);
+        }
+        qh = min(qh + 32u, qt);
+        s1_raster_lanes(tg, res, ras, rid);
+        append_nontrivial(p, res == S1_QUEUE, in, tri);
+        __syncwarp();
+    }
+}
+
+// Up to 32 triangles of a warp's ring, from qh to qt, to the survivor list.  What a full
+// list cannot take runs here.
+template <bool PACKED>
+__device__ __forceinline__ void append_survivors(const CrFrameParams& p, const Target& tg, const uint64_t* ring,
+                                                 uint32_t& qh, const uint32_t qt) {
+    const uint32_t lane = threadIdx.x & 31, n = min(32u, qt - qh);
+    unsigned long long b = 0;
+    if (lane == 0) b = atomicAdd(&p.counters[CR_CTR_SURVIVORS], (unsigned long long)n);
+    b = __shfl_sync(FULL, b, 0);
+    const uint64_t e = ring[(qh + lane) & (S1_RING - 1)];
+    qh += n;
+    if (lane < n && b + lane < p.s1Cap) p.s1List[b + lane] = e;
+    if (b + n > p.s1Cap) {
+        const uint32_t inst = (uint32_t)(e >> 32), tri = (uint32_t)e;
+        int res = S1_CULL;
+        if (lane < n && b + lane >= p.s1Cap) {
+            const CrInstance* I = p.instances + inst;
+            const GeomRef g = geom_of_t<PACKED>(I);
+            const V3 pa = pos_of(g, geom_index(g, 3ull * tri + 0));
+            const V3 pb = pos_of(g, geom_index(g, 3ull * tri + 1));
+            const V3 pc = pos_of(g, geom_index(g, 3ull * tri + 2));
+            res = stage1_triangle<false, true>(tg, tg.fa, load_mat(p.world_view + 4ull * inst), __ldg(&I->flip), pa, pb, pc,
+                                               __ldg(&I->cum) + tri);
+        }
+        append_nontrivial(p, res == S1_QUEUE, inst, tri);
+    }
+    __syncwarp();
+}
+
 // Box-culled frames (some mesh drawn more than once: no per-vertex records).
-// Persistent warps over the work items; per item a warp waits for the item's
-// index tile in the TMA ring while it proves, for every live instance and
-// every CR_SUB triangles of the item (a lane per pair), that their oriented box
-// misses every sample; the triangles of the other pairs run through the
-// reference's full path (stage1_triangle), two pairs at a time.  Nontrivial
-// triangles are appended with one atomic per warp (ballot / popc).
+// Persistent warps over the frame cull's items, 32 list entries at a time (fewer
+// where that leaves warps idle): the (item, instance) pairs of all of them are
+// taken four at a time, a lane per pair and CR_SUB triangles, which are dropped
+// when their oriented box misses every sample or they provably all face away.
+// Two of the sub-boxes left at a time go one triangle per lane through
+// quick_misses, and the triangles left then are collected per warp and appended 32
+// at a time to the survivor list, which k_s1raster takes through the reference's
+// full path.  (A list that is full is no error here: the warp then runs the path
+// itself.)
 //
-// Issue-bound.  Small instances of dense meshes are the frames that come here,
-// and almost every triangle in them misses every sample: of the 128 triangles of
-// a listed (item, instance) pair of 3000 x 1M-triangle spheres about 40 are left
-// by the sub-box proofs (3 of 8 boxes, 22 issue slots a pair), where cell records of
-// the item's 160 distinct vertices cost about 900 slots a pair.  Stage 1 of that
-// frame (with the oriented item boxes) went from 8.66 to 4.68 ms.
-#ifndef CR_S1_BOXES_MIN_BLOCKS
-#define CR_S1_BOXES_MIN_BLOCKS 3
-#endif
+// Issue-bound.  Sub-pixel triangles are the frames that come here, and almost
+// every one of them misses every sample: of the 7,813 items of an instance of 3000 x
+// 1M-triangle spheres 1,350 are listed, 3,900 of their 10,800 sub-boxes kept, and of
+// the 62,000 triangles in those 290 have to go through the full path.  Stage 1 of
+// that frame: cell records of each pair's distinct vertices 8.66 ms; with the
+// oriented boxes and the full path for every triangle left 4.68; quick_misses 3.65;
+// the pairs of 32 entries together instead of an index tile and three partly filled
+// steps per item 3.07, with the error bounds drawn tighter 2.78; the full path in a
+// kernel of its own 2.80, 2.69 with the fourth block per SM that this allows (and a
+// frame whose survivors crowd in a few items, the 400M planet from its surface, 315 ->
+// 130 us).
 // PACKED: compiled for frames with compressed meshes (plain frames carry no
 // decoding code).
 template <int WARPS, bool PACKED>
-__global__ void __launch_bounds__(WARPS * 32, CR_S1_BOXES_MIN_BLOCKS) k_stage1(const CrFrameParams p) {
+__global__ void __launch_bounds__(WARPS * 32, 4) k_stage1(const CrFrameParams p) {
     pdl_enter();
-    constexpr int STAGES = 2;
-    __shared__ __align__(128) uint32_t s_idx[WARPS][STAGES][CR_BATCH * 3];
-    __shared__ __align__(8) uint64_t s_bar[WARPS][STAGES];
+    __shared__ uint64_t s_ring[WARPS][S1_RING];
     const int lane = threadIdx.x & 31;
-    const int w = threadIdx.x >> 5;
-    const uint64_t gw = (uint64_t)blockIdx.x * WARPS + w;
+    const uint64_t gw = (uint64_t)blockIdx.x * WARPS + (threadIdx.x >> 5);
     const uint64_t nw = (uint64_t)gridDim.x * WARPS;
-
-    if (lane == 0) {
-        for (int s = 0; s < STAGES; ++s) mbar_init(&s_bar[w][s], 1);
-        fence_barrier_init();
-    }
-    __syncwarp();
-    // `pending` marks ring slots holding an issued, not yet consumed tile copy.
-    // Every lane tracks it identically; lane 0 issues the copies.
-    // work items: the item cull's survivors (with their instance masks) or,
-    // without an item list, every item
     const uint64_t nItems = p.itemList ? min((uint64_t)p.counters[CR_CTR_ITEMS], p.itemCap) : p.numItems;
-    auto item_at = [&](uint64_t k) -> uint64_t { return p.itemList ? (uint64_t)__ldg(&p.itemList[k].x) : k; };
-    uint32_t pending = 0;
-    for (int s = 0; s < STAGES; ++s) {
-        const uint64_t pk = gw + (uint64_t)s * nw;
-        if (pk >= nItems) break;
-        const Item it = decode_item(p, item_at(pk));
-        const TileSrc ts = tile_source(p.segments + it.seg, it.batch);
-        if (ts.src) {
-            pending |= 1u << s;
-            const bool drop = (p.debugFlags & 1u) && gw == 0 && s == 0;
-            if (lane == 0 && !drop) bulk_load(s_idx[w][s], ts.src, ts.bytes, &s_bar[w][s]);
-        }
-    }
-    __syncwarp();
-
     const Target tg = target_of(p);
     const float Wf = (float)p.W, Hf = (float)p.H;
-    uint32_t parity = 0;
-    uint32_t k = 0;
-    for (uint64_t pk = gw; pk < nItems; pk += nw, ++k) {
-        const int slot = (int)(k % STAGES);
-        const uint32_t bit = 1u << slot;
-        const uint64_t item = item_at(pk);
-        const uint32_t imask = p.itemList ? __ldg(&p.itemList[pk].y) : 0xffffffffu;
-        const Item it = decode_item(p, item);
-        const CrSegment* sg = p.segments + it.seg;
-        const uint32_t numTri = __ldg(&sg->numTriangles);
-        const GeomRef geo = geom_of_t<PACKED>(sg);
-        const bool tma = tile_source(sg, it.batch).src != nullptr;
-        const uint32_t tri0 = it.batch * CR_BATCH;
-        const uint32_t first = __ldg(&sg->firstInstance);
-        const uint32_t ib = first + it.chunk * CR_INST_CHUNK;
-        const uint32_t ie = min(ib + CR_INST_CHUNK, first + __ldg(&sg->instanceCount));
-        const uint32_t alive = imask & ((1u << (ie - ib)) - 1u);
-        // lane k: the slot of the k-th surviving instance
-        const uint32_t slotOf = lane < __popc(alive) ? __fns(alive, 0, lane + 1) : 0u;
-        // bit 8 (k % 4) + b of subw[k / 4] is set unless sub-box b of the k-th
-        // surviving instance is proven to miss every sample (or is empty)
-        uint32_t subw[4];
-        {
-            const float4* obbs = p.instProof ? ldg_ptr(&sg->subObbs) : nullptr;
-            const int nsub = (int)min((uint32_t)(CR_BATCH / CR_SUB), (numTri - tri0 + CR_SUB - 1) / CR_SUB);
-            const int pairs = __popc(alive) * (CR_BATCH / CR_SUB);
-            Obb ob;
-            if (obbs && (lane & 7) < nsub)
-                ob = load_obb(obbs + CR_OBB_F4 * ((uint64_t)it.batch * (CR_BATCH / CR_SUB) + (lane & 7)));
+    // triangles no proof culls, (instance << 32) | triangle
+    uint64_t* const ring = s_ring[threadIdx.x >> 5];
+    uint32_t qh = 0, qt = 0;  // ring head / tail (warp-uniform)
+    // at least four turns per warp, so that crowded items even out
+    const uint64_t per = min((uint64_t)32, max((uint64_t)1, nItems / (4 * nw)));
+    for (uint64_t base = gw * per; base < nItems; base += nw * per) {
+        // this lane's list entry: segment, item of the mesh, first instance
+        // of its chunk and the live ones
+        uint32_t seg = 0, batch = 0, ib = 0, live = 0;
+        if (lane < per && base + lane < nItems) {
+            const uint2 e = p.itemList ? __ldg(&p.itemList[base + lane]) : make_uint2((uint32_t)(base + lane), 0xffffu);
+            const Item it = decode_item(p, e.x);
+            const CrSegment* sg = p.segments + it.seg;
+            seg = it.seg;
+            batch = it.batch;
+            const uint32_t off = it.chunk * CR_INST_CHUNK;
+            ib = __ldg(&sg->firstInstance) + off;
+            live = e.y & ((1u << min((uint32_t)CR_INST_CHUNK, __ldg(&sg->instanceCount) - off)) - 1u);
+        }
+        int incl = __popc(live);
 #pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                subw[t] = 0;
-                if (t * 32 >= pairs) continue;
-                const int j = t * 32 + lane;
-                const uint32_t inst = ib + __shfl_sync(FULL, slotOf, (j >> 3) & 31);
-                bool keep = j < pairs && (j & 7) < nsub;
-                if (keep && obbs) keep = !obb_misses_samples(load_proof(p, inst), tg.fa, p.f, Wf, Hf, ob);
-                subw[t] = __ballot_sync(FULL, keep);
-            }
+        for (int d = 1; d < 32; d <<= 1) {
+            const int v = __shfl_up_sync(FULL, incl, d);
+            if (lane >= d) incl += v;
         }
-        static_assert(CR_BATCH / CR_SUB == 8 && CR_INST_CHUNK <= 16, "8 sub-boxes x 16 instances in 4 ballots");
-        if (tma) {
-            const bool ok =
-                __all_sync(FULL, mbar_wait_bounded(&s_bar[w][slot], (parity & bit) ? 1u : 0u, p.waitTimeoutNs));
-            if (!ok) {  // record, stop this warp, drain its copies below
-                if (lane == 0) atomicOr(&p.counters[CR_CTR_TIMEOUT], 1ull);
-                break;
+        const int total = __shfl_sync(FULL, incl, 31);
+        for (int q0 = 0; q0 < total; q0 += 4) {
+            // pair q0 + (lane >> 3): its entry (first with incl > pair) and instance
+            const int pr = q0 + (lane >> 3);
+            int o = 0;
+#pragma unroll
+            for (int step = 16; step >= 1; step >>= 1) {
+                const int c = __shfl_sync(FULL, incl, o + step - 1);
+                if (c <= pr) o += step;
             }
-            parity ^= bit;
-            pending &= ~bit;
-        }
-        const uint32_t* tile = s_idx[w][slot];
-        // vertex index of corner c of the triangle at tile position pos
-        auto index_of = [&](uint32_t pos, int c) -> uint32_t {
-            if (tma) return tile[3 * pos + c];
-            return geom_index(geo, 3ull * (tri0 + pos) + c);
-        };
-        // the sub-boxes that are left, two at a time across the item's
-        // instances: half a warp each, a triangle per lane
-#pragma unroll 1
-        for (int t = 0; t < 4; ++t) {
-            uint32_t rest = t == 0 ? subw[0] : t == 1 ? subw[1] : t == 2 ? subw[2] : subw[3];
+            o &= 31;  // a pair past the last one has no entry
+            uint32_t m = __shfl_sync(FULL, live, o);
+            int rank = pr - (__shfl_sync(FULL, incl, o) - __popc(m));
+            const CrSegment* sg = p.segments + __shfl_sync(FULL, seg, o);
+            const uint32_t sub = __shfl_sync(FULL, batch, o) * (CR_BATCH / CR_SUB) + (uint32_t)(lane & 7);
+            uint32_t inst = __shfl_sync(FULL, ib, o);
+            bool keep = pr < total;
+            if (keep) {
+                while (rank-- > 0) m &= m - 1;
+                inst += (uint32_t)__ffs(m) - 1;
+                keep = sub * CR_SUB < __ldg(&sg->numTriangles);
+            }
+            if (keep && p.instProof) {
+                const float4* obbs = ldg_ptr(&sg->subObbs);
+                if (obbs) {
+                    const Proof P = load_proof(p, inst);
+                    const Obb ob = load_obb(obbs + (uint64_t)CR_OBB_F4 * sub);
+                    const float4* cone = ldg_ptr(&sg->subCones) + 2ull * sub;
+                    keep = !obb_misses_samples(P, tg.fa, p.f, Wf, Hf, ob) &&
+                           !item_back_facing(P, __ldg(cone), __ldg(cone + 1), ob.c, obb_radius(ob));
+                }
+            }
+            uint32_t rest = __ballot_sync(FULL, keep);
             while (rest) {
-                const uint32_t b0 = (uint32_t)__ffs(rest) - 1;
+                const int b0 = __ffs(rest) - 1;
                 rest &= rest - 1;
-                const uint32_t b1 = rest ? (uint32_t)__ffs(rest) - 1 : 32u;
+                const int b1 = rest ? __ffs(rest) - 1 : -1;
                 rest &= rest - 1;
-                const uint32_t b = lane < 16 ? b0 : b1;  // pair 32 t + b: instance rank, sub-box
-                const uint32_t inst = ib + __shfl_sync(FULL, slotOf, (t * 4 + (int)(b >> 3)) & 31);
-                const uint32_t tp = CR_SUB * (b & 7u) + (uint32_t)(lane & 15);
-                const uint32_t tri = tri0 + tp;
-                int res = S1_CULL;
-                if (b < 32u && tri < numTri) {
-                    const V3 pa = pos_of(geo, index_of(tp, 0));
-                    const V3 pb = pos_of(geo, index_of(tp, 1));
-                    const V3 pc = pos_of(geo, index_of(tp, 2));
-                    res = stage1_triangle(tg, tg.fa, load_mat(p.world_view + 4ull * inst),
-                                          __ldg(&p.instances[inst].flip), pa, pb, pc,
-                                          __ldg(&p.instances[inst].cum) + tri);
+                const int b = lane < 16 ? b0 : b1;  // the lane that tested this half's sub-box
+                const uint32_t in = __shfl_sync(FULL, inst, b & 31);
+                const uint32_t tri = __shfl_sync(FULL, sub, b & 31) * CR_SUB + (uint32_t)(lane & 15);
+                const CrInstance* I = p.instances + in;
+                bool left = b >= 0 && tri < __ldg(&I->numTriangles);
+                if (left && p.instProof) {
+                    const GeomRef g = geom_of_t<PACKED>(I);
+                    const V3 pa = pos_of(g, geom_index(g, 3ull * tri + 0));
+                    const V3 pb = pos_of(g, geom_index(g, 3ull * tri + 1));
+                    const V3 pc = pos_of(g, geom_index(g, 3ull * tri + 2));
+                    left = !quick_misses(make_quick(load_proof(p, in), tg.fa, p.f, Wf, Hf), pa, pb, pc);
                 }
-                append_nontrivial(p, res == S1_QUEUE, inst, tri);
-            }
-        }
-        __syncwarp();
-        {  // every read of this slot is done: refill it with the item STAGES ahead
-            const uint64_t npk = pk + (uint64_t)STAGES * nw;
-            if (npk < nItems) {
-                const Item nt = decode_item(p, item_at(npk));
-                const TileSrc ns = tile_source(p.segments + nt.seg, nt.batch);
-                if (ns.src) {
-                    pending |= bit;
-                    if (lane == 0) {
-                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                        bulk_load(s_idx[w][slot], ns.src, ns.bytes, &s_bar[w][slot]);
-                    }
-                }
+                const unsigned lm = __ballot_sync(FULL, left);
+                if (left) ring[(qt + __popc(lm & ((1u << lane) - 1u))) & (S1_RING - 1)] = ((uint64_t)in << 32) | tri;
+                qt += __popc(lm);
+                __syncwarp();
+                if (qt - qh >= 32u) append_survivors<PACKED>(p, tg, ring, qh, qt);
             }
         }
     }
-    // only after a timeout can copies still be in flight: wait for them
-    // (bounded) so none lands in shared memory after the block has exited
-    for (int s = 0; s < STAGES; ++s)
-        if (pending & (1u << s)) (void)mbar_wait_bounded(&s_bar[w][s], (parity >> s) & 1u, p.waitTimeoutNs);
+    if (qt > qh) append_survivors<PACKED>(p, tg, ring, qh, qt);
 }
 
 // resolve.cu:213-232 (0xFFFFFFF0'00000000 per pixel), 16-byte stores; block 0
@@ -1005,6 +1070,10 @@ int cr_query_launch_shape(int device, CrLaunchShape* out) {
         cudaSuccess)
         return -1;
     out->s1RasterOwnBlocks = sms * (bo > 0 ? bo : 1);
+    int bd = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bd, k_s1direct<S1_WARPS, false>, S1_WARPS * 32, 0) != cudaSuccess)
+        return -1;
+    out->s1DirectBlocks = sms * (bd > 0 ? bd : 1);
     out->stage3Blocks = sms * (b3 > 0 ? b3 : 1);
     int bb = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bb, k_stage3_bins, B3_THREADS, 0) != cudaSuccess) return -1;
@@ -1059,37 +1128,49 @@ int cr_launch_cull(const CrFrameParams& p, const CrLaunchShape& s, void* stream)
     return launch_pdl(k_stamp<256>, (unsigned)(s.numSMs * 4), 256, stream, p);
 }
 
-// Box-culled frames: k_stage1.  Record-culled frames: k_s1cull (items ->
-// survivor list) then k_s1raster (survivors -> visbuffer / stage-2 queue).
-int cr_launch_stage1(const CrFrameParams& p, const CrLaunchShape& s, void* stream) {
-    if (p.numItems == 0) return 0;
-    if (p.direct) {
-        const uint64_t want = (p.direct + S1_WARPS * 32 - 1) / (S1_WARPS * 32);
-        const unsigned b = (unsigned)std::min<uint64_t>(want, (uint64_t)s.s1RasterBlocks);
-        const unsigned T = S1_WARPS * 32;
-        if (p.coopRaster)
-            return p.anyPacked ? launch_pdl(k_s1raster<S1_WARPS, true, true, true>, b, T, stream, p)
-                               : launch_pdl(k_s1raster<S1_WARPS, false, true, true>, b, T, stream, p);
-        return p.anyPacked ? launch_pdl(k_s1raster<S1_WARPS, true, false, true>, b, T, stream, p)
-                           : launch_pdl(k_s1raster<S1_WARPS, false, false, true>, b, T, stream, p);
-    }
-    const uint64_t itemBlocks = (p.numItems + S1_WARPS - 1) / S1_WARPS;
+namespace {
+// Survivors -> visbuffer / stage-2 queue.
+int launch_s1raster(const CrFrameParams& p, const CrLaunchShape& s, void* stream) {
     const unsigned T = S1_WARPS * 32;
-    if (p.cellMode == CR_REC_BOXES) {
-        const unsigned b = (unsigned)std::min<uint64_t>(itemBlocks, (uint64_t)s.stage1Blocks);
-        return p.anyPacked ? launch_pdl(k_stage1<S1_WARPS, true>, b, T, stream, p)
-                           : launch_pdl(k_stage1<S1_WARPS, false>, b, T, stream, p);
-    }
-    const unsigned bc = (unsigned)std::min<uint64_t>(itemBlocks, (uint64_t)s.s1CullBlocks);
-    if (p.anyPacked ? launch_pdl(k_s1cull<S1_WARPS, true>, bc, T, stream, p)
-                    : launch_pdl(k_s1cull<S1_WARPS, false>, bc, T, stream, p))
-        return -1;
     const unsigned br = (unsigned)(p.coopRaster || s.s1RasterOwnBlocks <= 0 ? s.s1RasterBlocks : s.s1RasterOwnBlocks);
     if (p.coopRaster)
         return p.anyPacked ? launch_pdl(k_s1raster<S1_WARPS, true, true>, br, T, stream, p)
                            : launch_pdl(k_s1raster<S1_WARPS, false, true>, br, T, stream, p);
     return p.anyPacked ? launch_pdl(k_s1raster<S1_WARPS, true, false>, br, T, stream, p)
                        : launch_pdl(k_s1raster<S1_WARPS, false, false>, br, T, stream, p);
+}
+}  // namespace
+
+// Box-culled frames: k_stage1, record-culled frames: k_s1cull (items -> survivor
+// list); then k_s1raster.
+int cr_launch_stage1(const CrFrameParams& p, const CrLaunchShape& s, void* stream) {
+    if (p.numItems == 0) return 0;
+    if (p.direct) {
+        const uint64_t want = (p.direct + S1_WARPS * 32 - 1) / (S1_WARPS * 32);
+        const unsigned T = S1_WARPS * 32;
+        if (p.coopRaster) {  // a warp may take as little as one triangle
+            const unsigned bc = (unsigned)std::min<uint64_t>(want * 32, (uint64_t)s.s1RasterBlocks);
+            return p.anyPacked ? launch_pdl(k_s1raster<S1_WARPS, true, true, true>, bc, T, stream, p)
+                               : launch_pdl(k_s1raster<S1_WARPS, false, true, true>, bc, T, stream, p);
+        }
+        const unsigned bd = (unsigned)std::min<uint64_t>(want, (uint64_t)s.s1DirectBlocks);
+        return p.anyPacked ? launch_pdl(k_s1direct<S1_WARPS, true>, bd, T, stream, p)
+                           : launch_pdl(k_s1direct<S1_WARPS, false>, bd, T, stream, p);
+    }
+    const uint64_t itemBlocks = (p.numItems + S1_WARPS - 1) / S1_WARPS;
+    const unsigned T = S1_WARPS * 32;
+    if (p.cellMode == CR_REC_BOXES) {
+        const unsigned b = (unsigned)std::min<uint64_t>(itemBlocks, (uint64_t)s.stage1Blocks);
+        if (p.anyPacked ? launch_pdl(k_stage1<S1_WARPS, true>, b, T, stream, p)
+                        : launch_pdl(k_stage1<S1_WARPS, false>, b, T, stream, p))
+            return -1;
+        return launch_s1raster(p, s, stream);
+    }
+    const unsigned bc = (unsigned)std::min<uint64_t>(itemBlocks, (uint64_t)s.s1CullBlocks);
+    if (p.anyPacked ? launch_pdl(k_s1cull<S1_WARPS, true>, bc, T, stream, p)
+                    : launch_pdl(k_s1cull<S1_WARPS, false>, bc, T, stream, p))
+        return -1;
+    return launch_s1raster(p, s, stream);
 }
 
 int cr_launch_stage2(const CrFrameParams& p, const CrLaunchShape& s, void* stream) {

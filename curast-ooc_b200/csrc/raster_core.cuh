@@ -255,8 +255,11 @@ __device__ __forceinline__ Target target_of(const CrFrameParams& p, uint32_t vie
 }
 
 // With COOP the tiny raster is not run here: its setup goes to *coop and
-// S1_RASTER is returned, for stage1_coop_raster to run across the warp.
-template <bool COOP = false>
+// S1_RASTER is returned, for stage1_coop_raster to run across the warp.  QUOT:
+// the frustum sides are tested on the quotients, for triangles that an earlier
+// test let through (few of them are off screen, and the division-free tests are
+// most of the code: instruction fetch held the kernels up).
+template <bool COOP = false, bool QUOT = REF_MATH>
 __device__ __forceinline__ int stage1_triangle(const Target& p, const float fa, const Mat& M,
                                                const uint32_t flip, const V3 pa, const V3 pb, const V3 pc,
                                                const uint64_t id, S1Raster* coop = nullptr) {
@@ -281,7 +284,7 @@ __device__ __forceinline__ int stage1_triangle(const Target& p, const float fa, 
     bool nontrivial = (da <= 0.0f || db <= 0.0f || dc <= 0.0f);
     const float Xa = fa * av.x, Xb = fa * bv.x, Xc = fa * cv.x;
     const float Ya = f * av.y, Yb = f * bv.y, Yc = f * cv.y;
-    if constexpr (!REF_MATH) {
+    if constexpr (!QUOT) {
         if (!nontrivial) {  // tv.cu:113-118, on fl(X/d) without dividing
             if (ndc_beyond(Xa, da) && ndc_beyond(Xb, db) && ndc_beyond(Xc, dc)) return S1_CULL;
             if (ndc_beyond(-Xa, da) && ndc_beyond(-Xb, db) && ndc_beyond(-Xc, dc)) return S1_CULL;
@@ -292,8 +295,8 @@ __device__ __forceinline__ int stage1_triangle(const Target& p, const float fa, 
     const V3 an = {Xa / da, Ya / da, da};  // viewToNDC, helpers:95-101
     const V3 bn = {Xb / db, Yb / db, db};
     const V3 cn = {Xc / dc, Yc / dc, dc};
-    if constexpr (REF_MATH) {
-        if (!nontrivial) {  // tv.cu:113-118 on the build's own quotients
+    if constexpr (QUOT) {
+        if (!nontrivial) {  // tv.cu:113-118
             if (an.x > +1.0f && bn.x > +1.0f && cn.x > +1.0f) return S1_CULL;
             if (an.x < -1.0f && bn.x < -1.0f && cn.x < -1.0f) return S1_CULL;
             if (an.y > +1.0f && bn.y > +1.0f && cn.y > +1.0f) return S1_CULL;
@@ -412,6 +415,7 @@ __device__ __forceinline__ void stage1_own_raster(const Target& p, const S1Raste
 // the same fragments are written; the warp no longer waits on its largest
 // triangle.  Rows of a triangle without columns are skipped (they write
 // nothing).  All lanes of the warp must call it.
+template <bool VIEWS = false>
 __device__ __forceinline__ void stage1_coop_raster(const Target& p, const bool mine, const S1Raster& r,
                                                    const uint64_t id) {
     const int lane = threadIdx.x & 31;
@@ -423,7 +427,10 @@ __device__ __forceinline__ void stage1_coop_raster(const Target& p, const bool m
         if (lane >= d) incl += v;
     }
     const int total = __shfl_sync(FULL, incl, 31);
-    const uint32_t numPixels = (uint32_t)p.W * (uint32_t)p.H;
+    uint32_t numPixels = (uint32_t)p.W * (uint32_t)p.H;
+    const uint32_t ownPixels = numPixels;
+    uint64_t* fb = p.fb;
+    int W = p.W;
     for (int base = 0; base < total; base += 32) {
         const int k = base + lane;
         int j = 0;  // the lane whose rows hold task k: first with incl > k
@@ -445,6 +452,11 @@ __device__ __forceinline__ void stage1_coop_raster(const Target& p, const bool m
         const int row_pid = __shfl_sync(FULL, r.row_pid, j);
         const int size_x = __shfl_sync(FULL, r.size_x, j);
         const uint64_t tid = __shfl_sync(FULL, (unsigned long long)id, j);
+        if constexpr (VIEWS) {
+            fb = (uint64_t*)__shfl_sync(FULL, (unsigned long long)p.fb, j);
+            W = __shfl_sync(FULL, p.W, j);
+            numPixels = __shfl_sync(FULL, ownPixels, j);
+        }
         if (k >= total) continue;
         const int fy = k - first;
         for (int i = 0; i < fy; ++i) {
@@ -453,19 +465,33 @@ __device__ __forceinline__ void stage1_coop_raster(const Target& p, const bool m
         }
         float s = s_row;
         float t = t_row;
-        int pid = row_pid + fy * p.W;
+        int pid = row_pid + fy * W;
         for (int fx = 0; fx < size_x; ++fx) {
             const float v = 1.0f - (s + t);
             if (s > 0.0f && t > 0.0f && v > 0.0f && (uint32_t)pid < numPixels) {
                 const float inv_depth = v * iza + s * izb + t * izc;
                 const float depth = ref_fdiv(1.0f, inv_depth);
-                fb_min(p.fb, (uint32_t)pid, pack_pixel(depth, tid));
+                fb_min(fb, (uint32_t)pid, pack_pixel(depth, tid));
             }
             s += ds_dx;
             t += dt_dx;
             pid++;
         }
     }
+}
+
+// A warp with a lane whose tiny raster has more fragments than this runs them together
+#ifndef CR_COOP_MIN_FRAGMENTS
+#define CR_COOP_MIN_FRAGMENTS 8
+#endif
+// The lanes' tiny rasters (S1_RASTER): spread over the warp when one of them
+// would hold the others up, else each lane its own.
+template <bool VIEWS = false>
+__device__ __forceinline__ void s1_raster_lanes(const Target& tg, const int res, const S1Raster& ras, const uint64_t rid) {
+    const bool mine = res == S1_RASTER;
+    const int frags = mine ? max(ras.size_x, 0) * max(ras.size_y, 0) : 0;
+    if (__reduce_max_sync(FULL, (unsigned)frags) > CR_COOP_MIN_FRAGMENTS) stage1_coop_raster<VIEWS>(tg, mine, ras, rid);
+    else if (mine) stage1_own_raster(tg, ras, rid);
 }
 
 // ---------------------------------------------------------------------------
@@ -624,6 +650,36 @@ __device__ __forceinline__ float row_pos(const float4 r, const V3 c) {
     return __fmaf_rn(r.x, c.x, __fmaf_rn(r.y, c.y, __fmaf_rn(r.z, c.z, r.w)));
 }
 
+// A radius about the centre that holds the box: its axes are orthogonal up to
+// 2^-23 of their lengths.
+__device__ __forceinline__ float obb_radius(const Obb& b) {
+    auto sq = [](const V3 a) { return __fmaf_rn(a.x, a.x, __fmaf_rn(a.y, a.y, a.z * a.z)); };
+    return sqrtf(sq(b.a0) + (sq(b.a1) + sq(b.a2))) * 1.00001f;
+}
+
+// The largest |coordinate| of the box, per axis.
+__device__ __forceinline__ V3 obb_max_abs(const Obb& b) {
+    return V3{fabsf(b.c.x) + fabsf(b.a0.x) + fabsf(b.a1.x) + fabsf(b.a2.x),
+              fabsf(b.c.y) + fabsf(b.a0.y) + fabsf(b.a1.y) + fabsf(b.a2.y),
+              fabsf(b.c.z) + fabsf(b.a0.z) + fabsf(b.a1.z) + fabsf(b.a2.z)};
+}
+
+// The rows and row sums obb_misses_samples needs (no eye: not for
+// item_back_facing), for points of at most mabs.  The sums are of positive terms,
+// within 6u of the exact ones.
+__device__ __forceinline__ Proof proof_rows(const Mat& M, const V3 mabs) {
+    auto sum = [&](float a, float b, float c, float t) {
+        return __fmaf_rn(fabsf(a), mabs.x, __fmaf_rn(fabsf(b), mabs.y, __fmaf_rn(fabsf(c), mabs.z, fabsf(t)))) * 1.000001f;
+    };
+    Proof P;
+    P.rx = make_float4(M.c0.x, M.c1.x, M.c2.x, M.c3.x);
+    P.ry = make_float4(M.c0.y, M.c1.y, M.c2.y, M.c3.y);
+    P.rz = make_float4(M.c0.z, M.c1.z, M.c2.z, M.c3.z);
+    P.S = make_float4(sum(M.c0.x, M.c1.x, M.c2.x, M.c3.x), sum(M.c0.y, M.c1.y, M.c2.y, M.c3.y),
+                      sum(M.c0.z, M.c1.z, M.c2.z, M.c3.z), 0.0f);
+    return P;
+}
+
 // One screen axis of obb_misses_samples: true if every point of the box has
 // a stage-1 screen coordinate strictly inside (k, k + 1) for one integer
 // k >= 0.  F = fa (or f), row the x (or y) row, S its bound, size W (or H); dz
@@ -632,14 +688,14 @@ __device__ __forceinline__ float row_pos(const float4 r, const V3 c) {
 //
 // The exact coordinate is s(p) = W ((X / D) / 2 + 1/2) - 1/2.  For any number
 // r0, X / D - r0 = (X - r0 D) / D, and X - r0 D is affine: its centre value plus
-// at most e = sum_j |F g_xj + r0 g_zj| (D = -q.z).  With r0 the float quotient of
-// the centre, everything float about this -- the centre's X, D and quotient, the
-// steps, e -- is off by less than 48u (|F| S + |r0| Sz) in the numerator (u =
-// 2^-24; each row form errs by 3u S per term, and an axis' terms are at most
-// twice S), and stage 1's own X and d of a vertex by 5u of the same, over a d no
-// less than the least depth; 96u is allowed.  Its quotient, and the scale to
-// pixels there and here, round by less than 16u W (|r0| + 2) pixels; 32u is
-// allowed.  k >= 0: for k = -1 the bounding box's clamp to 0 makes floor(min_x)
+// at most e = sum_j |F g_xj + r0 g_zj| (D = -q.z).  With u = 2^-24, the centre's
+// float X and D are off by less than 4u |F| S and 3u Sz, the three steps and their
+// sum by less than 16u (|F| S + |r0| Sz) together (a step's terms add up to at most
+// twice S), and stage 1's own X and d of a vertex by 5u |F| S and 4u Sz: all over a d
+// no less than the least depth.  25u (|F| S + |r0| Sz) in the numerator; 28u is
+// allowed (the quotient of a vertex is within 1e-3 of r0 where anything is
+// proven).  Its quotient, and the scale to pixels there and here, round by less
+// than 4u W pixels at r0 = 0 and 7u W at |r0| = 1; 6u W (|r0| + 1) is allowed.  k >= 0: for k = -1 the bounding box's clamp to 0 makes floor(min_x)
 // = 0 and the cull fails; for k >= W - 1 the clamp of max_x to W - 1 keeps
 // max_x < k + 1 and the cull holds.  NaN and infinity fail the comparisons.
 __device__ __forceinline__ bool axis_misses_samples(float F, const float4 row, float S, float Sz, const Obb& b, float D0,
@@ -650,8 +706,8 @@ __device__ __forceinline__ bool axis_misses_samples(float F, const float4 row, f
                     fabsf(__fmaf_rn(r0, gz.y, F * row_dir(row, b.a1))) +
                     fabsf(__fmaf_rn(r0, gz.z, F * row_dir(row, b.a2)));
     const float ar = fabsf(r0);
-    const float h = 0.5f * W * ((e + (96.0f * u * (fabsf(F) * S + (ar + 1.0f) * Sz) + 1e-30f)) * iD) +
-                    32.0f * u * W * (ar + 2.0f);
+    const float h = 0.5f * W * ((e + (28.0f * u * (fabsf(F) * S + (ar + 1e-3f) * Sz) + 1e-30f)) * iD) +
+                    6.0f * u * W * (ar + 1.0f);
     const float s0 = W * (0.5f * r0 + 0.5f) - 0.5f;
     const float lo = s0 - h, hi = s0 + h, k = floorf(lo);
     return lo > k && k >= 0.0f && hi < k + 1.0f && h < 0.5f;
@@ -669,11 +725,75 @@ __device__ __forceinline__ bool obb_misses_samples(const Proof& P, float fa, flo
     const float3 gz = make_float3(row_dir(P.rz, b.a0), row_dir(P.rz, b.a1), row_dir(P.rz, b.a2));
     const float D0 = -row_pos(P.rz, b.c);
     // the least depth, less every rounding of it (here and in stage 1)
-    const float Dmin = (D0 - (fabsf(gz.x) + fabsf(gz.y) + fabsf(gz.z))) - (64.0f * u * P.S.z + 1e-30f);
+    const float Dmin = (D0 - (fabsf(gz.x) + fabsf(gz.y) + fabsf(gz.z))) - (32.0f * u * P.S.z + 1e-30f);
     if (!(Dmin > 1e-30f && Dmin < 1e30f)) return false;
     const float iD = __fdividef(1.0f, Dmin) * 1.00000095367431640625f;
     return axis_misses_samples(fa, P.rx, P.S.x, P.S.z, b, D0, gz, iD, W) ||
            axis_misses_samples(f, P.ry, P.S.y, P.S.z, b, D0, gz, iD, H);
+}
+
+// The sample-miss (or frustum-side) proof of one triangle: obb_misses_samples' argument with a
+// point for a box, cheap enough to run ahead of the exact path.  Of the triangles
+// of a dense mesh that reach stage 1 with no record most miss every sample (87 % of
+// those of a 60M-triangle terrain's visible items are culled, 99.5 % of those of
+// 3000 x 1M-triangle spheres), and stage1_triangle finds that out after six
+// divisions, at about 500 issue slots per 32 triangles; this takes about 60.
+//
+// rx, ry are scaled to pixels (F W / 2, f H / 2).  With u = 2^-24 and an on-screen
+// quotient (|X / D| <= 1.01; where every vertex is further out than that on an
+// axis, every one is beyond the same side and the triangle is culled all the same),
+// this position and stage 1's own differ from the exact one by less than
+// (W / 2) u (11 |F| S + 8 Sz) / D and 6u W together: fused sums of the scaled rows
+// (6u S), the reciprocal (2 ulp), the depth (3u Sz), stage 1's transform (4u S,
+// 4u Sz), quotient and scale.  c1 allows 12u and 12u, c2 8u W.
+struct Quick {
+    float4 rx, ry, rz;
+    float cx, cy, c1x, c1y, c2x, c2y, ez;
+};
+
+__device__ __forceinline__ Quick make_quick(const Proof& P, float fa, float f, float W, float H) {
+    const float u = 5.9604644775390625e-08f;
+    const float kx = 0.5f * W * fa, ky = 0.5f * H * f;
+    Quick q;
+    q.rx = make_float4(P.rx.x * kx, P.rx.y * kx, P.rx.z * kx, P.rx.w * kx);
+    q.ry = make_float4(P.ry.x * ky, P.ry.y * ky, P.ry.z * ky, P.ry.w * ky);
+    q.rz = P.rz;
+    q.cx = 0.5f * W - 0.5f;
+    q.cy = 0.5f * H - 0.5f;
+    q.c1x = 6.0f * u * W * (fabsf(fa) * P.S.x + P.S.z);
+    q.c1y = 6.0f * u * H * (fabsf(f) * P.S.y + P.S.z);
+    q.c2x = 8.0f * u * W;
+    q.c2y = 8.0f * u * H;
+    q.ez = 16.0f * u * P.S.z + 1e-30f;
+    return q;
+}
+
+__device__ __forceinline__ float rcp_fast(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+__device__ __forceinline__ bool quick_misses(const Quick& q, const V3 a, const V3 b, const V3 c) {
+    const float da = -row_pos(q.rz, a), db = -row_pos(q.rz, b), dc = -row_pos(q.rz, c);
+    const float ra = rcp_fast(da), rb = rcp_fast(db), rc = rcp_fast(dc);
+    const float iD = fmaxf(ra, fmaxf(rb, rc)) * 1.00000095367431640625f;
+    const float xa = __fmaf_rn(row_pos(q.rx, a), ra, q.cx), xb = __fmaf_rn(row_pos(q.rx, b), rb, q.cx),
+                xc = __fmaf_rn(row_pos(q.rx, c), rc, q.cx);
+    const float ya = __fmaf_rn(row_pos(q.ry, a), ra, q.cy), yb = __fmaf_rn(row_pos(q.ry, b), rb, q.cy),
+                yc = __fmaf_rn(row_pos(q.ry, c), rc, q.cy);
+    const float mx = __fmaf_rn(q.c1x, iD, q.c2x), my = __fmaf_rn(q.c1y, iD, q.c2y);
+    const float lx = fminf(xa, fminf(xb, xc)) - mx, hx = fmaxf(xa, fmaxf(xb, xc)) + mx;
+    const float ly = fminf(ya, fminf(yb, yc)) - my, hy = fmaxf(ya, fmaxf(yb, yc)) + my;
+    const float kx = floorf(lx), ky = floorf(ly);
+    // NaN: fminf drops a NaN operand, so it is looked for in the sum
+    const bool num = (xa + xb + xc) + (ya + yb + yc) < INFINITY;
+    // one pixel column or row, or beyond one side (sx < -1/2 is X / D < -1,
+    // sx > W - 1/2 is X / D > 1; further out the error grows as the distance does,
+    // far below it)
+    return num && da > q.ez && db > q.ez && dc > q.ez &&
+           ((kx >= 0.0f && hx < kx + 1.0f) || (ky >= 0.0f && hy < ky + 1.0f) || hx < -0.5f || hy < -0.5f ||
+            lx > 2.0f * q.cx + 0.5f || ly > 2.0f * q.cy + 0.5f);
 }
 
 // True if every triangle of an item is culled by stage 1's back-face test
@@ -695,10 +815,10 @@ __device__ __forceinline__ bool obb_misses_samples(const Proof& P, float fa, flo
 // is doubled, and its own single-precision sum (all terms positive) is covered by
 // 1.001.  When |det R| nMin G > E every triangle's float res has the sign that
 // culls it (1e-30: products that underflow prove nothing).
-// c0, c1: the item's CR_CONE_FLOATS; mid: the centre of its box, r half its
-// diagonal.
-__device__ __forceinline__ bool item_back_facing(const Proof& P, const float4 c0, const float4 c1, const V3 mid) {
-    const float detA = P.det.x, cosT = c0.w, nMin = c1.x, edge = c1.y, sinT = c1.z, r = c1.w;
+// c0, c1: the item's CR_CONE_FLOATS; mid, r: a ball that holds its vertices.
+__device__ __forceinline__ bool item_back_facing(const Proof& P, const float4 c0, const float4 c1, const V3 mid,
+                                                 const float r) {
+    const float detA = P.det.x, cosT = c0.w, nMin = c1.x, edge = c1.y, sinT = c1.z;
     if (!(detA > 0.0f) || !(cosT > 0.0f)) return false;
     const V3 w = {mid.x - P.eye.x, mid.y - P.eye.y, mid.z - P.eye.z};
     const float p = fmaxf(fabsf(mid.x), fmaxf(fabsf(mid.y), fabsf(mid.z))) + r;  // >= max |p_j|
@@ -746,21 +866,17 @@ __device__ __forceinline__ uint64_t vertex_cell_record(const Mat& M, V3 p, float
     return rec;
 }
 
-// 32-bit cell record (shared-memory records of box-culled frames, W and H at
-// most 4096): bits 0..4 the outcode, bit 5 on screen, bit 6 x not an
+// 32-bit cell record (W and H at most 4096): bits 0..4 the outcode, bit 5 on screen, bit 6 x not an
 // integer, bit 7 y not an integer, bits 8..19 floor(x), bits 20..31 floor(y).
-// `sides`: false when the vertex is known to be in front of the camera and
-// inside every frustum side (outcode 0, no predicates evaluated).
 #define CR_C32_INSIDE 0x20u
 #define CR_C32_FRACX 0x40u
 #define CR_C32_FRACY 0x80u
-template <bool SIDES>
 __device__ __forceinline__ uint32_t vertex_cell32(const Mat& M, V3 p, float fa, float f, float Wf, float Hf,
                                                   float Wm1, float Hm1) {
     const V3 q = xform(M, p);
     const float d = -q.z;
     const float X = fa * q.x, Y = f * q.y;
-    if (SIDES && d <= 0.0f) return CR_OC_BEHIND;
+    if (d <= 0.0f) return CR_OC_BEHIND;
     const float qx = X / d, qy = Y / d;
     const V2 s = to_screen(V3{qx, qy, d}, Wf, Hf);
     const float sx = s.x - 0.5f, sy = s.y - 0.5f;
@@ -772,7 +888,6 @@ __device__ __forceinline__ uint32_t vertex_cell32(const Mat& M, V3 p, float fa, 
         return CR_C32_INSIDE | (sx > fx ? CR_C32_FRACX : 0u) | (sy > fy ? CR_C32_FRACY : 0u) |
                ((uint32_t)(int)fx << 8) | ((uint32_t)(int)fy << 20);
     }
-    if (!SIDES) return 0u;
     // the sides from the quotients themselves: ndc_beyond(X, d) is fl(X / d)
     // > 1, and ndc_beyond(-X, d) is fl(X / d) < -1 (rounding to nearest is
     // symmetric)
@@ -847,7 +962,7 @@ __device__ __forceinline__ bool item_uses_tma(const CrSegment* sg, uint32_t batc
 
 constexpr int S1_STAGES = 3;
 constexpr int S1_R = CR_BATCH / 32;  // triangles per lane per work item
-constexpr int S1_RING = 256;         // stage-1 survivor ring entries per warp
+constexpr uint32_t S1_RING = 64;     // per-warp queue for the full path: below 32 before a push of at most 32
 
 
 // ---------------------------------------------------------------------------

@@ -191,12 +191,6 @@ __device__ __forceinline__ const ulonglong2* record_of(const CrFrameParams& p, c
     return reinterpret_cast<const ulonglong2*>(rec + v);
 }
 
-struct TileSrc {
-    const void* src;
-    uint32_t bytes;
-    bool local;
-};
-
 // Views of one triangle that survive the all-behind and all-beyond-one-side
 // culls (tv.cu:110-119) given its three vertex records.
 __device__ __forceinline__ unsigned long long surviving_views(const CrFrameParams& p, const CrViewMasks* rec,
@@ -594,263 +588,211 @@ __global__ void __launch_bounds__(256) k_cull_views(const CrFrameParams p) {
     }
 }
 
-#ifndef CR_RECORD_SPAN_PX
-#define CR_RECORD_SPAN_PX 12.0f
-#endif
-// Whether cell records of an item's vertices are likely to cull most of its
-// triangles in one view: the item box's projected extent, bounded from its
-// bounding sphere, is small enough for its 128 triangles to be about a pixel
-// or less.  Only the speed depends on the answer.
-__device__ __forceinline__ bool records_pay(const Mat& M, const Target& tg, const float box[6], bool hasBox) {
-    if (!hasBox) return true;
-    const float cx = 0.5f * (box[0] + box[3]), cy = 0.5f * (box[1] + box[4]), cz = 0.5f * (box[2] + box[5]);
-    const float ex = box[3] - box[0], ey = box[4] - box[1], ez = box[5] - box[2];
-    const float r = 0.5f * sqrtf(ex * ex + ey * ey + ez * ez);
-    // largest column norm of the 3x3 part: the view-space radius bound
-    const float s0 = M.c0.x * M.c0.x + M.c0.y * M.c0.y + M.c0.z * M.c0.z;
-    const float s1 = M.c1.x * M.c1.x + M.c1.y * M.c1.y + M.c1.z * M.c1.z;
-    const float s2 = M.c2.x * M.c2.x + M.c2.y * M.c2.y + M.c2.z * M.c2.z;
-    const float rv = r * sqrtf(fmaxf(s0, fmaxf(s1, s2))) * 1.01f;
-    const float d = -((M.c0.z * cx + M.c1.z * cy) + (M.c2.z * cz + M.c3.z));
-    if (!(d - rv > 0.0f)) return false;  // near or behind the camera: large on screen
-    const float spanPx = rv * fmaxf(tg.f, tg.fa) * (float)max(tg.W, tg.H) / (d - rv);
-    return spanPx < CR_RECORD_SPAN_PX;
-}
-
-// Stage 1 of batched frames whose meshes have per-item vertex lists (the
-// frame cull's item list is required; no vertex pass runs).  Per item the
-// warp's TMA ring carries the item's 1536-byte vertex-list block.  Per
-// (instance, view) of the item: where the item is small on screen, the warp
-// computes the 32-bit cell records of the item's distinct vertices in shared
-// memory -- without the frustum predicates in views whose frustum holds the
-// item's box -- culls each triangle from its three records and queues the
-// rest (view, instance, triangle) in a per-warp ring that runs the
-// reference's full path 32 at a time; where it is large, every triangle runs
-// the full path at once with the view's target and matrix for the warp.
-// Items without a list run every triangle in every view of the item.
-template <int WARPS, int MINB, bool PACKED>
-__global__ void __launch_bounds__(WARPS * 32, MINB) k_stage1_views_lists(const CrFrameParams p) {
-    constexpr int STAGES = 2;
-    __shared__ __align__(128) uint32_t s_idx[WARPS][STAGES][CR_BATCH * 3];
-    __shared__ __align__(8) uint64_t s_bar[WARPS][STAGES];
-    __shared__ uint32_t s_rec[WARPS][CR_LOCAL_MAX];
-    __shared__ uint32_t s_ring[WARPS][S1_RING];
+// Stage 1 of batched frames from the frame cull's item list alone (no vertex
+// pass runs).  Per (instance, view) of an item the warp proves, four views at a time
+// (a lane per view and CR_SUB triangles), that an oriented sub-box misses every
+// sample or that its triangles all face away, tests the triangles of the other sub-boxes
+// one per lane (quick_misses), two sub-boxes at a time, and queues those still left for
+// the reference's full path, 32 at a time across its items.  COARSE (views of half a
+// pixel and more per triangle): the triangles are not tested ahead of the path, and the
+// warp shares its lanes' rasters.
+//
+// Bound by instruction issue.  64 views over the 60M-triangle terrain (0.02 pixels per
+// triangle; 33 % of the triangles face away, 52 % miss every sample, 13 % are drawn), ms:
+// every triangle of an item that is large on screen through the full path, and cell
+// records of the distinct vertices of the others, 18.4; quick_misses ahead of the path
+// 14.0; indices by plain loads instead of a TMA tile per item, which freed 20 registers
+// of spilled state, 13.2.  Where the triangles are larger the test is wasted and one
+// lane's needle holds the others up: 33 views, fine / COARSE, ms: 732K triangles at
+// 0.9 pixels each 0.578 / 0.500, at 3.5 1.04 / 0.80, 180K at 14 0.69 / 0.42, 2.9M at 0.9
+// 1.51 / 1.40; but 732K at 0.22 0.337 / 0.347, 2.9M at 0.05 0.56 / 0.74.
+constexpr uint32_t V1_UNITS = 4;   // units of work per warp, at least
+template <int WARPS, int MINB, bool PACKED, bool COARSE>
+__global__ void __launch_bounds__(WARPS * 32, MINB) k_stage1_views_boxes(const CrFrameParams p) {
+    __shared__ uint64_t s_ring[WARPS][S1_RING];
     const int lane = threadIdx.x & 31;
     const int w = threadIdx.x >> 5;
     const uint64_t gw = (uint64_t)blockIdx.x * WARPS + w;
     const uint64_t nw = (uint64_t)gridDim.x * WARPS;
     const unsigned long long valid = valid_views(p.numViews);
 
-    if (lane == 0) {
-        for (int s = 0; s < STAGES; ++s) mbar_init(&s_bar[w][s], 1);
-        fence_barrier_init();
-    }
-    __syncwarp();
     const uint64_t nItems = min((uint64_t)p.counters[CR_CTR_ITEMS], p.itemCap);
-    // the ring slot's source: vertex-list block, index tile, or nothing
-    auto source = [&](uint64_t k) -> TileSrc {
-        const Item it = decode_item(p, (uint64_t)__ldg(&p.itemViews[k].item));
-        const CrSegment* sg = p.segments + it.seg;
-        const uint32_t* lc = ldg_ptr(&sg->localCounts);
-        if (lc && __ldg(lc + it.batch) <= CR_LOCAL_MAX)
-            return TileSrc{ldg_ptr(&sg->localLists) + (uint64_t)it.batch * CR_LOCAL_BYTES, CR_LOCAL_BYTES, true};
-        if (item_uses_tma(sg, it.batch))
-            return TileSrc{ldg_ptr(&sg->indices) + (uint64_t)it.batch * (CR_BATCH * 3), CR_BATCH * 12, false};
-        return TileSrc{nullptr, 0, false};
-    };
-    uint32_t pending = 0;
-    for (int s = 0; s < STAGES; ++s) {
-        const uint64_t pk = gw + (uint64_t)s * nw;
-        if (pk >= nItems) break;
-        const TileSrc ts = source(pk);
-        if (ts.src) {
-            pending |= 1u << s;
-            if (lane == 0) bulk_load(s_idx[w][s], ts.src, ts.bytes, &s_bar[w][s]);
-        }
-    }
-    __syncwarp();
+    // Some units of work per warp: an item, or its part in `per` consecutive views
+    // where there are too few items (a 33-view frame of 180K triangles has 1,407 for
+    // 3,552 warps: 0.375 -> 0.287 ms).  The parts of all items in the first views come
+    // first: with an item's parts next to one another the views' targets
+    // compete for L2 (2.9M triangles at 0.9 pixels 1.49 unsplit, 1.68; so 1.53).
+    const uint32_t fours = (p.numViews + 3) / 4;
+    const uint64_t parts = max((uint64_t)1, min((uint64_t)fours, (V1_UNITS * nw + nItems) / (nItems + 1)));
+    const uint32_t per = 4 * (uint32_t)((fours + parts - 1) / parts);
+    const uint32_t split = (p.numViews + per - 1) / per;
 
-    uint32_t parity = 0;
-    uint32_t k = 0;
-    for (uint64_t pk = gw; pk < nItems; pk += nw, ++k) {
-        const int slot = (int)(k % STAGES);
-        const uint32_t bit = 1u << slot;
+    // Triangles no proof culls, as stage-2 queue entries (view, instance,
+    // triangle), queued across the warp's items and run through the reference's
+    // full path 32 at a time.
+    uint64_t* const ring = s_ring[w];
+    uint32_t qh = 0, qt = 0;  // ring head / tail (warp-uniform)
+    auto drain = [&]() {
+        const uint32_t j = qh + lane;
+        int res = S1_CULL;
+        uint64_t e = 0;
+        Target tg = {};
+        S1Raster ras;
+        uint64_t rid = 0;
+        if (j < qt) {
+            e = ring[j & (S1_RING - 1)];
+            const uint32_t view = (uint32_t)(e >> CR_ENTRY_VIEW_SHIFT);
+            const uint32_t inst = (uint32_t)((e >> 32) & CR_ENTRY_INST_MASK), tri = (uint32_t)e;
+            const uint64_t vi = (uint64_t)view * p.numInstances + inst;
+            tg = target_of(p, view);
+            const CrInstance* I = p.instances + inst;
+            const GeomRef g = geom_of_t<PACKED>(I);
+            const V3 pa = pos_of(g, geom_index(g, 3ull * tri + 0));
+            const V3 pb = pos_of(g, geom_index(g, 3ull * tri + 1));
+            const V3 pc = pos_of(g, geom_index(g, 3ull * tri + 2));
+            rid = __ldg(&I->cum) - tg.idBase + tri;
+            res = stage1_triangle<COARSE, true>(tg, tg.fa, load_mat(p.world_view + 4ull * vi), __ldg(p.flips + vi), pa, pb, pc, rid,
+                                                 &ras);
+        }
+        if constexpr (COARSE) s1_raster_lanes<true>(tg, res, ras, rid);
+        qh = min(qh + 32u, qt);
+        const unsigned qmask = __ballot_sync(FULL, res == S1_QUEUE);
+        if (qmask) {  // warp-aggregated append, tv.cu:190-197, tagged with the view
+            const int leader = __ffs(qmask) - 1;
+            unsigned long long b = 0;
+            if (lane == leader) b = atomicAdd(&p.counters[CR_CTR_NONTRIVIAL], (unsigned long long)__popc(qmask));
+            b = __shfl_sync(FULL, b, leader);
+            if (res == S1_QUEUE) {
+                const uint64_t q = b + __popc(qmask & ((1u << lane) - 1u));
+                if (q < p.ntCap) p.ntList[q] = e;
+                else atomicOr(&p.counters[CR_CTR_OVERFLOW], 1ull);
+            }
+        }
+        __syncwarp();
+    };
+    uint64_t pk = gw;
+    for (uint32_t part = 0; nItems; pk += nw) {
+        while (pk >= nItems && part < split) {
+            pk -= nItems;
+            ++part;
+        }
+        if (part >= split) break;
+        const unsigned long long partViews = (per < 64 ? (1ull << per) - 1ull : ~0ull) << (part * per);
+        const unsigned long long itemViews = __ldg(&p.itemViews[pk].views) & valid & partViews;
+        if (!itemViews) continue;
         const Item it = decode_item(p, (uint64_t)__ldg(&p.itemViews[pk].item));
-        const unsigned long long itemViews = __ldg(&p.itemViews[pk].views) & valid;
-        const unsigned long long itemStraddle = __ldg(&p.itemViews[pk].straddle) & itemViews;
         const CrSegment* sg = p.segments + it.seg;
         const uint32_t numTri = __ldg(&sg->numTriangles);
         const GeomRef geo = geom_of_t<PACKED>(sg);
-        const TileSrc ts = source(pk);
-        const bool tma = ts.src != nullptr;
-        const bool local = ts.local;
         const uint32_t tri0 = it.batch * CR_BATCH;
-        if (tma) {
-            const bool ok =
-                __all_sync(FULL, mbar_wait_bounded(&s_bar[w][slot], (parity & bit) ? 1u : 0u, p.waitTimeoutNs));
-            if (!ok) {
-                if (lane == 0) atomicOr(&p.counters[CR_CTR_TIMEOUT], 1ull);
-                break;
-            }
-            parity ^= bit;
-            pending &= ~bit;
-        }
-        const uint32_t* tile = s_idx[w][slot];
-        auto index_of = [&](uint32_t pos, int c) -> uint32_t {
-            if (local) return tile[(tile[CR_LOCAL_MAX + pos] >> (8 * c)) & 0xffu];
-            if (tma) return tile[3 * pos + c];
-            return geom_index(geo, 3ull * (tri0 + pos) + c);
-        };
-        bool act[S1_R];
-#pragma unroll
-        for (int r = 0; r < S1_R; ++r) act[r] = tri0 + r * 32 + lane < numTri;
         const uint32_t first = __ldg(&sg->firstInstance);
         const uint32_t ib = first + it.chunk * CR_INST_CHUNK;
         const uint32_t ie = min(ib + CR_INST_CHUNK, first + __ldg(&sg->instanceCount));
-        const uint32_t nLocal = local ? __ldg(ldg_ptr(&sg->localCounts) + it.batch) : 0u;
-        float itemBox[6] = {0, 0, 0, 0, 0, 0};
-        const float* boxes = ldg_ptr(&sg->itemBoxes);
-        const bool hasBox = boxes != nullptr;
-        if (hasBox)
-            for (int j = 0; j < 6; ++j) itemBox[j] = __ldg(boxes + 6ull * it.batch + j);
-
-        // survivors: view << 12 | instance slot << 8 | tile position
-        uint32_t* ring = s_ring[w];
-        uint32_t qh = 0, qt = 0;
-        auto drain = [&](bool all) {
-            while (qt - qh >= 32u || (all && qt > qh)) {
-                const uint32_t j = qh + lane;
-                int res = S1_CULL;
-                uint32_t tri = 0, inst = 0, view = 0;
-                if (j < qt) {
-                    const uint32_t e = ring[j & (S1_RING - 1)];
-                    const uint32_t tp = e & 0xffu;
-                    inst = ib + ((e >> 8) & 0xfu);
-                    view = e >> 12;
-                    tri = tri0 + tp;
-                    const uint64_t vi = (uint64_t)view * p.numInstances + inst;
-                    const Target tg = target_of(p, view);
-                    const V3 pa = pos_of(geo, index_of(tp, 0));
-                    const V3 pb = pos_of(geo, index_of(tp, 1));
-                    const V3 pc = pos_of(geo, index_of(tp, 2));
-                    res = stage1_triangle(tg, tg.fa, load_mat(p.world_view + 4ull * vi), __ldg(p.flips + vi), pa, pb,
-                                          pc, __ldg(&p.instances[inst].cum) - tg.idBase + tri);
-                }
-                qh = min(qh + 32u, qt);
-                const unsigned qmask = __ballot_sync(FULL, res == S1_QUEUE);
-                if (qmask) {  // warp-aggregated append, tv.cu:190-197, tagged with the view
-                    const int leader = __ffs(qmask) - 1;
-                    unsigned long long b = 0;
-                    if (lane == leader) b = atomicAdd(&p.counters[CR_CTR_NONTRIVIAL], (unsigned long long)__popc(qmask));
-                    b = __shfl_sync(FULL, b, leader);
-                    if (res == S1_QUEUE) {
-                        const uint64_t q = b + __popc(qmask & ((1u << lane) - 1u));
-                        if (q < p.ntCap)
-                            p.ntList[q] = ((uint64_t)view << CR_ENTRY_VIEW_SHIFT) | ((uint64_t)inst << 32) | tri;
-                        else atomicOr(&p.counters[CR_CTR_OVERFLOW], 1ull);
-                    }
-                }
-                __syncwarp();
-            }
-        };
+        // this lane's sub-box (lane & 7); read again for every four views (it
+        // stays in L1), so that it holds no registers over the full path
+        const float4* obbs = ldg_ptr(&sg->subObbs);
+        const float4* cones = ldg_ptr(&sg->subCones);
+        const uint64_t sub = (uint64_t)it.batch * (CR_BATCH / CR_SUB) + (lane & 7);
+        const bool hasSub = CR_SUB * (uint32_t)(lane & 7) < numTri - tri0;
+        V3 itemAbs = {};
+        if (obbs && hasSub) itemAbs = obb_max_abs(load_obb(obbs + CR_OBB_F4 * sub));
+        // the largest coordinates in the whole item, for quick_misses
+#pragma unroll
+        for (int d = 4; d >= 1; d >>= 1) {
+            itemAbs.x = fmaxf(itemAbs.x, __shfl_xor_sync(FULL, itemAbs.x, d));
+            itemAbs.y = fmaxf(itemAbs.y, __shfl_xor_sync(FULL, itemAbs.y, d));
+            itemAbs.z = fmaxf(itemAbs.z, __shfl_xor_sync(FULL, itemAbs.z, d));
+        }
         for (uint32_t inst = ib; inst < ie; ++inst) {
             unsigned long long todo = itemViews;
             while (todo) {
-                const uint32_t view = (uint32_t)(__ffsll((long long)todo) - 1);
-                todo &= todo - 1ull;
-                bool culledR[S1_R];
-                const Target tg = target_of(p, view);
-                const Mat M = load_mat(p.world_view + 4ull * ((uint64_t)view * p.numInstances + inst));
-                if (local && records_pay(M, tg, itemBox, hasBox)) {
-                    const float Wf = (float)tg.W, Hf = (float)tg.H;
-                    const float Wm1 = (float)(tg.W - 1), Hm1 = (float)(tg.H - 1);
-                    uint32_t* rec = s_rec[w];
-                    if ((itemStraddle >> view) & 1ull) {
-                        for (uint32_t v = lane; v < nLocal; v += 32)
-                            rec[v] = vertex_cell32<true>(M, pos_of(geo, tile[v]), tg.fa, tg.f, Wf, Hf, Wm1, Hm1);
-                    } else {  // the item's box is inside this view's frustum
-                        for (uint32_t v = lane; v < nLocal; v += 64) {
-                            const uint32_t v2 = v + 32;
-                            const uint32_t r0 = vertex_cell32<false>(M, pos_of(geo, tile[v]), tg.fa, tg.f, Wf, Hf, Wm1, Hm1);
-                            const uint32_t r1 =
-                                v2 < nLocal ? vertex_cell32<false>(M, pos_of(geo, tile[v2]), tg.fa, tg.f, Wf, Hf, Wm1, Hm1)
-                                            : 0u;
-                            rec[v] = r0;
-                            if (v2 < nLocal) rec[v2] = r1;
-                        }
-                    }
-                    __syncwarp();
-                    const uint32_t* cw = tile + CR_LOCAL_MAX;
+                // the next four views; view (lane >> 3) of them is this lane's
+                unsigned long long four = todo;
+                uint32_t mine = CR_MAX_VIEWS;
 #pragma unroll
-                    for (int r = 0; r < S1_R; ++r) {
-                        const uint32_t c = cw[r * 32 + lane];
-                        culledR[r] = !act[r] || cell32_culled(rec[c & 0xffu], rec[(c >> 8) & 0xffu], rec[(c >> 16) & 0xffu]);
-                    }
-                } else {
-                    // large on screen: every triangle through the full path
-                    // now, with this view's target and matrix for the warp
-                    const uint64_t vi = (uint64_t)view * p.numInstances + inst;
-                    const uint32_t flip = __ldg(p.flips + vi);
-                    const uint64_t cum = __ldg(&p.instances[inst].cum);
-                    const uint64_t entryHi = ((uint64_t)view << CR_ENTRY_VIEW_SHIFT) | ((uint64_t)inst << 32);
+                for (int i = 0; i < 4; ++i) {
+                    if (!todo) break;
+                    if ((lane >> 3) == i) mine = (uint32_t)(__ffsll((long long)todo) - 1);
+                    todo &= todo - 1ull;
+                }
+                four &= ~todo;
+                bool keep = mine < CR_MAX_VIEWS && hasSub;
+                if (keep && obbs) {
+                    const Target tg = target_of(p, mine);
+                    const uint64_t vi = (uint64_t)mine * p.numInstances + inst;
+                    const Obb ob = load_obb(obbs + CR_OBB_F4 * sub);
+                    Proof P = proof_rows(load_mat(p.world_view + 4ull * vi), obb_max_abs(ob));
+                    P.eye = __ldg(p.instProof + 2 * vi);
+                    P.det = __ldg(p.instProof + 2 * vi + 1);
+                    keep = !item_back_facing(P, __ldg(cones + 2 * sub), __ldg(cones + 2 * sub + 1), ob.c, obb_radius(ob)) &&
+                           !obb_misses_samples(P, tg.fa, tg.f, (float)tg.W, (float)tg.H, ob);
+                }
+                const uint32_t kept = __ballot_sync(FULL, keep);
 #pragma unroll 1
-                    for (int r = 0; r < S1_R; ++r) {
-                        const uint32_t tp = r * 32 + lane;
-                        int res = S1_CULL;
-                        if (act[r]) {
-                            const V3 pa = pos_of(geo, index_of(tp, 0));
-                            const V3 pb = pos_of(geo, index_of(tp, 1));
-                            const V3 pc = pos_of(geo, index_of(tp, 2));
-                            res = stage1_triangle(tg, tg.fa, M, flip, pa, pb, pc, cum - tg.idBase + tri0 + tp);
-                        }
-                        const unsigned qmask = __ballot_sync(FULL, res == S1_QUEUE);
-                        if (qmask) {
-                            const int leader = __ffs(qmask) - 1;
-                            unsigned long long b = 0;
-                            if (lane == leader)
-                                b = atomicAdd(&p.counters[CR_CTR_NONTRIVIAL], (unsigned long long)__popc(qmask));
-                            b = __shfl_sync(FULL, b, leader);
-                            if (res == S1_QUEUE) {
-                                const uint64_t q = b + __popc(qmask & ((1u << lane) - 1u));
-                                if (q < p.ntCap) p.ntList[q] = entryHi | (tri0 + tp);
-                                else atomicOr(&p.counters[CR_CTR_OVERFLOW], 1ull);
-                            }
-                        }
-                    }
-                    continue;
-                }
-#pragma unroll
-                for (int r = 0; r < S1_R; ++r) {
-                    const bool keep = !culledR[r];
-                    const unsigned m = __ballot_sync(FULL, keep);
-                    if (keep)
-                        ring[(qt + __popc(m & ((1u << lane) - 1u))) & (S1_RING - 1)] =
-                            (view << 12) | ((inst - ib) << 8) | (uint32_t)(r * 32 + lane);
-                    qt += __popc(m);
-                }
-                __syncwarp();
-                drain(false);
-            }
-        }
-        drain(true);
-
-        __syncwarp();
-        {  // refill this slot with the item STAGES ahead
-            const uint64_t nxt = pk + (uint64_t)STAGES * nw;
-            if (nxt < nItems) {
-                const TileSrc ns = source(nxt);
-                if (ns.src) {
-                    pending |= bit;
-                    if (lane == 0) {
-                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                        bulk_load(s_idx[w][slot], ns.src, ns.bytes, &s_bar[w][slot]);
+                for (int i = 0; i < 4 && four; ++i) {
+                    const uint32_t view = (uint32_t)(__ffsll((long long)four) - 1);
+                    four &= four - 1ull;
+                    uint32_t rest = (kept >> (8 * i)) & 0xffu;
+                    if (!rest) continue;
+                    const Target tg = target_of(p, view);
+                    const Quick Q = make_quick(
+                        proof_rows(load_mat(p.world_view + 4ull * ((uint64_t)view * p.numInstances + inst)), itemAbs),
+                        tg.fa, tg.f, (float)tg.W, (float)tg.H);
+                    const uint64_t entry = ((uint64_t)view << CR_ENTRY_VIEW_SHIFT) | ((uint64_t)inst << 32) | tri0;
+                    while (rest) {
+                        const uint32_t b0 = (uint32_t)__ffs(rest) - 1;
+                        rest &= rest - 1;
+                        const uint32_t b1 = rest ? (uint32_t)__ffs(rest) - 1 : 8u;
+                        rest &= rest - 1;
+                        const uint32_t tp = CR_SUB * (lane < 16 ? b0 : b1) + (uint32_t)(lane & 15);
+                        bool left = tp < CR_BATCH && tri0 + tp < numTri;
+                        if (!COARSE && left && obbs)
+                            left = !quick_misses(Q, pos_of(geo, geom_index(geo, 3ull * (tri0 + tp) + 0)),
+                                                 pos_of(geo, geom_index(geo, 3ull * (tri0 + tp) + 1)),
+                                                 pos_of(geo, geom_index(geo, 3ull * (tri0 + tp) + 2)));
+                        const unsigned m = __ballot_sync(FULL, left);
+                        if (left) ring[(qt + __popc(m & ((1u << lane) - 1u))) & (S1_RING - 1)] = entry + tp;
+                        qt += __popc(m);
+                        __syncwarp();
+                        if (qt - qh >= 32u) drain();
                     }
                 }
             }
         }
     }
-    for (int s = 0; s < STAGES; ++s)
-        if (pending & (1u << s)) (void)mbar_wait_bounded(&s_bar[w][s], (parity >> s) & 1u, p.waitTimeoutNs);
+    if (qt > qh) drain();
+}
+
+// The back-face proof's data of every (view, instance): proof_data of api.cpp, a
+// thread each (64 views of thousands of instances would take the host longer
+// than the frame takes).  Two float4 per entry: eye and |eye|; |det|, |R|_F, the largest
+// row sum of |R| and |t|.
+__global__ void __launch_bounds__(256) k_view_proofs(const float4* wv, uint32_t n, float4* out) {
+    const uint32_t k = blockIdx.x * 256 + threadIdx.x;
+    if (k >= n) return;
+    const Mat M = load_mat(wv + 4ull * k);
+    const double r00 = M.c0.x, r01 = M.c1.x, r02 = M.c2.x, r10 = M.c0.y, r11 = M.c1.y, r12 = M.c2.y, r20 = M.c0.z,
+                 r21 = M.c1.z, r22 = M.c2.z, t0 = M.c3.x, t1 = M.c3.y, t2 = M.c3.z;
+    const double a00 = r11 * r22 - r12 * r21, a01 = r02 * r21 - r01 * r22, a02 = r01 * r12 - r02 * r11,
+                 a10 = r12 * r20 - r10 * r22, a11 = r00 * r22 - r02 * r20, a12 = r02 * r10 - r00 * r12,
+                 a20 = r10 * r21 - r11 * r20, a21 = r01 * r20 - r00 * r21, a22 = r00 * r11 - r01 * r10;
+    const double det = r00 * a00 + r01 * a10 + r02 * a20;
+    const double had = (fabs(r00) + fabs(r10) + fabs(r20)) * (fabs(r01) + fabs(r11) + fabs(r21)) *
+                       (fabs(r02) + fabs(r12) + fabs(r22));
+    const double frob = r00 * r00 + r01 * r01 + r02 * r02 + r10 * r10 + r11 * r11 + r12 * r12 + r20 * r20 + r21 * r21 +
+                        r22 * r22;
+    const double row = fmax(fabs(r00) + fabs(r01) + fabs(r02),
+                            fmax(fabs(r10) + fabs(r11) + fabs(r12), fabs(r20) + fabs(r21) + fabs(r22)));
+    const double tAbs = fmax(fabs(t0), fmax(fabs(t1), fabs(t2)));
+    const double e0 = -(a00 * t0 + a01 * t1 + a02 * t2) / det, e1 = -(a10 * t0 + a11 * t1 + a12 * t2) / det,
+                 e2 = -(a20 * t0 + a21 * t1 + a22 * t2) / det;
+    const bool ok = isfinite(det) && fabs(det) > 1e-4 * had && isfinite(e0) && isfinite(e1) && isfinite(e2) &&
+                    isfinite(tAbs) && isfinite(frob);
+    const double up = 1.0 + 1e-6;  // above the rounding to float
+    out[2ull * k] = ok ? make_float4((float)e0, (float)e1, (float)e2, (float)(sqrt(e0 * e0 + e1 * e1 + e2 * e2) * up))
+                       : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    out[2ull * k + 1] = make_float4(ok ? (float)(fabs(det) * (1.0 - 1e-6)) : 0.0f, (float)(sqrt(frob) * up),
+                                    (float)(row * up), (float)(tAbs * up));
 }
 
 // Clears every view's visbuffer (resolve.cu:213-232); blockIdx.y is the view.
@@ -870,6 +812,8 @@ __global__ void __launch_bounds__(256) k_clear_views(const CrView* views, unsign
 }  // namespace
 
 constexpr int VS1_WARPS_MAX = 8;
+// resident blocks per SM of k_stage1_views_boxes
+constexpr int V1_MINB = 3;
 
 int cr_query_batch_shape(int device, CrBatchShape* out) {
     int sms = 0;
@@ -922,11 +866,20 @@ int cr_launch_stage1_views(const CrFrameParams& p, const CrBatchShape& s, void* 
     if (blocks > (uint64_t)s.stage1Blocks) blocks = (uint64_t)s.stage1Blocks;
     const unsigned b = (unsigned)blocks;
     cudaStream_t st = (cudaStream_t)stream;
-    if (p.cellMode == CR_REC_BOXES && p.itemViews) {  // vertex lists (no vertex pass)
-        uint64_t lb = (p.numItems + 7) / 8;
-        if (lb > (uint64_t)s.numSMs * 3) lb = (uint64_t)s.numSMs * 3;
-        if (p.anyPacked) k_stage1_views_lists<8, 3, true><<<(unsigned)lb, 256, 0, st>>>(p);
-        else k_stage1_views_lists<8, 3, false><<<(unsigned)lb, 256, 0, st>>>(p);
+    if (p.cellMode == CR_REC_BOXES && p.itemViews) {  // oriented sub-boxes (no vertex pass)
+        const uint32_t pairs = p.numViews * p.numInstances;
+        k_view_proofs<<<(pairs + 255) / 256, 256, 0, st>>>(p.world_view, pairs, p.viewProof);
+        uint64_t lb = (p.numItems * ((p.numViews + 3) / 4) + 7) / 8;
+        if (lb > (uint64_t)s.numSMs * V1_MINB) lb = (uint64_t)s.numSMs * V1_MINB;
+        const unsigned g = (unsigned)lb;
+        if (p.coopRaster) {
+            if (p.anyPacked) k_stage1_views_boxes<8, V1_MINB, true, true><<<g, 256, 0, st>>>(p);
+            else k_stage1_views_boxes<8, V1_MINB, false, true><<<g, 256, 0, st>>>(p);
+        } else if (p.anyPacked) {
+            k_stage1_views_boxes<8, V1_MINB, true, false><<<g, 256, 0, st>>>(p);
+        } else {
+            k_stage1_views_boxes<8, V1_MINB, false, false><<<g, 256, 0, st>>>(p);
+        }
         return cudaGetLastError() == cudaSuccess ? 0 : -1;
     }
     // the register-capped variants let more blocks share an SM

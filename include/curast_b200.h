@@ -83,11 +83,13 @@ typedef struct cr_config {
  * off-screen, CELLS (8 bytes: also the exact pixel cell) additionally culls
  * sub-pixel triangles that miss every sample.  BOXES writes no records to
  * device memory: per instance it proves from the mesh's precomputed boxes
- * that whole 128-triangle groups miss every sample, and culls the rest from
- * cell records of each group's distinct vertices kept in shared memory
- * (per-group vertex lists, built on first use) -- suited to many instances that are small on screen.  AUTO picks
- * BOXES for frames that draw some mesh more than once, CELLS for other frames
- * with more than one instance, else OUTCODES. */
+ * that whole 128-triangle groups, then 16-triangle ones (oriented boxes built
+ * on first use) and then single triangles miss every sample or face away --
+ * suited to triangles that are small on screen.  AUTO picks
+ * BOXES for frames that draw some mesh more than once and for frames of mostly
+ * sub-pixel triangles (given memory for the boxes), CELLS for other frames
+ * with more than one instance, else OUTCODES; and small frames take every
+ * triangle straight through the per-triangle path. */
 #define CR_CULL_AUTO 0u
 #define CR_CULL_OUTCODES 1u
 #define CR_CULL_CELLS 2u
@@ -202,7 +204,9 @@ typedef struct cr_frame_stats {
     float reserved;
     /* hierarchical culling: stage-1 work items (128 triangles x an instance
      * chunk) and vertex-pass chunks (1024 vertices of an instance), in all
-     * and after the per-view box tests */
+     * and after the per-view box tests.  Small frames take every triangle
+     * straight through stage 1's per-triangle path: all of them count as
+     * drawn, evaluated and survivors */
     uint64_t work_items;
     uint64_t work_items_drawn;
     uint64_t vertex_chunks;

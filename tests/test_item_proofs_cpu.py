@@ -77,8 +77,8 @@ def axis_misses(Fa, row, S, Sz, b, D0, gz, iD, W, margin):
     for j in range(3):
         e = e + np.abs(fma(r0, gz[j], Fa * dot_dir(row, b[1][j])))
     ar = np.abs(r0)
-    h = F(0.5) * W * ((e + margin * (F(96) * U * (np.abs(Fa) * S + (ar + F(1)) * Sz) + F(1e-30))) * iD) + \
-        margin * F(32) * U * W * (ar + F(2))
+    h = F(0.5) * W * ((e + margin * (F(28) * U * (np.abs(Fa) * S + (ar + F(1e-3)) * Sz) + F(1e-30))) * iD) + \
+        margin * F(6) * U * W * (ar + F(1))
     s0 = W * (F(0.5) * r0 + F(0.5)) - F(0.5)
     lo, hi = s0 - h, s0 + h
     k = np.floor(lo)
@@ -89,7 +89,7 @@ def proof_misses(M, fa, f, W, H, b, S, margin=F(1)):
     rows = M.reshape(4, 4).T.astype(F)
     gz = [dot_dir(rows[2], a) for a in b[1]]
     D0 = -dot_pos(rows[2], b[0])
-    Dmin = (D0 - (np.abs(gz[0]) + np.abs(gz[1]) + np.abs(gz[2]))) - margin * (F(64) * U * S[2] + F(1e-30))
+    Dmin = (D0 - (np.abs(gz[0]) + np.abs(gz[1]) + np.abs(gz[2]))) - margin * (F(32) * U * S[2] + F(1e-30))
     if not (Dmin > F(1e-30) and Dmin < F(1e30)):
         return False
     iD = F(1) / Dmin * F(1.00000095367431640625)
@@ -163,6 +163,67 @@ def test_sample_miss_proof_is_sound():
 def test_sample_miss_margins_matter():
     claimed, wrong = clusters(np.random.default_rng(5), 6000, True)
     assert claimed > 800 and wrong > 0, (claimed, wrong)
+
+
+def proof_quick(M, fa, f, W, H, tri, S, margin=F(1)):
+    """raster_core.cuh make_quick and quick_misses (the reciprocal within 2 ulp either way)."""
+    rows = M.reshape(4, 4).T.astype(F)
+    kx, ky = F(0.5) * W * fa, F(0.5) * H * f
+    rx, ry = (rows[0] * kx).astype(F), (rows[1] * ky).astype(F)
+    d = np.array([-dot_pos(rows[2], p) for p in tri], F)
+    if not (d > margin * (F(16) * U * S[2] + F(1e-30))).all():
+        return False
+    r = np.array([F(1) / v for v in d], F)
+    for _ in range(2):
+        r = np.nextafter(r, F(np.inf) * np.where(np.arange(3) % 2, F(1), F(-1)))
+    iD = r.max() * F(1.00000095367431640625)
+    for rr, c, n, Fa, Sa in ((rx, F(0.5) * W - F(0.5), W, fa, S[0]), (ry, F(0.5) * H - F(0.5), H, f, S[1])):
+        x = [fma(dot_pos(rr, p), r[i], c) for i, p in enumerate(tri)]
+        m = margin * fma(F(6) * U * n * (np.abs(Fa) * Sa + S[2]), iD, F(8) * U * n)
+        lo, hi = min(x) - m, max(x) + m
+        k = np.floor(lo)
+        if (k >= 0 and hi < k + F(1)) or hi < F(-0.5) or lo > F(2) * c + F(0.5):
+            return True
+    return False
+
+
+@pytest.mark.parametrize("margin", [1, 0])
+def test_quick_miss_is_sound(margin):
+    """Triangles a fraction of a pixel wide whose edge ends next to a sample line."""
+    rng = np.random.default_rng(9)
+    W, H = F(1920), F(1080)
+    f = F(1.7320508)
+    fa = F(f / F(W / H))
+    claimed = wrong = 0
+    for _ in range(6000):
+        size = 10.0 ** rng.uniform(-5, 0)
+        dist = size * 10.0 ** rng.uniform(3.1, 5.0)
+        Vr = np.linalg.qr(rng.normal(size=(3, 3)))[0]
+        p = (rng.normal(size=(3, 3)) * size + rng.uniform(-1, 1, 3) * rng.choice([0.0, 1.0, 100.0])).astype(F)
+        v = p.astype(np.float64) @ Vr.T
+        t = np.array([0.0, 0.0, -dist]) - v.mean(0)
+        v2 = v + t
+        sx = (fa * v2[:, 0] / -v2[:, 2] * 0.5 + 0.5) * W - 0.5
+        sy = (f * v2[:, 1] / -v2[:, 2] * 0.5 + 0.5) * H - 0.5
+        gap = rng.choice([0.0, 3e-5, 1e-4, 3e-3, 0.01, 0.1])
+        if rng.random() < 0.3:  # just beyond the left or right side
+            sxt = -0.5 - gap - sx.max() if rng.random() < 0.5 else 1919.5 + gap - sx.min()
+        else:
+            sxt = rng.integers(1, 1918) + gap - sx.min()
+        t[0] += sxt / W * 2 / float(fa) * dist
+        t[1] += (rng.integers(1, 1078) - sy.mean()) / H * 2 / float(f) * dist
+        M = np.eye(4)
+        M[:3, :3], M[:3, 3] = Vr, t
+        M = M.astype(F).T.reshape(16)
+        S = instance_proof(M, p.min(0), p.max(0))[-1]
+        if proof_quick(M, fa, f, W, H, p, S, F(margin)):
+            claimed += 1
+            x, y, d = stage1_screen(M, p, fa, f, W, H)
+            q = xform(M, p)
+            ndc = (fa * q[:, 0]) / d
+            wrong += not ((d > 0).all() and (missed(x, y, W, H) or (ndc > 1).all() or (ndc < -1).all()))
+    assert claimed > 800
+    assert (wrong == 0) if margin else (wrong > 0), (claimed, wrong)
 
 
 @pytest.mark.parametrize("drop", [False, True])
