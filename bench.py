@@ -368,11 +368,12 @@ def plain_algorithmic_bytes(wl, fstats, T):
     record of each vertex those triangles use once (counted as one per two
     triangles, as in a closed mesh, and at most the records written), and
     writes and reads 8 B per survivor of the records.
-    Frames that draw a mesh more than once cull from box proofs and per-item
-    vertex lists (no per-vertex records in device memory).  Returns (bytes per
-    stage, triangles in drawn items, vertices evaluated)."""
-    mids = [m for m, _ in wl["instances"]]
-    direct = len(set(mids)) < len(mids)
+    Frames without a vertex pass (no chunks: some mesh drawn more than once, or
+    mostly sub-pixel triangles) cull from oriented boxes: stage 1 reads the
+    eight sub-boxes and cones of each drawn item, and the list entry, indices and
+    positions of each survivor (of the triangles it tests on the way it is not
+    told the number).  Small frames take every triangle straight through stage
+    1.  Returns (bytes per stage, triangles in drawn items, vertices evaluated)."""
     rec = 4 if max(wl["W"], wl["H"]) <= 4096 else 8
     items, items_drawn = int(fstats.work_items), int(fstats.work_items_drawn)
     chunks, chunks_eval = int(fstats.vertex_chunks), int(fstats.vertex_chunks_evaluated)
@@ -380,14 +381,15 @@ def plain_algorithmic_bytes(wl, fstats, T):
     surv = int(getattr(fstats, "stage1_survivors", 0))
     nV_inst = sum(wl["meshes"][m][0].shape[0] for m, _ in wl["instances"])
     stamps = 56 * items_drawn if slices_eval else 0
-    if direct:
+    if items and not chunks:
         # frame cull: one 24-byte item box per item (the instance matrices
-        # stay in L1) and 8 B per listed item; stage 1: the 1408-byte vertex
-        # list block of each listed item and the positions of its distinct
-        # vertices (at most 128 x 12 B for these meshes)
+        # stay in L1) and 8 B per listed item; a sub-box is 48 B, a cone 32
         v_eval, tri_drawn = 0, min(T, items_drawn * 128)
-        algo = {"vertex": 24 * items + 8 * items_drawn,
-                "stage1": (1408 + 12 * 128) * items_drawn, "boxes": True}
+        algo = {"vertex": 24 * items + 8 * items_drawn, "stage1": 8 * (48 + 32) * items_drawn + (16 + 48) * surv,
+                "boxes": True}
+    elif chunks and surv >= T:
+        v_eval, tri_drawn = nV_inst, T
+        algo = {"vertex": 0, "stage1": 12 * T + 12 * nV_inst, "straight": True}
     elif chunks:
         # the vertex pass evaluates the slices (128 vertices) of its listed
         # chunks that hold a vertex of a drawn item
@@ -398,7 +400,9 @@ def plain_algorithmic_bytes(wl, fstats, T):
     else:
         v_eval, tri_drawn = nV_inst, T
         algo = {"vertex": (12 + rec) * nV_inst, "stage1": 12 * T + rec * min(nV_inst, T // 2) + 16 * surv}
-    if wl.get("compressed"):
+    if wl.get("compressed") and algo.get("straight"):
+        algo["stage1"] = 3 * wl["compressed"][0].bits / 8.0 * T + 6 * nV_inst
+    elif wl.get("compressed"):
         # compressed meshes: 6-byte positions, 3 x bits / 8 bytes of indices per triangle
         ib = 3 * wl["compressed"][0].bits / 8.0
         algo = {"vertex": 24 * (chunks + items) + (6 + rec) * v_eval + 8 * items_drawn + stamps,
@@ -586,8 +590,9 @@ def run_ours(args, rank, world, local):
                 "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": 4 * W * H,
                 "mode": "steps back to back, each image read back while the next step renders",
                 "latency_ms_per_step": e2e_latency},
-        "roofline": {"kernel": {"vertex": "k_cull_groups + k_cull + k_stamp + k_vertex",
-                                "stage1": "k_stage1" if algo.get("boxes") else "k_s1cull + k_s1raster"}.get(
+        "roofline": {"kernel": {"vertex": "k_cull_groups + k_cull" + ("" if algo.get("boxes") else " + k_stamp + k_vertex"),
+                                "stage1": "k_stage1 + k_s1raster" if algo.get("boxes") else
+                                   "k_s1direct or k_s1raster" if algo.get("straight") else "k_s1cull + k_s1raster"}.get(
                                     rk, f"k_{rk}"), "bound": "hbm",
                      "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_kind": peak_kind,
@@ -596,7 +601,7 @@ def run_ours(args, rank, world, local):
         # clear, the two frame-cull kernels, the vertex pass (record-culled
         # frames), stage 1 (two kernels when record-culled), stages 2 and 3,
         # the resolve
-        "gpu_launches": (7 if algo.get("boxes") else 10) * args.steps,
+        "gpu_launches": (8 if algo.get("boxes") else 5 if algo.get("straight") else 10) * args.steps,
         "clocks": clk,
     }
     if parity is not None:
@@ -730,8 +735,9 @@ def sub_plain(args, wl, ctx, handles, with_parity):
                     "vertex_slices_evaluated": int(getattr(fstats, "vertex_slices_evaluated", 0)),
                     "stage1_survivors": int(fstats.stage1_survivors), "nontrivial": int(fstats.nontrivial),
                     "huge_tiles": int(fstats.huge_tiles)},
-           "roofline": {"kernel": {"vertex": "k_cull_groups + k_cull + k_stamp + k_vertex",
-                                   "stage1": "k_stage1" if algo.get("boxes") else "k_s1cull + k_s1raster"}.get(
+           "roofline": {"kernel": {"vertex": "k_cull_groups + k_cull" + ("" if algo.get("boxes") else " + k_stamp + k_vertex"),
+                                   "stage1": "k_stage1 + k_s1raster" if algo.get("boxes") else
+                                   "k_s1direct or k_s1raster" if algo.get("straight") else "k_s1cull + k_s1raster"}.get(
                                        rk, f"k_{rk}"),
                         "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                         "peak_kind": peak_kind, "algorithmic_bytes": algo[rk], "kernel_ms": stage_ms[rk],
@@ -1192,11 +1198,12 @@ def run_batched(args, rank, world, local, wl):
         ctx.close()
         return None
     peak, peak_kind = load_peaks()
-    # algorithmic bytes: vertex pass 12 B position read + 48 B record write per
-    # vertex; stage 1 12 B index tile per triangle + each 48 B record once;
+    # algorithmic bytes: the frame cull (timed as the vertex stage) reads a 24 B
+    # box per item and per vertex chunk; stage 1 indices, positions, sub-boxes and
+    # cones (80 B per 16 triangles) once for all views;
     # whole frame 12T + 12V (geometry once for all views) + 28 B per pixel of
     # every view (visbuffer clear and write-back, resolve read + RGBA8 write)
-    algo = {"vertex": 60 * V, "stage1": 12 * T + 48 * V}
+    algo = {"vertex": 24 * (T // 128 + V // 1024), "stage1": 12 * T + 12 * V + 5 * T}
     dominant = max(("vertex", "stage1", "stage2", "stage3", "resolve", "clear"), key=lambda s: stage_ms[s])
     rk = "stage1" if dominant not in algo else dominant
     t_k = stage_ms[rk]
