@@ -1206,12 +1206,13 @@ cr_status cr_render(cr_context* ctx, const cr_instance* instances, uint32_t coun
 }  // extern "C"
 
 // Frames of at most this many triangles take every triangle straight through
-// the per-triangle path (CrFrameParams::direct).  Below it the five kernels that
-// decide which triangles not to draw cost more than drawing them: planets of
-// sub-pixel triangles at 1280x720, culled / direct: 200K 95.7 / 71.3 us, 1M 110 / 85, 4M
-// 119 / 111, 8M 126 / 159 (seen whole: 61 / 35, 75 / 48, 93 / 87, 113 / 146); instances, 30 x
-// 1,000 136 / 28, 300 x 5,000 172 / 79, 100 x 50,000 91 / 101, 10 x 1M 62 / 154.
-static constexpr uint64_t kDirectLimit = 4ull << 20;
+// the per-triangle path (CrFrameParams::direct).  Below it the kernels that decide
+// which triangles not to draw mostly cost more than drawing them.  Direct / culled from
+// boxes, whole frame in us: planet from its surface at 1280x720 1.1M 87 / 109, 1.6M
+// 96 / 109, 2.2M 168 / 106, 4.1M 185 / 104; seen whole 1.1M 50 / 75, 2.2M 84 / 71, 4.1M
+// 114 / 75; 10 x 300K instances 50 / 51, 100 x 20K 48 / 76.  (Heightfields of needles gain from
+// it further up: 2.1M at 391x220 164 / 199, 4M 289 / 336; by records 228, 364.)
+static constexpr uint64_t kDirectLimit = 2ull << 20;
 
 cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_t count, const uint64_t* firstIds,
                           const cr_camera* cam, uint64_t d_visbuffer, uint64_t d_rgba, uint64_t d_colorbuffer,

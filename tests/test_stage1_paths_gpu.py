@@ -80,7 +80,7 @@ def test_small_frames_match_every_record_mode(gpu, kind, sizes):
     assert all(s.stage1_survivors == s.triangles for _, _, s in got)
 
 
-@pytest.mark.parametrize("tris,orbit,W,H", [(4_300_000, False, 319, 181), (6_000_001, True, 640, 360)])
+@pytest.mark.parametrize("tris,orbit,W,H", [(2_300_000, False, 319, 181), (6_000_001, True, 640, 360)])
 def test_large_sub_pixel_frames_are_box_culled(gpu, tris, orbit, W, H):
     pos, idx, col = keep = scenes.planet(tris, seed=3, device="cuda", width=W, height=H)
     cams = [(*(scenes.planet_orbit_camera(W, H) if o else scenes.planet_camera(W, H)), W, H) for o in (orbit, not orbit)]
