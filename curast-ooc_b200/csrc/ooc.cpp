@@ -370,32 +370,20 @@ cr_status cr_ooc_render(cr_ooc* o, const cr_camera* cam, uint64_t d_visbuffer, u
     }
     st.visible_nodes = (uint32_t)order.size();
     st.visible_triangles = sum;
-    // passes of at most numSlots nodes, each in draw order.  A frame of several
-    // starts with the nodes that are resident already (the order of the passes is
-    // free: ids are fixed and the visbuffer is a minimum), so that no pass
-    // evicts what a later one would find.
+    // Passes of at most numSlots nodes: runs of the draw order, the same whatever
+    // is resident.  (What a pass asks of the work queues then does not depend
+    // on the frames before: queues that held the frame once hold it again.)
+    std::vector<std::vector<uint32_t>> passes;  // places in `order`
+    for (size_t a = 0; a < order.size(); a += o->numSlots) {
+        passes.emplace_back(std::min(order.size() - a, (size_t)o->numSlots));
+        std::iota(passes.back().begin(), passes.back().end(), (uint32_t)a);
+    }
+    if (passes.empty()) passes.emplace_back();
+    const bool multi = passes.size() > 1;
     // Stage 2 keeps 32 bits of an id (tv.cu:414), so past 2^32 triangles a pixel
     // may name a node of an earlier pass: such frames resolve after every
     // raster pass, node groups in draw order.
-    const bool multi = order.size() > o->numSlots;
     const bool wide = sum > (1ull << 32);
-    std::vector<std::vector<uint32_t>> passes;  // places in `order`
-    if (multi && !wide) {
-        std::vector<uint32_t> first, rest;
-        for (uint32_t k = 0; k < (uint32_t)order.size(); k++) (o->nodes[order[k]].slot >= 0 ? first : rest).push_back(k);
-        const size_t fill = std::min(rest.size(), (size_t)o->numSlots - first.size());
-        first.insert(first.end(), rest.begin(), rest.begin() + fill);
-        std::sort(first.begin(), first.end());
-        passes.push_back(std::move(first));
-        for (size_t a = fill; a < rest.size(); a += o->numSlots)
-            passes.emplace_back(rest.begin() + a, rest.begin() + std::min(rest.size(), a + o->numSlots));
-    } else {
-        for (size_t a = 0; a < order.size(); a += o->numSlots) {
-            passes.emplace_back(std::min(order.size() - a, (size_t)o->numSlots));
-            std::iota(passes.back().begin(), passes.back().end(), (uint32_t)a);
-        }
-        if (passes.empty()) passes.emplace_back();
-    }
     st.passes = (uint32_t)passes.size();
     const bool resolve = !(flags & CR_RENDER_NO_RESOLVE);
     auto run_pass = [&](size_t p, uint32_t passFlags, uint64_t idLo, uint64_t idHi, ResolvePart part) -> cr_status {
@@ -421,13 +409,22 @@ cr_status cr_ooc_render(cr_ooc* o, const cr_camera* cam, uint64_t d_visbuffer, u
     // the pixels that its own nodes hold by then: a pixel keeps its last
     // winner's pass's colour, and that winner's geometry is resident in that
     // pass, where a resolve after all passes would upload the evicted nodes
-    // again.
+    // again.  The passes' order is free then (ids are fixed and the visbuffer is
+    // a minimum): they run by the number of nodes to upload, so that what the
+    // frame before left resident is drawn before it is evicted.
     const uint32_t keep = flags & (CR_RENDER_SYNC | CR_RENDER_TIMING);
     const bool late = multi && wide;
-    for (size_t p = 0; p < passes.size(); p++) {
-        uint32_t f = keep | (p > 0 ? CR_RENDER_NO_CLEAR : 0u) | ((late || !resolve) ? CR_RENDER_NO_RESOLVE : 0u);
-        s = run_pass(p, f, 0, ~0ull,
-                     !multi || late ? ResolvePart::Whole : p == 0 ? ResolvePart::First : ResolvePart::Later);
+    std::vector<uint32_t> turn(passes.size()), missing(passes.size(), 0);
+    std::iota(turn.begin(), turn.end(), 0u);
+    if (multi && !late) {
+        for (size_t p = 0; p < passes.size(); p++)
+            for (uint32_t place : passes[p]) missing[p] += o->nodes[order[place]].slot < 0 ? 1u : 0u;
+        std::stable_sort(turn.begin(), turn.end(), [&](uint32_t a, uint32_t b) { return missing[a] < missing[b]; });
+    }
+    for (size_t k = 0; k < turn.size(); k++) {
+        uint32_t f = keep | (k > 0 ? CR_RENDER_NO_CLEAR : 0u) | ((late || !resolve) ? CR_RENDER_NO_RESOLVE : 0u);
+        s = run_pass(turn[k], f, 0, ~0ull,
+                     !multi || late ? ResolvePart::Whole : k == 0 ? ResolvePart::First : ResolvePart::Later);
         if (s) return s;
     }
     if (late && resolve) {  // last group first (it is still resident)

@@ -1,0 +1,85 @@
+"""Out-of-core frames of several passes: what a frame draws does not depend on
+what the frames before it left in the cache."""
+import numpy as np
+import pytest
+
+import pycurast as pc
+import scenes
+
+pytestmark = pytest.mark.gpu
+
+QUADS, NODES, SLOTS = 16, 20, 10
+
+
+def grid(x0, x1, y0, y1, z):
+    """QUADS x QUADS quads in the plane z, facing the camera at the origin."""
+    n = QUADS + 1
+    x, y = np.meshgrid(np.linspace(x0, x1, n), np.linspace(y0, y1, n))
+    pos = np.stack([x, y, np.full_like(x, z)], -1).reshape(-1, 3).astype(np.float32)
+    a = (np.arange(QUADS)[:, None] * n + np.arange(QUADS)[None]).reshape(-1)
+    idx = np.concatenate([np.stack([a, a + 1, a + n], -1), np.stack([a + 1, a + n + 1, a + n], -1)])
+    return pos, idx.astype(np.uint32)
+
+
+def node_set():
+    """Nodes of equal size; the even ones fill the middle of the screen (every
+    triangle goes to stage 2), the odd ones are specks near its edges."""
+    import torch
+
+    rng = np.random.default_rng(8)
+    nodes, keep = [], []
+    for k in range(NODES):
+        if k % 2 == 0:
+            pos, idx = grid(-0.5, 0.5, -0.4, 0.4, -2.0 - 0.01 * k)
+        else:
+            y = -0.9 + 0.09 * k
+            pos, idx = grid(1.2, 1.22, y, y + 0.02, -2.0)
+        col = rng.integers(0, 2**32, len(pos), np.uint64).astype(np.uint32)
+        t = [torch.from_numpy(a).pin_memory() for a in (pos, idx.view(np.int32), col.view(np.int32))]
+        keep.append(t)
+        nodes.append((t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), len(pos), len(idx), pos.min(0), pos.max(0),
+                      scenes.identity()))
+    return nodes, keep
+
+
+def slot_bytes():
+    nv, nt = (QUADS + 1) ** 2, 2 * QUADS * QUADS
+    return sum(-(-b // 256) * 256 for b in (12 * nv, 12 * nt, 4 * nv))
+
+
+def camera(fov, W, H):
+    return pc.make_camera(scenes.identity(), scenes.perspective(fov, W / H, 0.01, 100.0), W, H)
+
+
+def frame(scene, cam, flags, stream=0):
+    import torch
+
+    n = cam.width * cam.height
+    vis = torch.full((n,), 7, dtype=torch.int64, device="cuda")
+    rgba = torch.full((n,), 7, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    st = scene.render(cam, vis.data_ptr(), rgba.data_ptr(), flags=flags, stream=stream)
+    torch.cuda.synchronize()
+    return vis.cpu().numpy(), rgba.cpu().numpy(), st
+
+
+def test_queues_that_held_a_frame_hold_it_again(gpu):
+    """Rendered once with SYNC, which sizes the queues for the frame's passes, then
+    without: between two frames of the whole scene another brings the nodes
+    that fill stage 2's queue into the cache together."""
+    nodes, keep = node_set()
+    whole, middle = camera(60.0, 1024, 768), camera(20.0, 64, 48)
+    with pc.Context() as ctx, pc.OocScene(ctx, nodes, 1 << 30) as sc:
+        want = [frame(sc, cam, pc.CR_RENDER_SYNC) for cam in (whole, middle)]
+        assert want[0][2].passes == 1 and want[1][2].visible_nodes == NODES // 2
+    with pc.Context(max_nontrivial=1024) as ctx, pc.OocScene(ctx, nodes, SLOTS * slot_bytes()) as sc:
+        for flags in (pc.CR_RENDER_SYNC, 0, 0, 0):
+            for k, cam in enumerate((whole, middle)):
+                vis, rgba, st = frame(sc, cam, flags)
+                assert st.passes == 2 - k
+                assert ctx.stats()[0] == pc.CR_OK
+                assert np.array_equal(vis, want[k][0]) and np.array_equal(rgba, want[k][1]), (flags, k)
+        # the same view again and again uploads no more than the cache cannot hold
+        for _ in range(3):
+            st = frame(sc, whole, 0)[2]
+        assert st.uploaded_nodes == NODES - SLOTS
