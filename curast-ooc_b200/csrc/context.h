@@ -212,6 +212,10 @@ cr_status assemble(cr_context* ctx, const cr_instance* instances, uint32_t count
 
 // Internal render flag: resolve only (the frame's raster passes are done).
 constexpr uint32_t kRenderResolveOnly = 1u << 31;
+// Internal render flag: a further pass of an asynchronous frame of several.  The
+// overflow and timeout words of the passes before stay, so that cr_sync reports
+// those of any pass.
+constexpr uint32_t kRenderNextPass = 1u << 30;
 
 // What the resolve of one pass of a multi-pass frame writes: every pixel, or
 // those whose triangle belongs to the pass's own instances (and, in the first

@@ -413,6 +413,9 @@ cr_status cr_ooc_render(cr_ooc* o, const cr_camera* cam, uint64_t d_visbuffer, u
     // a minimum): they run by the number of nodes to upload, so that what the
     // frame before left resident is drawn before it is evicted.
     const uint32_t keep = flags & (CR_RENDER_SYNC | CR_RENDER_TIMING);
+    // an asynchronous frame's overflow is that of all its passes (a SYNC one
+    // grows the queues pass by pass)
+    const uint32_t next = (flags & CR_RENDER_SYNC) ? 0u : kRenderNextPass;
     const bool late = multi && wide;
     std::vector<uint32_t> turn(passes.size()), missing(passes.size(), 0);
     std::iota(turn.begin(), turn.end(), 0u);
@@ -422,7 +425,7 @@ cr_status cr_ooc_render(cr_ooc* o, const cr_camera* cam, uint64_t d_visbuffer, u
         std::stable_sort(turn.begin(), turn.end(), [&](uint32_t a, uint32_t b) { return missing[a] < missing[b]; });
     }
     for (size_t k = 0; k < turn.size(); k++) {
-        uint32_t f = keep | (k > 0 ? CR_RENDER_NO_CLEAR : 0u) | ((late || !resolve) ? CR_RENDER_NO_RESOLVE : 0u);
+        uint32_t f = keep | (k > 0 ? CR_RENDER_NO_CLEAR | next : 0u) | ((late || !resolve) ? CR_RENDER_NO_RESOLVE : 0u);
         s = run_pass(turn[k], f, 0, ~0ull,
                      !multi || late ? ResolvePart::Whole : k == 0 ? ResolvePart::First : ResolvePart::Later);
         if (s) return s;
@@ -431,7 +434,7 @@ cr_status cr_ooc_render(cr_ooc* o, const cr_camera* cam, uint64_t d_visbuffer, u
         for (size_t q = passes.size(); q-- > 0;) {
             const uint64_t lo = firstId[passes[q].front()];
             const uint64_t hi = q + 1 < passes.size() ? firstId[passes[q + 1].front()] : ~0ull;
-            s = run_pass(q, (flags & CR_RENDER_SYNC) | kRenderResolveOnly, lo, hi, ResolvePart::Whole);
+            s = run_pass(q, (flags & CR_RENDER_SYNC) | next | kRenderResolveOnly, lo, hi, ResolvePart::Whole);
             if (s) return s;
         }
     }

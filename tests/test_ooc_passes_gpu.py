@@ -83,3 +83,20 @@ def test_queues_that_held_a_frame_hold_it_again(gpu):
         for _ in range(3):
             st = frame(sc, whole, 0)[2]
         assert st.uploaded_nodes == NODES - SLOTS
+
+
+@pytest.mark.parametrize("resolve", [0, pc.CR_RENDER_NO_RESOLVE])
+def test_an_overflow_of_any_pass_is_reported(gpu, resolve):
+    """The first pass overflows stage 2's queue, the last has nothing for it."""
+    nodes, keep = node_set()
+    two = [nodes[0], nodes[1]]
+    cam = camera(60.0, 1024, 768)
+    with pc.Context(max_nontrivial=64) as ctx, pc.OocScene(ctx, two, slot_bytes()) as sc:
+        assert frame(sc, cam, resolve)[2].passes == 2
+        st, stats = ctx.stats()
+        assert st == pc.CR_ERR_QUEUE_OVERFLOW and stats.overflow & 1 and stats.nontrivial == 0
+        frame(sc, cam, pc.CR_RENDER_SYNC)
+        assert ctx.stats()[0] == pc.CR_OK
+        frame(sc, cam, resolve)  # the queues are large enough now: nothing is left of the word
+        st, stats = ctx.stats()
+        assert st == pc.CR_OK and stats.overflow == 0
