@@ -696,7 +696,11 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) k_stage1_views_boxes(const C
         const bool hasSub = CR_SUB * (uint32_t)(lane & 7) < numTri - tri0;
         V3 itemAbs = {};
         if (obbs && hasSub) itemAbs = obb_max_abs(load_obb(obbs + CR_OBB_F4 * sub));
-        // the largest coordinates in the whole item, for quick_misses
+        // the largest coordinates in the whole item, for quick_misses.  A sub-box with a
+        // vertex that is not finite or is huge has a NaN centre and bounds none of its
+        // vertices: the item's bound is then infinite, and nothing of it is dropped
+        // (fmaxf would lose the NaN).
+        if (!(itemAbs.x < INFINITY)) itemAbs = V3{INFINITY, INFINITY, INFINITY};
 #pragma unroll
         for (int d = 4; d >= 1; d >>= 1) {
             itemAbs.x = fmaxf(itemAbs.x, __shfl_xor_sync(FULL, itemAbs.x, d));

@@ -104,3 +104,40 @@ def test_hostile_soup_batched_views_equal_single_views(gpu):
             a = batched(c, inst, cams, colorbuffer=True)
             b = plain_loop(c, inst, cams, colorbuffer=True)
             assert_views_equal(a, b, f"hostile batched vs plain ({len(inst)} instances)")
+
+
+@pytest.mark.parametrize("hostile", [np.nan, np.inf, 1e19])
+def test_batched_sub_boxes_that_bound_nothing(gpu, hostile):
+    """Sub-pixel triangles far from the object's origin, sheared to the screen, so
+    that stage 1 rounds their positions by about a pixel; their group of 16 has a
+    vertex that leaves it without a box, and the other groups of the item lie
+    near the origin.  The batch may not bound the rounding by the others."""
+    from test_batch_gpu import assert_views_equal, batched, plain_loop
+
+    rng = np.random.default_rng(31)
+    items, T = 160, 128
+    p = rng.uniform(-0.4, 0.4, (items, T, 1, 3)) + rng.uniform(-0.01, 0.01, (items, T, 3, 3))
+    far = slice(0, 16)
+    step = rng.integers(-64, 65, (items, 16, 1)) + rng.integers(0, 2, (items, 16, 3))
+    other = step - rng.integers(-12, 13, (items, 16, 1))
+    p[:, far, :, 0] = 1e6 + step / 16.0
+    p[:, far, :, 1] = 1e6 + other / 16.0
+    p[:, far, :, 2] = rng.uniform(-0.45, 0.45, (items, 16, 1)) + rng.uniform(-0.03, 0.03, (items, 16, 3))
+    p[:, 0, 1, 2] = hostile
+    pos = p.reshape(-1, 3).astype(np.float32)
+    idx = np.arange(len(pos), dtype=np.uint32).reshape(-1, 3)
+    mesh = (pos, idx, rng.integers(0, 2**32, len(pos), np.uint64).astype(np.uint32))
+    world = np.array([0.7, 0, 1e-7, 0, -0.7, 0, 1e-7, 0, 0, 1, 0, 0, 0, 0, -1.2, 1], np.float32)
+    W, H = 64, 48
+    cams = []
+    for dx in (0.0, 0.013, -0.05):
+        view = np.array(scenes.identity(), np.float32)
+        view[12] = dx
+        cams.append((view, scenes.perspective(60.0, W / H), W, H))
+    with pc.Context() as c:
+        inst = [(c.mesh_from_host(*mesh), world)]
+        b = plain_loop(c, inst, cams)
+        first = b[0][0]
+        ids = (first[first != pc.CLEAR_PIXEL] & np.uint64((1 << 32) - 1)) % np.uint64(T)
+        assert (ids < 16).mean() > 0.1  # the far triangles are seen
+        assert_views_equal(batched(c, inst, cams), b, "groups without a box")
