@@ -455,7 +455,10 @@ static void free_sub_obbs(cr_context* ctx, MeshRec& m) {
 // built once on first use (absent after a failure: the frame then draws every triangle of
 // its listed items, with the same output).
 void ensure_sub_obbs(cr_context* ctx, MeshRec& m) {
-    if (m.subTried || m.numTriangles == 0) return;
+    // a mesh without item boxes is a node of an out-of-core scene: what lies at
+    // its addresses changes with the cache, ordered by other streams than this
+    // build, so nothing is derived from it that outlives the frame
+    if (m.subTried || m.numTriangles == 0 || !m.itemObbs) return;
     m.subTried = true;
     const size_t n = (m.numTriangles + CR_SUB - 1) / CR_SUB, ob = n * CR_OBB_F4 * 16;
     const size_t bytes = ob + n * CR_CONE_FLOATS * 4;

@@ -100,3 +100,40 @@ def test_an_overflow_of_any_pass_is_reported(gpu, resolve):
         frame(sc, cam, resolve)  # the queues are large enough now: nothing is left of the word
         st, stats = ctx.stats()
         assert st == pc.CR_OK and stats.overflow == 0
+
+
+def test_box_culled_contexts_keep_nothing_of_evicted_nodes(gpu):
+    """CR_CULL_BOXES on a stream that does not wait for the legacy one: frames of
+    several passes, nodes evicted and uploaded to other slots, against AUTO."""
+    import torch
+
+    nodes, keep = scenes.ooc_terrain(nodes_x=6, nodes_z=6, quads=20, extent=8.0, with_colors=True)
+    node_bytes = nodes[0][3] * 16 + nodes[0][4] * 12
+    W, H = 160, 90
+    cams = [pc.make_camera(scenes.look_at((4.0, 5.0 - k, 4.01 + k), (4.0, 0.0, 4.0 - k)),
+                           scenes.perspective(60.0, W / H, 0.001, 100.0), W, H) for k in range(4)]
+    with pc.Context() as ctx, pc.OocScene(ctx, nodes, 1 << 30) as sc:
+        want = [frame(sc, cam, pc.CR_RENDER_SYNC) for cam in cams]
+    stream = torch.cuda.Stream()
+    with pc.Context(cull_records=pc.CR_CULL_BOXES) as ctx, pc.OocScene(ctx, nodes, 7 * (node_bytes + 1024)) as sc:
+        evicted = 0
+        for _ in range(3):
+            for cam, (vis, rgba, _) in zip(cams, want):
+                got = frame(sc, cam, 0, stream.cuda_stream)
+                evicted += got[2].evicted_nodes
+                assert np.array_equal(got[0], vis) and np.array_equal(got[1], rgba)
+        assert evicted > 36
+
+
+def test_a_closed_scene_gives_its_memory_back(gpu):
+    """Scenes opened, drawn and closed in a context with a memory budget that
+    does not hold 200 times what a scene's nodes could keep beside the cache (4 KB
+    of boxes each); then one with a larger cache."""
+    nodes, keep = scenes.ooc_terrain(nodes_x=6, nodes_z=6, quads=20, extent=8.0, with_colors=True)
+    cam = pc.make_camera(scenes.look_at((4.0, 9.0, 4.01), (4.0, 0.0, 4.0)), scenes.perspective(60.0, 1.0, 0.001, 100.0), 96, 96)
+    with pc.Context(cull_records=pc.CR_CULL_BOXES, max_nontrivial=4096, max_huge=4096, memory_budget=44 << 20) as ctx:
+        for _ in range(200):
+            with pc.OocScene(ctx, nodes, 2 << 20) as sc:
+                assert frame(sc, cam, pc.CR_RENDER_SYNC)[2].visible_nodes == 36
+        with pc.OocScene(ctx, nodes, 6 << 20) as sc:
+            assert frame(sc, cam, pc.CR_RENDER_SYNC)[2].cache_slots > 36
