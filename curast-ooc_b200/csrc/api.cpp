@@ -373,8 +373,10 @@ cr_status ensure_queues(cr_context* ctx, uint64_t ntWant, uint64_t hugeWant) {
 
 // The chain heads, entry counts and unit list of the binned stage 3 for a frame
 // of `tiles` screen tiles and the current stage-3 queue; without memory for
-// them the frame takes the unbinned stage 3.
-void ensure_bins(cr_context* ctx, uint64_t tiles) {
+// them the frame takes the unbinned stage 3.  The heads are cleared on the
+// frame's own stream (which may not wait for the legacy one): later frames wait
+// for it.
+void ensure_bins(cr_context* ctx, uint64_t tiles, cudaStream_t stream) {
     // a unit per tile and per CR_BIN_PART further entries
     const uint64_t units = tiles + ctx->hugeCap / CR_BIN_PART;
     if (tiles <= ctx->binTiles && units <= ctx->binUnitCap) return;
@@ -387,7 +389,7 @@ void ensure_bins(cr_context* ctx, uint64_t tiles) {
     ctx->binBytes = 0;
     void* heads = nullptr;
     if (ctx->dev_alloc(&heads, hb + cb + ub, "stage-3 bins") != CR_OK) return;
-    if (cudaMemset(heads, 0, hb + cb) != cudaSuccess) {
+    if (cudaMemsetAsync(heads, 0, hb + cb, stream) != cudaSuccess) {
         cudaGetLastError();
         ctx->dev_free(heads, hb + cb + ub);
         return;
@@ -1442,7 +1444,7 @@ cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_
 
     auto issue = [&](cudaEvent_t* tev, cudaEvent_t rasterEnd) -> cr_status {
         fp.binHeads = nullptr;
-        if (bins && ctx->hugeCap < 0xffffffffull) ensure_bins(ctx, binTiles);  // the queue may have grown
+        if (bins && ctx->hugeCap < 0xffffffffull) ensure_bins(ctx, binTiles, stream);  // the queue may have grown
         if (bins && ctx->hugeCap < 0xffffffffull && ctx->binHeads) {
             if (++ctx->binStamp == 0) {  // the stamps wrapped: empty every chain
                 CR_CUDA(cudaMemsetAsync(ctx->binHeads, 0, ctx->binTiles * CR_BIN_CHAINS * 8, stream), "stage-3 bins");

@@ -53,3 +53,31 @@ def test_bins_match_the_oracle_and_the_unbinned_kernel(gpu, n, W, H):
     assert np.array_equal(got[0][0], got[1][0])
     fb, _ = ol.raster(ol.Frame([(*mesh, scenes.identity())], view), W, H, proj[5])
     assert np.array_equal(got[0][0], fb)
+
+
+def test_bins_that_grow_on_a_side_stream(gpu):
+    """Windows and a queue that grow from frame to frame, so that the chains are
+    laid out anew, on a stream that does not wait for the legacy one."""
+    import torch
+
+    mesh = triangles(400, 77)
+    sizes = [(64, 64), (200, 130), (640, 360), (65, 129), (1917, 1083)]
+    got = []
+    for budget in (8 << 30, 0):
+        stream = torch.cuda.Stream()
+        with pc.Context(memory_budget=budget, max_huge=64) as ctx:
+            inst = [(ctx.mesh_from_host(*mesh), scenes.identity())]
+            outs = []
+            with torch.cuda.stream(stream):
+                for W, H in sizes:
+                    vis = torch.empty(W * H, dtype=torch.int64, device="cuda")
+                    rgba = torch.empty(W * H, dtype=torch.int32, device="cuda")
+                    cam = pc.make_camera(scenes.identity(), scenes.perspective(60.0, W / H, 0.01, 100.0), W, H)
+                    ctx.render(inst, cam, vis.data_ptr(), rgba.data_ptr(), stream=stream.cuda_stream)
+                    outs.append(vis)
+            torch.cuda.synchronize()
+            st, stats = ctx.stats()
+            assert st == pc.CR_OK and stats.huge_tiles > 64
+            got.append(outs)
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
