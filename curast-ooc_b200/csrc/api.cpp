@@ -372,35 +372,40 @@ cr_status ensure_queues(cr_context* ctx, uint64_t ntWant, uint64_t hugeWant) {
 }
 
 // The chain heads, entry counts and unit list of the binned stage 3 for a frame
-// of `tiles` screen tiles and the current stage-3 queue; without memory for
-// them the frame takes the unbinned stage 3.  The heads are cleared on the
+// of `tiles` screen tiles and the current stage-3 queue: false without memory for
+// them (the frame then takes the unbinned stage 3).  The heads are cleared on the
 // frame's own stream (which may not wait for the legacy one): later frames wait
 // for it.
-void ensure_bins(cr_context* ctx, uint64_t tiles, cudaStream_t stream) {
+bool ensure_bins(cr_context* ctx, uint64_t tiles, cudaStream_t stream) {
     // a unit per tile and per CR_BIN_PART further entries
     const uint64_t units = tiles + ctx->hugeCap / CR_BIN_PART;
-    if (tiles <= ctx->binTiles && units <= ctx->binUnitCap) return;
-    if (cudaDeviceSynchronize() != cudaSuccess) return;
+    if (tiles <= ctx->binTiles && units <= ctx->binUnitCap) return true;
     tiles = std::max(tiles, ctx->binTiles);
     const size_t hb = tiles * CR_BIN_CHAINS * 8, cb = align_up(tiles * 4, 256), ub = units * sizeof(uint2);
-    ctx->dev_free(ctx->binHeads, ctx->binBytes);
-    ctx->binHeads = nullptr;
-    ctx->binTiles = ctx->binUnitCap = 0;
-    ctx->binBytes = 0;
+    const size_t bytes = hb + cb + ub;
+    if (ctx->binRefusal.stands(bytes)) return false;
     void* heads = nullptr;
-    if (ctx->dev_alloc(&heads, hb + cb + ub, "stage-3 bins") != CR_OK) return;
-    if (cudaMemsetAsync(heads, 0, hb + cb, stream) != cudaSuccess) {
-        cudaGetLastError();
-        ctx->dev_free(heads, hb + cb + ub);
-        return;
+    const size_t ask = (ctx->cfg.debug_flags & CR_DEBUG_REFUSE_STAGE3_BINS) ? SIZE_MAX / 4 : bytes;
+    if (ctx->dev_alloc(&heads, ask, "stage-3 bins") != CR_OK) {
+        cr_internal_set_error("");
+        ctx->binRefusal.refused(bytes);
+        return false;
     }
+    if (cudaMemsetAsync(heads, 0, hb + cb, stream) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
+        cudaGetLastError();
+        ctx->dev_free(heads, bytes);
+        ctx->binRefusal.refused(bytes);
+        return false;
+    }
+    ctx->dev_free(ctx->binHeads, ctx->binBytes);  // no frame in flight reads them any more
     ctx->binHeads = (unsigned long long*)heads;
     ctx->binCounts = (uint32_t*)((char*)heads + hb);
     ctx->binUnits = (uint2*)((char*)heads + hb + cb);
     ctx->binTiles = tiles;
     ctx->binUnitCap = units;
-    ctx->binBytes = hb + cb + ub;
+    ctx->binBytes = bytes;
     ctx->binStamp = 0;
+    return true;
 }
 
 // Allocates (once) and launches the mesh's box pass on the legacy stream.
@@ -1257,7 +1262,8 @@ cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_
         cellMode = CR_REC_CELLS32;  // 12-bit coordinates fit: half the record bytes
     // the failure-detection hook drops an index-tile copy, which box-culled
     // frames do not make
-    if (ctx->cfg.debug_flags && cellMode == CR_REC_BOXES && !refMath)
+    const bool dropCopy = (ctx->cfg.debug_flags & CR_DEBUG_DROP_FIRST_TILE_COPY) != 0;
+    if (dropCopy && cellMode == CR_REC_BOXES && !refMath)
         cellMode = cam->width <= 4096 && cam->height <= 4096 ? CR_REC_CELLS32 : CR_REC_OUTCODES;
     bool boxes = cellMode == CR_REC_BOXES;
     uint64_t triangles = 0;
@@ -1266,7 +1272,7 @@ cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_
     // explicit ids may have gaps, a forced record mode is kept, and the
     // failure-detection hook drops a copy that the direct path does not make
     const bool mayDirect = rec == CR_CULL_AUTO && !refMath && !firstIds && count > 0 && triangles > 0 &&
-                           !(flags & kRenderResolveOnly) && ctx->cfg.debug_flags == 0;
+                           !(flags & kRenderResolveOnly) && !dropCopy;
     bool direct = mayDirect && triangles <= kDirectLimit;
 
     Assembled A;
@@ -1444,8 +1450,7 @@ cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_
 
     auto issue = [&](cudaEvent_t* tev, cudaEvent_t rasterEnd) -> cr_status {
         fp.binHeads = nullptr;
-        if (bins && ctx->hugeCap < 0xffffffffull) ensure_bins(ctx, binTiles, stream);  // the queue may have grown
-        if (bins && ctx->hugeCap < 0xffffffffull && ctx->binHeads) {
+        if (bins && ctx->hugeCap < 0xffffffffull && ensure_bins(ctx, binTiles, stream)) {  // the queue may have grown
             if (++ctx->binStamp == 0) {  // the stamps wrapped: empty every chain
                 CR_CUDA(cudaMemsetAsync(ctx->binHeads, 0, ctx->binTiles * CR_BIN_CHAINS * 8, stream), "stage-3 bins");
                 ctx->binStamp = 1;

@@ -18,6 +18,7 @@
 
 #include "cr_device.h"
 #include "curast_b200.h"
+#include "refusal.h"
 
 namespace cr {
 
@@ -170,6 +171,7 @@ struct cr_context {
     uint2* binUnits = nullptr;
     uint64_t binTiles = 0, binUnitCap = 0;
     size_t binBytes = 0;
+    cr::Refusal binRefusal;
     uint32_t binStamp = 0;                    // the last issued frame's stamp (0 is never issued)
     unsigned long long* counters = nullptr;
     unsigned long long* hCounters = nullptr;  // pinned

@@ -73,6 +73,7 @@ CR_CULL_BOXES = 3
 
 
 CR_DEBUG_DROP_FIRST_TILE_COPY = 1
+CR_DEBUG_REFUSE_STAGE3_BINS = 2
 
 
 class CrMeshDesc(ctypes.Structure):

@@ -99,6 +99,9 @@ typedef struct cr_config {
  * copy, so the bounded wait for it runs out; the frame then reports
  * CR_ERR_TIMEOUT and the context stays usable. */
 #define CR_DEBUG_DROP_FIRST_TILE_COPY 1u
+/* Test hook: the memory of the binned stage 3 is refused; frames take the
+ * unbinned one, with the same output and no error. */
+#define CR_DEBUG_REFUSE_STAGE3_BINS 2u
 
 typedef enum cr_memory { CR_MEM_HOST = 0, CR_MEM_DEVICE = 1 } cr_memory;
 

@@ -81,3 +81,26 @@ def test_bins_that_grow_on_a_side_stream(gpu):
             got.append(outs)
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+def test_frames_without_memory_for_the_bins(gpu):
+    """Drawn by the unbinned kernel, and no error is left behind."""
+    import torch
+
+    W, H = 333, 197
+    mesh = triangles(300, 78)
+    cam = pc.make_camera(scenes.identity(), scenes.perspective(60.0, W / H, 0.01, 100.0), W, H)
+    got = []
+    for debug in (0, pc.CR_DEBUG_REFUSE_STAGE3_BINS):
+        with pc.Context(debug_flags=debug) as ctx:
+            inst = [(ctx.mesh_from_host(*mesh), scenes.identity())]
+            for _ in range(3):
+                vis = torch.empty(W * H, dtype=torch.int64, device="cuda")
+                rgba = torch.empty(W * H, dtype=torch.int32, device="cuda")
+                ctx.render(inst, cam, vis.data_ptr(), rgba.data_ptr())
+                got.append((vis, rgba))
+            assert ctx.stats()[1].huge_tiles > 0
+            if debug:
+                assert pc.load().cr_last_error() == b""
+    for v, r in got[1:]:
+        assert torch.equal(v, got[0][0]) and torch.equal(r, got[0][1])
