@@ -490,19 +490,15 @@ bool sub_obbs_fit(cr_context* ctx, const cr_instance* instances, uint32_t count)
     for (uint32_t i = 0; i < count; i++) {
         if (instances[i].mesh >= ctx->meshes.size()) return false;
         const MeshRec& m = ctx->meshes[instances[i].mesh];
-        if (!m.live || !m.itemObbs || m.subDeclined || (m.subTried && !m.subObbs)) return false;
+        if (!m.live || !m.itemObbs || (m.subTried && !m.subObbs)) return false;
         if (!m.subObbs) need += (size_t)((m.numTriangles + CR_SUB - 1) / CR_SUB) * (CR_OBB_F4 * 16 + CR_CONE_FLOATS * 4);
     }
     if (need == 0) return true;
+    if (ctx->cfg.memory_budget != 0 || ctx->subRefusal.stands(need)) return false;
     size_t freeBytes = 0, total = 0;
-    const bool fits = ctx->cfg.memory_budget == 0 && cudaMemGetInfo(&freeBytes, &total) == cudaSuccess &&
-                      freeBytes > 2 * need + (1ull << 30);
-    if (!fits)
-        for (uint32_t i = 0; i < count; i++) {
-            MeshRec& m = ctx->meshes[instances[i].mesh];
-            if (!m.subObbs) m.subDeclined = true;  // not asked again every frame
-        }
-    return fits;
+    if (cudaMemGetInfo(&freeBytes, &total) == cudaSuccess && freeBytes > 2 * need + (1ull << 30)) return true;
+    ctx->subRefusal.refused(need);
+    return false;
 }
 
 void ensure_sub_obbs_for(cr_context* ctx, const cr_instance* instances, uint32_t count) {
@@ -1164,6 +1160,7 @@ cr_status cr_mesh_refresh(cr_context* ctx, uint32_t mesh) {
     if (m.subObbs && cr_launch_sub_obbs(m.indices, m.positions, m.compressed ? m.dCodec : nullptr, m.numTriangles,
                                         m.subObbs, (float*)m.subCones, 0))
         return fail(CR_ERR_CUDA, "sub-box launch: %s", cudaGetErrorString(cudaGetLastError()));
+    if (!m.subObbs) m.subTried = false;  // a build that failed is tried again on next use
     return build_mesh_boxes(ctx, m);
 }
 

@@ -62,7 +62,6 @@ struct MeshRec {
     float4* subCones = nullptr;   // CR_CONE_FLOATS each, in the same allocation
     size_t subBytes = 0;
     bool subTried = false;
-    bool subDeclined = false;     // no room for them when a frame would have liked them
 };
 
 void mat4_mul(const float* a, const float* b, float* out);  // glm order
@@ -172,6 +171,7 @@ struct cr_context {
     uint64_t binTiles = 0, binUnitCap = 0;
     size_t binBytes = 0;
     cr::Refusal binRefusal;
+    cr::Refusal subRefusal;                   // oriented sub-boxes of frames that can do without them
     uint32_t binStamp = 0;                    // the last issued frame's stamp (0 is never issued)
     unsigned long long* counters = nullptr;
     unsigned long long* hCounters = nullptr;  // pinned

@@ -96,6 +96,34 @@ def test_large_sub_pixel_frames_are_box_culled(gpu, tris, orbit, W, H):
     assert got[1][0][2].vertex_chunks == 0  # no vertex pass
 
 
+def test_sub_boxes_are_built_once_memory_is_back(gpu):
+    """A frame that had no room for the oriented boxes is drawn from records, and
+    box-culled some frames after the room is there."""
+    import torch
+
+    W, H = 640, 360
+    pos, idx, col = scenes.planet(2_300_000, seed=3, device="cuda", width=W, height=H)
+    cam = pc.make_camera(*scenes.planet_orbit_camera(W, H), W, H)
+    vis = torch.empty(W * H, dtype=torch.int64, device="cuda")
+    rgba = torch.empty(W * H, dtype=torch.int32, device="cuda")
+    with pc.Context() as ctx:
+        h = ctx.mesh_from_device(pos.data_ptr(), pos.shape[0], idx.data_ptr(), idx.shape[0], col.data_ptr())
+        inst = [(h, scenes.identity())]
+        chunks, seen = [], []
+        torch.cuda.empty_cache()
+        held = torch.empty(torch.cuda.mem_get_info()[0] - (900 << 20), dtype=torch.uint8, device="cuda")
+        for k in range(140):
+            if k == 2:
+                del held
+                torch.cuda.empty_cache()
+            ctx.render(inst, cam, vis.data_ptr(), rgba.data_ptr())
+            chunks.append(int(ctx.stats()[1].vertex_chunks))
+            if k in (0, 139):
+                seen.append((vis.clone(), rgba.clone()))
+    assert chunks[0] > 0 and chunks[1] > 0 and chunks[-1] == 0  # no vertex pass in the end
+    assert torch.equal(seen[0][0], seen[1][0]) and torch.equal(seen[0][1], seen[1][1])
+
+
 def test_more_survivors_than_the_list_holds(gpu):
     W, H = 2560, 1440
     pos, idx, col = keep = scenes.terrain(1500, seed=3, device="cuda")
