@@ -1214,11 +1214,15 @@ cr_status cr_render(cr_context* ctx, const cr_instance* instances, uint32_t coun
 
 // Frames of at most this many triangles take every triangle straight through
 // the per-triangle path (CrFrameParams::direct).  Below it the kernels that decide
-// which triangles not to draw mostly cost more than drawing them.  Direct / culled from
-// boxes, whole frame in us: planet from its surface at 1280x720 1.1M 87 / 109, 1.6M
-// 96 / 109, 2.2M 168 / 106, 4.1M 185 / 104; seen whole 1.1M 50 / 75, 2.2M 84 / 71, 4.1M
-// 114 / 75; 10 x 300K instances 50 / 51, 100 x 20K 48 / 76.  (Heightfields of needles gain from
-// it further up: 2.1M at 391x220 164 / 199, 4M 289 / 336; by records 228, 364.)
+// which triangles not to draw cost more than drawing them, for every kind of scene
+// measured; planets cross near 2.6M, heightfields (needles) gain beyond 4M.  Direct / culled
+// from boxes, whole frame in us, windows of 242x180, 640x480 and 1280x720:
+//   planet from its surface 1.1M 48 / 58, 85 / 91, 87 / 106; 2.1M 54 / 61, 88 / 97, 101 / 104;
+//     2.6M 61 / 61, 97 / 96, 108 / 105; 4.1M 73 / 62, 111 / 95, 123 / 106
+//   planet seen whole 1.1M 33 / 43, 48 / 60, 50 / 74; 2.1M 41 / 48, 60 / 61, 66 / 71;
+//     2.6M 48 / 49, 61 / 64, 73 / 75; 4.1M 62 / 49, 75 / 64, 86 / 77
+//   heightfield 2.1M at 160x90 86 / 122, 391x220 156 / 199, 813x610 371 / 431; 4M 135 / 193, 257 / 336, 587 / 672
+//   at 816x612 10 x 300K instances 51 / 53, 100 x 20K 51 / 76, 1000 x 2K 246 / 258
 static constexpr uint64_t kDirectLimit = 2ull << 20;
 
 cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_t count, const uint64_t* firstIds,

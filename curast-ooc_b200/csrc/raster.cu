@@ -790,13 +790,18 @@ __global__ void __launch_bounds__(WARPS * 32) k_s1raster(const CrFrameParams p) 
 
 // k_s1direct: direct frames whose triangles are mostly sub-pixel.  Every
 // triangle of every instance, one per lane, through quick_misses; the few it
-// leaves queue in a per-warp ring for the full path, 32 at a time.  A warp takes
-// consecutive triangles, so that its instance (and what the test needs of it)
-// changes rarely.  (300 x 5,121 triangles at 1280x720: every triangle through the
-// full path 35 us, so 26.  A 2M-triangle heightfield of needles at 391x220: each lane
-// its own raster 205 us, the rasters shared over the warp 136; by way of the survivor
-// list and k_s1raster 159.)
-template <int WARPS, bool PACKED>
+// leaves queue in a per-warp ring for the full path, 32 at a time, whose rasters the
+// warp shares.  (2M-triangle heightfield of needles at 391x220: each lane its own
+// raster 205 us, shared 136; by way of the survivor list and k_s1raster 159.)
+//
+// Which triangles a warp takes: FEW (at most S1D_FEW instances): 32 here and there, the
+// warps side by side, so that a crowded part of a mesh is shared out.  Otherwise one run of
+// consecutive ones, so that its instance (and what the test needs of it) changes rarely.
+// Stage 1, runs / FEW: planet from its surface at 1280x720 1.85M 99 / 43 us, at 640x480 62 / 41,
+// seen whole at 1280x720 61 / 40; 2M heightfield at 391x220 146 / 126; 100,000-triangle meshes
+// and larger drawn 2 and 4 times 23 / 23.  300 x 5,121 triangles at 1280x720 in runs 23, a search per
+// 32 triangles 34.
+template <int WARPS, bool PACKED, bool FEW>
 __global__ void __launch_bounds__(WARPS * 32, 4) k_s1direct(const CrFrameParams p) {
     pdl_enter();
     __shared__ uint64_t s_ring[WARPS][S1_RING];
@@ -807,14 +812,15 @@ __global__ void __launch_bounds__(WARPS * 32, 4) k_s1direct(const CrFrameParams 
     const float Wf = (float)p.W, Hf = (float)p.H;
     uint64_t* const ring = s_ring[threadIdx.x >> 5];
     uint32_t qh = 0, qt = 0;  // ring head / tail (warp-uniform)
-    const uint64_t share = (p.direct + 32 * nw - 1) / (32 * nw) * 32;
-    const uint64_t end = min(p.direct, (gw + 1) * share);
+    const uint64_t share = FEW ? 32 : (p.direct + 32 * nw - 1) / (32 * nw) * 32;
+    const uint64_t step = FEW ? 32 * nw : 32;
+    const uint64_t end = FEW ? p.direct : min(p.direct, (gw + 1) * share);
     uint32_t inst = gw * share < p.direct ? instance_of_triangle(p, gw * share, gw * share) : 0u;
     uint32_t of = 0xffffffffu;  // the instance that q, g and cum are of
     Quick q;
     GeomRef g;
     uint64_t cum = 0;
-    for (uint64_t base = gw * share; qh < qt || base < end; base += 32) {
+    for (uint64_t base = gw * share; qh < qt || base < end; base += step) {
         if (base < end) {
             const uint64_t j = base + lane;
             bool keep = j < end;
@@ -838,7 +844,7 @@ __global__ void __launch_bounds__(WARPS * 32, 4) k_s1direct(const CrFrameParams 
             qt += __popc(m);
             __syncwarp();
         }
-        if (qt - qh < 32u && base + 32 < end) continue;
+        if (qt - qh < 32u && base + step < end) continue;
         const uint32_t k = qh + lane;
         int res = S1_CULL;
         uint32_t tri = 0, in = 0;
@@ -1034,6 +1040,8 @@ __global__ void __launch_bounds__(256) k_clear(uint64_t* fb, uint64_t n, unsigne
 }  // namespace
 
 constexpr int S1_WARPS = 8;
+// k_s1direct: at most this many instances: a warp's triangles lie apart (FEW)
+constexpr uint32_t S1D_FEW = 4;
 constexpr int S2_WARPS = 8;
 constexpr int S3_WARPS = 8;
 constexpr int VX_THREADS = 256;
@@ -1071,7 +1079,7 @@ int cr_query_launch_shape(int device, CrLaunchShape* out) {
         return -1;
     out->s1RasterOwnBlocks = sms * (bo > 0 ? bo : 1);
     int bd = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bd, k_s1direct<S1_WARPS, false>, S1_WARPS * 32, 0) != cudaSuccess)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bd, k_s1direct<S1_WARPS, false, false>, S1_WARPS * 32, 0) != cudaSuccess)
         return -1;
     out->s1DirectBlocks = sms * (bd > 0 ? bd : 1);
     out->stage3Blocks = sms * (b3 > 0 ? b3 : 1);
@@ -1157,8 +1165,11 @@ int cr_launch_stage1(const CrFrameParams& p, const CrLaunchShape& s, void* strea
                                : launch_pdl(k_s1raster<S1_WARPS, false, true, true>, bc, T, stream, p);
         }
         const unsigned bd = (unsigned)std::min<uint64_t>(want, (uint64_t)s.s1DirectBlocks);
-        return p.anyPacked ? launch_pdl(k_s1direct<S1_WARPS, true>, bd, T, stream, p)
-                           : launch_pdl(k_s1direct<S1_WARPS, false>, bd, T, stream, p);
+        if (p.numInstances <= S1D_FEW)
+            return p.anyPacked ? launch_pdl(k_s1direct<S1_WARPS, true, true>, bd, T, stream, p)
+                               : launch_pdl(k_s1direct<S1_WARPS, false, true>, bd, T, stream, p);
+        return p.anyPacked ? launch_pdl(k_s1direct<S1_WARPS, true, false>, bd, T, stream, p)
+                           : launch_pdl(k_s1direct<S1_WARPS, false, false>, bd, T, stream, p);
     }
     const uint64_t itemBlocks = (p.numItems + S1_WARPS - 1) / S1_WARPS;
     const unsigned T = S1_WARPS * 32;

@@ -80,6 +80,26 @@ def test_small_frames_match_every_record_mode(gpu, kind, sizes):
     assert all(s.stage1_survivors == s.triangles for _, _, s in got)
 
 
+# one, the most and more instances than a direct frame shares out 32 triangles at a time;
+# meshes whose ends lie inside a warp's 32, one without triangles among them
+@pytest.mark.parametrize("count,compressed", [(1, False), (4, False), (4, True), (5, False)])
+def test_direct_frames_of_few_instances(gpu, count, compressed):
+    W, H = 201, 113
+    meshes = [scenes.heightfield(131 + 7 * k, 61 + k, seed=k) for k in range(count)]
+    if count > 2 and not compressed:
+        p, i, c = meshes[1]
+        meshes[1] = (p, i[:0], c)
+    cams = [(scenes.heightfield_camera(W, H)[0], scenes.perspective(60.0, W / H, 0.01, 100.0), W, H)]
+    got = []
+    for mode in (pc.CR_CULL_CELLS, pc.CR_CULL_AUTO):
+        with pc.Context(cull_records=mode) as ctx:
+            inst = [(upload(ctx, m, compressed), scenes.translate_scale(0.05 * k, 0.03 * k, -0.1 * k))
+                    for k, m in enumerate(meshes)]
+            got += frames(ctx, inst, cams)
+    assert (got[0][0] != pc.CLEAR_PIXEL).any() and got[1][2].stage1_survivors == got[1][2].triangles
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+
+
 @pytest.mark.parametrize("tris,orbit,W,H", [(2_300_000, False, 319, 181), (6_000_001, True, 640, 360)])
 def test_large_sub_pixel_frames_are_box_culled(gpu, tris, orbit, W, H):
     pos, idx, col = keep = scenes.planet(tris, seed=3, device="cuda", width=W, height=H)
