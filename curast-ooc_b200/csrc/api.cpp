@@ -1481,13 +1481,8 @@ cr_status cr::render_impl(cr_context* ctx, const cr_instance* instances, uint32_
         CR_CUDA(mark(0), "event");
         const bool raster = !(flags & kRenderResolveOnly);
         if ((flags & CR_RENDER_NO_CLEAR) || !raster) {
-            static_assert(CR_CTR_TIMEOUT == CR_CTR_OVERFLOW + 1 && CR_CTR_TIMEOUT + 1 < CR_CTR_COUNT, "two neighbouring words");
-            const int kept = (flags & kRenderNextPass) ? CR_CTR_OVERFLOW : CR_CTR_COUNT;  // counters before the words that stay
-            CR_CUDA(cudaMemsetAsync(ctx->counters, 0, kept * sizeof(unsigned long long), stream), "counters");
-            if (kept < CR_CTR_COUNT)
-                CR_CUDA(cudaMemsetAsync(ctx->counters + CR_CTR_TIMEOUT + 1, 0,
-                                        (CR_CTR_COUNT - CR_CTR_TIMEOUT - 1) * sizeof(unsigned long long), stream),
-                        "counters");
+            const int own = (flags & kRenderNextPass) ? CR_CTR_PASS : CR_CTR_COUNT;
+            CR_CUDA(cudaMemsetAsync(ctx->counters, 0, own * sizeof(unsigned long long), stream), "counters");
             if (fp.binHeads) CR_CUDA(cudaMemsetAsync(ctx->binCounts, 0, binTiles * 4, stream), "stage-3 bins");
         } else if (cr_launch_clear(fp.fb, numPixels, ctx->counters, stream, fp.binHeads ? ctx->binCounts : nullptr,
                                    (uint32_t)binTiles)) {

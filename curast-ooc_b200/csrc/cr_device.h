@@ -20,9 +20,6 @@
 // counters[] slots
 #define CR_CTR_NONTRIVIAL 0     // entries appended to the stage-2 queue
 #define CR_CTR_HUGE 1           // tiles appended to the stage-3 queue
-#define CR_CTR_OVERFLOW 2       // bit 0: stage-2 queue, bit 1: stage-3 queue,
-                                // bit 2: stage-1 survivor list
-#define CR_CTR_TIMEOUT 3        // nonzero if a bounded device wait gave up
 #define CR_CTR_ITEMS 4          // stage-1 work items that survive the item cull
 #define CR_CTR_CHUNKS 5         // vertex-pass chunks that need per-vertex records
 #define CR_CTR_SURVIVORS 6      // stage-1 triangles the records do not cull
@@ -32,7 +29,12 @@
 #define CR_CTR_VSLICES 9        // slices the vertex pass evaluated (frames with slice stamps)
 #define CR_CTR_S3UNIT 10        // units taken by k_stage3_bins
 #define CR_CTR_BINUNITS 11      // units of the binned stage 3
+#define CR_CTR_OVERFLOW 14      // bit 0: stage-2 queue, bit 1: stage-3 queue,
+                                // bit 2: stage-1 survivor list
+#define CR_CTR_TIMEOUT 15       // nonzero if a bounded device wait gave up
 #define CR_CTR_COUNT 16
+#define CR_CTR_PASS 14          // the counters before this one are a pass's own, the others an
+                                // asynchronous frame's of several passes
 
 // Compressed geometry (the reference's IX_PU16 meshes, CMesh fields
 // compressionFactor / index_min / aabb.min / bitsPerIndex / compressed,
