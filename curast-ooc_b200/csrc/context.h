@@ -109,6 +109,7 @@ struct Assembled {
     uint64_t numItems = 0;
     uint64_t outBytes = 0;     // vertex-pass record slots of all instances
     uint64_t numVChunks = 0;   // vertex-pass chunks of all instances
+    uint64_t numVSlices = 0;   // their vertices in slices of CR_VSLICE
     uint64_t numUnits = 0;     // group-cull units (CR_GROUP items of one instance chunk)
     uint64_t numChunkGroups = 0;  // group-cull chunk groups (CR_GROUP chunks of one instance)
 };
