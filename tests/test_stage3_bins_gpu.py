@@ -55,6 +55,48 @@ def test_bins_match_the_oracle_and_the_unbinned_kernel(gpu, n, W, H):
     assert np.array_equal(got[0][0], fb)
 
 
+def covering(n, seed):
+    """Front-facing triangles over the whole screen, one behind the other and
+    slanted; past 600, every eighth leaves a part of it free."""
+    rng = np.random.default_rng(seed)
+    z = rng.uniform(2.0, 9.0, (n, 1))
+    corner = np.array([[-9.0, -7.0], [9.0, -7.0], [0.0, 14.0]]) * (1 + 0.3 * rng.uniform(-1, 1, (n, 3, 2)))
+    corner[600::8] += rng.uniform(-6, 6, (len(corner[600::8]), 1, 2))
+    depth = z * (1 + 0.2 * rng.uniform(-1, 1, (n, 3)))
+    tri = np.concatenate([corner * z[:, :, None], -depth[:, :, None]], -1)
+    pos = tri.reshape(-1, 3).astype(np.float32)
+    return pos, np.arange(3 * n, dtype=np.uint32).reshape(n, 3), rng.integers(0, 2**32, 3 * n, np.uint64).astype(np.uint32)
+
+
+# a tile's entries: one past a unit's 512, several units, more than 128 units
+# (which then take more than 512 each); one tile and several, whose edge is ragged
+@pytest.mark.parametrize("n,W,H", [(513, 72, 64), (1024, 64, 72), (3000, 130, 70), (70000, 72, 64)])
+def test_crowded_tiles_are_shared_out(gpu, n, W, H):
+    import torch
+
+    tiles = ((W + 63) // 64) * ((H + 63) // 64)
+    mesh = covering(n, n)
+    view, proj = scenes.identity(), scenes.perspective(60.0, W / H, 0.01, 100.0)
+    got = []
+    for budget in (0, 8 << 30):
+        with pc.Context(memory_budget=budget) as ctx:
+            inst = [(ctx.mesh_from_host(*mesh), scenes.identity())]
+            vis = torch.empty(W * H, dtype=torch.int64, device="cuda")
+            rgba = torch.empty(W * H, dtype=torch.int32, device="cuda")
+            ctx.render(inst, pc.make_camera(view, proj, W, H), vis.data_ptr(), rgba.data_ptr())
+            torch.cuda.synchronize()
+            st, stats = ctx.stats()
+            assert st == pc.CR_OK and stats.overflow == 0
+            # queued in every tile: the first 600 and at least seven of every further eight
+            assert stats.huge_tiles >= tiles * (min(n, 600) + max(n - 600, 0) * 7 // 8)
+            got.append(vis.cpu().numpy().view(np.uint64))
+    assert np.array_equal(got[0], got[1])
+    assert len(np.unique(got[0])) > W * H // 2
+    if n <= 3000:
+        fb, _ = ol.raster(ol.Frame([(*mesh, scenes.identity())], view), W, H, proj[5])
+        assert np.array_equal(got[0], fb)
+
+
 def test_bins_that_grow_on_a_side_stream(gpu):
     """Windows and a queue that grow from frame to frame, so that the chains are
     laid out anew, on a stream that does not wait for the legacy one."""
