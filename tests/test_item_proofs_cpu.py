@@ -1,8 +1,10 @@
 """Soundness of the frame cull's single-precision item proofs (raster_core.cuh
-item_back_facing and obb_misses_samples, with the oriented boxes of meshprep.cu
-k_obbs and the per-instance data of api.cpp proof_data), restated in numpy with
-the same float operations: whenever a proof says an item is culled, every one of
-its triangles (vertices) meets stage 1's float test."""
+item_back_facing and obb_misses_samples, with the per-instance data of api.cpp
+proof_data), restated in numpy with the same float operations: whenever a proof
+says an item is culled, every one of its triangles (vertices) meets stage 1's
+float test.  The proofs are given tight oriented boxes (obb); that those of
+meshprep.cu k_obbs hold their vertices is a test of its own, on a restatement of
+that kernel."""
 import numpy as np
 import pytest
 from test_backface_proof_cpu import back_face_data, det3_glm, item_cone, items, look_at, stage1_backface_culled, xform
@@ -61,7 +63,7 @@ def proof_back_facing(M, lo, hi, cone, drop_error=False):
 
 
 def obb(p):
-    """meshprep.cu k_obbs on an (n, 3) float32 set, with a given frame's axes."""
+    """A box of an (n, 3) float32 set along its principal axes, tighter than meshprep.cu's."""
     q = p.astype(np.float64)
     _, _, ax = np.linalg.svd(q - q.mean(0), full_matrices=True)
     x = q @ ax.T
@@ -259,3 +261,116 @@ def test_back_face_proof_is_sound(drop):
                 wrong += not stage1_backface_culled(M, det3_glm(M) < 0, pa, pb, pc).all()
     assert proved > 100
     assert (wrong > 0) if drop else (wrong == 0), (proved, wrong)
+
+
+def lanes_sum(v):
+    """A warp's butterfly sum over axis 0 in float32: every lane gets the same value."""
+    i = np.arange(len(v))
+    d = len(v) // 2
+    while d:
+        v = (v + v[i ^ d]).astype(F)
+        d //= 2
+    return v[0]
+
+
+def off_by(rng, x):
+    """A float32 function value, up to 2 ulp from the rounded one."""
+    x = F(x)
+    for _ in range(int(rng.integers(0, 3))):
+        x = np.nextafter(x, F(np.inf) if rng.random() < 0.5 else F(-np.inf))
+    return F(x)
+
+
+def kernel_obb(rng, q, lanes, slack=True):
+    """meshprep.cu k_obbs: q (lanes, R, 3 corners, 3) float32, NaN where a lane's
+    triangle is past the mesh's end.  Every operation rounded to float32 in the
+    kernel's order; rsqrtf, atan2f, sinf and cosf within 2 ulp either way."""
+    live = ~np.isnan(q[..., 0, 0])
+    R = q.shape[1]
+    with np.errstate(all="ignore"):
+        n = np.zeros((lanes, 3), F)
+        for r in range(R):
+            u, v = q[:, r, 1] - q[:, r, 0], q[:, r, 2] - q[:, r, 0]
+            x = u[:, 1] * v[:, 2] - u[:, 2] * v[:, 1]
+            y = u[:, 2] * v[:, 0] - u[:, 0] * v[:, 2]
+            z = u[:, 0] * v[:, 1] - u[:, 1] * v[:, 0]
+            l2 = (x * x + y * y) + z * z
+            for k in range(lanes):
+                if live[k, r] and l2[k] > 0 and l2[k] < np.inf:
+                    s = off_by(rng, 1.0 / np.sqrt(float(l2[k])))
+                    n[k] = n[k] + np.array([x[k] * s, y[k] * s, z[k] * s], F)
+        pts = q[live].reshape(-1, 3)
+        lo, hi = pts.min(0), pts.max(0)
+        m = lanes_sum(n)
+        ml2 = (m[0] * m[0] + m[1] * m[1]) + m[2] * m[2]
+        if not (ml2 > F(1e-12) and ml2 < np.inf):
+            m = np.array([0, 0, 1], F)
+        m = (m * (F(1) / np.sqrt((m[0] * m[0] + m[1] * m[1]) + m[2] * m[2]))).astype(F)
+        b1 = np.array([0, m[2], -m[1]] if abs(m[0]) < F(0.6) else [-m[2], 0, m[0]], F)
+        b1 = (b1 * (F(1) / np.sqrt((b1[0] * b1[0] + b1[1] * b1[1]) + b1[2] * b1[2]))).astype(F)
+        b2 = np.array([m[1] * b1[2] - m[2] * b1[1], m[2] * b1[0] - m[0] * b1[2], m[0] * b1[1] - m[1] * b1[0]], F)
+        mid = (F(0.5) * (lo + hi)).astype(F)
+        scale = F(1) / (max(hi - lo) + F(1e-30))
+
+        def dot(d, a):
+            return (d[..., 0] * a[0] + d[..., 1] * a[1]) + d[..., 2] * a[2]
+
+        acc = np.zeros((lanes, 6), F)  # n, sx, sy, xx, xy, yy
+        for r in range(R):
+            for k in range(3):
+                d = q[:, r, k] - mid
+                x, y = dot(d, b1) * scale, dot(d, b2) * scale
+                add = np.stack([np.ones(lanes, F), x, y, x * x, x * y, y * y], -1)
+                acc = np.where(live[:, r, None], acc + add, acc).astype(F)
+        cnt, sx, sy, xx, xy, yy = (lanes_sum(acc[:, j]) for j in range(6))
+        inv = F(1) / max(cnt, F(1))
+        th = F(0.5) * off_by(rng, np.arctan2(F(2) * (xy - sx * sy * inv), (xx - sx * sx * inv) - (yy - sy * sy * inv)))
+        if not np.isfinite(th):
+            th = F(0)
+        ct, sn = off_by(rng, np.cos(float(th))), off_by(rng, np.sin(float(th)))
+        ax = np.stack([ct * b1 + sn * b2, ct * b2 - sn * b1, m]).astype(F)
+        x = np.stack([dot(pts - mid, a) for a in ax], -1).astype(F)
+        pl, ph = x.min(0), x.max(0)
+        h, a = (F(0.5) * (ph - pl)).astype(F), (F(0.5) * (hi - lo)).astype(F)
+        if (a[0] * a[1] + a[1] * a[2]) + a[2] * a[0] <= (h[0] * h[1] + h[1] * h[2]) + h[2] * h[0]:
+            c, h, ax = mid, a, np.eye(3, dtype=F)
+        else:
+            t = (pl + ph).astype(F)
+            c = (mid + F(0.5) * ((t[0] * ax[0] + t[1] * ax[1]) + t[2] * ax[2])).astype(F)
+        M = max(np.abs(lo).max(), np.abs(hi).max())
+        grow = F(3.814697265625e-06) * ((h[0] + h[1]) + h[2]) + F(9.5367431640625e-07) * M + F(1e-37)
+        hj = (h * F(1.0000019073486328125) + grow).astype(F) if slack else h
+        return c, (ax * hj[:, None]).astype(F), pts
+
+
+def outside(c, A, pts):
+    """Whether a vertex lies outside the box c + sum t_j A_j, |t_j| <= 1 (solved in float64)."""
+    A = A.astype(np.float64)
+    ln = np.linalg.norm(A, axis=1)
+    d = pts.astype(np.float64) - c.astype(np.float64)
+    if not (ln > 0).all():
+        return bool((np.abs(d).max(0) > 0).any())
+    t = np.linalg.solve((A / ln[:, None]).T, d.T).T / ln
+    return bool((np.abs(t) > 1 + 1e-12).any())
+
+
+@pytest.mark.parametrize("lanes,R", [(16, 1), (32, 4)])
+def test_kernel_boxes_hold_their_vertices(lanes, R):
+    """Patches, needles, points and lumps, near the origin and far from it, of
+    every scale, whole groups and the ends of meshes."""
+    rng = np.random.default_rng(lanes)
+    bare = 0
+    for k in range(400 if lanes == 16 else 120):
+        shape = [(1.0, 0.4, 1e-3), (1.0, 1e-4, 1e-5), (1.0, 1.0, 1.0), (0.0, 0.0, 0.0), (1.0, 1e-7, 0.3)][k % 5]
+        size = 10.0 ** rng.uniform(-12, 8)
+        rot = np.linalg.qr(rng.normal(size=(3, 3)))[0] if k % 3 else np.eye(3)
+        p = (rng.uniform(-1, 1, (lanes, R, 3, 3)) * shape * size) @ rot.T
+        p += rng.uniform(-1, 1, 3) * size * rng.choice([0.0, 1.0, 1e3, 1e6])
+        q = p.astype(F)
+        if k % 4 == 1:  # the mesh ends inside the group
+            flat = np.arange(lanes * R).reshape(R, lanes).T  # triangle r * lanes + lane
+            q[flat >= int(rng.integers(1, lanes * R))] = np.nan
+        c, A, pts = kernel_obb(rng, q, lanes)
+        assert not outside(c, A, pts), (k, size)
+        bare += outside(*kernel_obb(rng, q, lanes, slack=False))
+    assert bare > 20  # without the slack many do not
