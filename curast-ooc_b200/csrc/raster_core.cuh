@@ -1543,7 +1543,10 @@ __device__ __forceinline__ float intersect_mt(V3 dir, V3 v0, V3 e1, V3 e2) {
 // as perturbations of d), and of the division and sum (<= 6u |det|); the
 // margins below over-cover all of them by 2x, in double precision, so a
 // column outside the span cannot pass the float test.  A triangle whose T is
-// within its error bound of 0, or with non-finite values, is not pruned.
+// within its error bound of 0, or with non-finite values, is not pruned; nor is
+// one so large that a product of det, U or V could overflow in float (a NaN u or
+// v passes the reference's comparisons): each is at most S1 S2, St S2 or St S1,
+// the products of the 1-norms of e1, e2 and tvec.
 //
 // The fast-math build (REF_MATH) divides and takes square roots within 2 ulp
 // instead of half of one, which no term above exceeds by more than 3x, and
@@ -1586,7 +1589,7 @@ __device__ __forceinline__ S3Prune s3_prune_setup(V3 av, V3 e1f, V3 e2f, float f
     P.mK = L * 6.0 * u * 1.001 * n1s(P.n1) + 1.01 * eD + eU + eV;
     P.ex = L * 8.0 * u * (1.0 / (double)fa);
     P.ey = L * 8.0 * u * (1.0 / (double)f);
-    P.on = isfinite(T) && isfinite(eT) && fabs(T) > 2.0 * eT && isfinite(P.mK);
+    P.on = isfinite(T) && isfinite(eT) && fabs(T) > 2.0 * eT && isfinite(P.mK) && fmax(S1, St) * S2 < 1e36 && St * S1 < 1e36;
     P.s = T > 0.0 ? 1 : -1;
     return P;
 }

@@ -199,10 +199,11 @@ __device__ __forceinline__ void bin_setup(const CrFrameParams& p, const CrTile& 
     float mD = m * (S1 * S2), mU = m * (St * S2), mV = m * (St * S1);
     float aT = fabsf(T) * 0.99999618530273438f;  // 1 - 2^-18
     // products that underflow keep an absolute margin; sums that are huge or
-    // not finite reject nothing; a T that never hits rejects everything
+    // not finite, or a product of det, U or V that could overflow (its NaN passes
+    // the reference's comparisons), reject nothing; a T that never hits rejects everything
     mD += 1e-30f, mU += 1e-30f, mV += 1e-30f;
     const bool never = !(T != 0.0f && fabsf(T) < INFINITY);
-    const float sum = ((mD + mU) + mV) * Dn + (fabsf(n1.x) + fabsf(n1.y) + fabsf(n1.z)) * Dn +
+    const float sum = (S1 * S2 + (St * S2 + St * S1)) + ((mD + mU) + mV) * Dn + (fabsf(n1.x) + fabsf(n1.y) + fabsf(n1.z)) * Dn +
                       (fabsf(n2.x) + fabsf(n2.y) + fabsf(n2.z)) * Dn + (fabsf(q.x) + fabsf(q.y) + fabsf(q.z)) * Dn +
                       (fabsf(k.x) + fabsf(k.y) + fabsf(k.z)) * Dn;
     if (never || !(sum < 1e36f)) {

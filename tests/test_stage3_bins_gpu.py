@@ -146,3 +146,64 @@ def test_frames_without_memory_for_the_bins(gpu):
                 assert pc.load().cr_last_error() == b""
     for v, r in got[1:]:
         assert torch.equal(v, got[0][0]) and torch.equal(r, got[0][1])
+
+
+def huge(n, seed):
+    """Triangles with one coordinate so large that the float products of stage 3
+    overflow for some of them (a NaN u or v passes the reference's comparisons)."""
+    rng = np.random.default_rng(seed)
+    tri = rng.uniform(-1, 1, (n, 3, 3))
+    tri[..., 2] = -rng.uniform(0.2, 3.0, (n, 3))
+    at = (np.arange(n), rng.integers(0, 3, n), rng.integers(0, 3, n))
+    tri[at] = rng.choice([3e38, -3e38, 1e38, 1e30, -1e30, 1e25], n)
+    pos = tri.reshape(-1, 3).astype(np.float32)
+    return pos, np.arange(3 * n, dtype=np.uint32).reshape(n, 3), rng.integers(0, 2**32, 3 * n, np.uint64).astype(np.uint32)
+
+
+HUGE_VIEW = ((0.1, -0.2, 0.15), (0.4, 0.3, -2.0))  # eye and target: no axis of the view is one of the object's
+
+
+@pytest.mark.parametrize("seed", range(6))
+def test_coordinates_whose_products_overflow(gpu, seed):
+    """The binned kernel, the unbinned one (a context with a memory budget) and
+    batched views against the oracle."""
+    import torch
+    from test_batch_gpu import batched
+
+    W = H = 192
+    mesh = huge(40, 300 + seed)
+    view, proj = scenes.look_at(*HUGE_VIEW), scenes.perspective(60.0, W / H, 0.01, 100.0)
+    fb, st = ol.raster(ol.Frame([(*mesh, scenes.identity())], view), W, H, proj[5])
+    assert st.huge_tiles > 9 and (fb != pc.CLEAR_PIXEL).any()
+    for budget in (0, 8 << 30):
+        with pc.Context(memory_budget=budget) as ctx:
+            inst = [(ctx.mesh_from_host(*mesh), scenes.identity())]
+            vis = torch.empty(W * H, dtype=torch.int64, device="cuda")
+            ctx.render(inst, pc.make_camera(view, proj, W, H), vis.data_ptr(), flags=pc.CR_RENDER_SYNC | pc.CR_RENDER_NO_RESOLVE)
+            torch.cuda.synchronize()
+            assert np.array_equal(vis.cpu().numpy().view(np.uint64), fb), budget
+            for v in batched(ctx, inst, [(view, proj, W, H)] * 2)[0]:
+                assert np.array_equal(v, fb)
+
+
+# SHA-1 of the words that a kernel draws which traces every pixel of every tile (the
+# build before rows were narrowed in this arithmetic)
+UNPRUNED = ["9feb764a075283de", "be7eff0ecfe3ccdc", "0825419f40ee4a45",
+            "5f5f26d43c1c0d4c", "53a26ff30a3af861", "c41377cadbfd2a5a"]
+
+
+@pytest.mark.parametrize("seed", range(6))
+def test_overflow_in_the_reference_build_s_arithmetic(gpu, seed):
+    import hashlib
+
+    import torch
+
+    W = H = 192
+    view, proj = scenes.look_at(*HUGE_VIEW), scenes.perspective(60.0, W / H, 0.01, 100.0)
+    with pc.Context() as ctx:
+        inst = [(ctx.mesh_from_host(*huge(40, 300 + seed)), scenes.identity())]
+        vis = torch.empty(W * H, dtype=torch.int64, device="cuda")
+        ctx.render(inst, pc.make_camera(view, proj, W, H), vis.data_ptr(),
+                   flags=pc.CR_RENDER_SYNC | pc.CR_RENDER_NO_RESOLVE | pc.CR_RENDER_REF_MATH_NO_FMA)
+        torch.cuda.synchronize()
+    assert hashlib.sha1(vis.cpu().numpy().tobytes()).hexdigest()[:16] == UNPRUNED[seed]
