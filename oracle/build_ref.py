@@ -182,7 +182,7 @@ def main(argv=None):
     ap.add_argument("--reference", default=os.environ.get("CURAST_REFERENCE", "/root/reference"))
     ap.add_argument("--force", action="store_true")
     a = ap.parse_args(argv)
-    if not os.path.isdir(a.reference):
+    if not os.path.exists(os.path.join(a.reference, "src", "kernels", "triangles_visbuffer.cu")):
         print("reference checkout not present; keeping prebuilt oracle/_ref", file=sys.stderr)
         return 0
     build(a.reference, a.force)
