@@ -85,11 +85,12 @@ typedef struct cr_config {
  * device memory: per instance it proves from the mesh's precomputed boxes
  * that whole 128-triangle groups, then 16-triangle ones (oriented boxes built
  * on first use) and then single triangles miss every sample or face away --
- * suited to triangles that are small on screen.  AUTO picks
- * BOXES for frames that draw some mesh more than once and for frames of mostly
- * sub-pixel triangles (given memory for the boxes), CELLS for other frames
- * with more than one instance, else OUTCODES; and small frames take every
- * triangle straight through the per-triangle path. */
+ * suited to triangles that are small on screen.  AUTO takes
+ * every triangle of small frames (at most 2M triangles, and larger ones wholly
+ * on screen whose triangles cover half a pixel and more) straight through the
+ * per-triangle path; of the others it picks BOXES for frames that draw some mesh more
+ * than once and for frames of mostly sub-pixel triangles (given memory for the
+ * boxes), else CELLS (OUTCODES in windows of more than 65535 pixels a side). */
 #define CR_CULL_AUTO 0u
 #define CR_CULL_OUTCODES 1u
 #define CR_CULL_CELLS 2u
@@ -175,9 +176,9 @@ enum cr_render_flags {
      * build (its __fdividef calls, approximate divisions and square roots,
      * contracted products), so that the visbuffer matches a CuRast built
      * with its default recipe.  Every triangle takes the reference's
-     * per-triangle path (no exact culling proofs): a frame costs about what
-     * the reference's kernels cost.  Per-stage times report stages 1-3 as
-     * stage 1. */
+     * per-triangle path (no culling proofs beyond the rows of stages 2 and
+     * 3): a frame costs a quarter to two thirds of what the reference's
+     * kernels cost.  Per-stage times report stages 1-3 as stage 1. */
     CR_RENDER_REF_MATH = 1u << 5,
     /* cr_render only (implies CR_RENDER_REF_MATH): the arithmetic of the
      * reference's recipe with --fmad=false added after --use_fast_math (no
@@ -444,8 +445,11 @@ uint32_t cr_scene_class(uint64_t triangles, uint64_t pixels, uint32_t num_views)
  * one frame in the reference's order (triangle count descending, then node
  * index; src/CuRast_render.h:316-345), ids being the prefix sum over the
  * selected nodes.  A selection larger than the cache is drawn in several
- * passes into the same visbuffer with the same ids, resolved pass by
- * pass, so the output does not depend on the budget. */
+ * passes -- runs of the draw order, whatever is resident -- into the same
+ * visbuffer with the same ids, each pass resolving the pixels of its own nodes:
+ * the output depends neither on the budget nor on the frames before.  (Except the
+ * MESH_ID display, whose ids are a node's place within its cache-sized run.)
+ * cr_sync reports an overflow of any pass. */
 #define CR_OOC_MAX_NODE_TRIANGLES 65536u
 
 typedef struct cr_ooc_node {
