@@ -1221,6 +1221,7 @@ cr_status cr_order_instances(const uint32_t* mesh, const uint32_t* triangles, ui
 cr_status cr_render(cr_context* ctx, const cr_instance* instances, uint32_t count, const cr_camera* cam,
                     uint64_t d_visbuffer, uint64_t d_rgba, uint64_t d_colorbuffer, int32_t display, uint32_t flags,
                     void* stream_) {
+    flags &= ~kRenderNextPass;  // the library's own
     return render_impl(ctx, instances, count, nullptr, cam, d_visbuffer, d_rgba, d_colorbuffer, display, flags,
                        stream_, 0, ~0ull, ResolvePart::Whole, nullptr);
 }

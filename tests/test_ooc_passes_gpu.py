@@ -137,3 +137,19 @@ def test_a_closed_scene_gives_its_memory_back(gpu):
                 assert frame(sc, cam, pc.CR_RENDER_SYNC)[2].visible_nodes == 36
         with pc.OocScene(ctx, nodes, 6 << 20) as sc:
             assert frame(sc, cam, pc.CR_RENDER_SYNC)[2].cache_slots > 36
+
+
+def test_a_caller_cannot_keep_the_overflow_words(gpu):
+    """The bit that marks a further pass of a frame is the library's own."""
+    import torch
+
+    pos, idx = grid(-0.5, 0.5, -0.4, 0.4, -2.0)
+    cam, small = camera(60.0, 1024, 768), camera(20.0, 64, 48)
+    vis = torch.empty(1024 * 768, dtype=torch.int64, device="cuda")
+    with pc.Context(max_nontrivial=64) as ctx:
+        inst = [(ctx.mesh_from_host(pos, idx), scenes.identity())]
+        flags = pc.CR_RENDER_NO_RESOLVE | pc.CR_RENDER_NO_CLEAR | 1 << 30
+        for c, want in ((cam, pc.CR_ERR_QUEUE_OVERFLOW), (small, pc.CR_OK)):
+            ctx.render(inst, c, vis.data_ptr(), flags=flags)
+            torch.cuda.synchronize()
+            assert ctx.stats()[0] == want
