@@ -131,7 +131,10 @@ def test_sub_boxes_are_built_once_memory_is_back(gpu):
         inst = [(h, scenes.identity())]
         chunks, seen = [], []
         torch.cuda.empty_cache()
-        held = torch.empty(torch.cuda.mem_get_info()[0] - (900 << 20), dtype=torch.uint8, device="cuda")
+        try:  # leaves less than the gigabyte that the rule wants
+            held = torch.empty(torch.cuda.mem_get_info()[0] - (900 << 20), dtype=torch.uint8, device="cuda")
+        except torch.OutOfMemoryError:
+            pytest.skip("the GPU's free memory cannot be held in one piece")
         for k in range(140):
             if k == 2:
                 del held
