@@ -65,10 +65,11 @@ float det3_glm(const float* m) {
 
 // The item proofs' data of one instance (CR_PROOF_F4) from its float world-view
 // matrix (column-major) and the largest coordinates in its mesh's box (infinite
-// where it is not finite): R its 3x3 part, t its translation, all exact in double.  e = -R^-1 t by cofactors; |det R| only when it exceeds
-// 1e-4 of the product of the columns' 1-norms, which bounds the float
-// det3_glm's error far below it, so the mirror flag the kernels use has the
-// exact sign (else 0: no back-face proof for this instance).
+// where it is not finite): R its 3x3 part, t its translation, all exact in double.
+// e = -R^-1 t by cofactors; |det R| only when it exceeds 1e-4 of the product of
+// the columns' 1-norms, which bounds the float det3_glm's error far below it, so
+// the mirror flag the kernels use has the exact sign (else 0: no back-face proof
+// for this instance).
 void proof_data(const float* wv, const double* mabs, float* o) {
     double R[3][3];
 #pragma GCC unroll 3  // as loops 20 % slower (93 / 73 us per 3,000 instances)

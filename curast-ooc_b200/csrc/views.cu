@@ -599,7 +599,8 @@ __global__ void __launch_bounds__(256) k_cull_views(const CrFrameParams p) {
 //
 // Bound by instruction issue and by dependent arithmetic that 3 blocks of 80 registers
 // do not hide (61 % of the slots, 8 views of a 4M terrain).  64 views over the
-// 60M-triangle terrain (0.02 pixels per triangle; 33 % of the triangles face away, 52 % miss every sample, 13 % are drawn), ms:
+// 60M-triangle terrain (0.02 pixels per triangle; 33 % of the triangles face away,
+// 52 % miss every sample, 13 % are drawn), ms:
 // every triangle of an item that is large on screen through the full path, and cell
 // records of the distinct vertices of the others, 18.4; quick_misses ahead of the path
 // 14.0; indices by plain loads instead of a TMA tile per item, which freed 20 registers
